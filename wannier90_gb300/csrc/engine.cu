@@ -792,7 +792,7 @@ int Engine::finish(std::string& err) {
     launches_ += 1;
   }
   // final unitarity check (src/wannierise.F90:890-892)
-  k_unitarity<<<n_k_, 128, 0, st>>>(dprobs_, wmk, d_unit_);
+  k_unitarity<<<n_k_, 256, 0, st>>>(dprobs_, wmk, d_unit_);
   W90G_CHECK(cudaGetLastError());
   launches_ += 1;
   std::vector<double> unit(n_k_);
