@@ -41,97 +41,272 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 // |H_pq|^2 <= skip_rel ||H||_F^2 are left alone and a sweep that rotates no pair also ends
 // the solve (the threshold-Jacobi rule: reachable at any size, where the plain criterion
 // can sit at the roundoff floor of large matrices).
-// Returns the number of sweeps used (or -1 when not converged within max_sweeps).
+// Returns the number of FP64 sweeps used (or -1 when not converged within max_sweeps).
+//
+// What bounds it is the FP64 pipe (2 lanes per SM), so the work is arranged to need few
+// FP64 instructions:
+//   * a round's rotations touch pairs of pairs: each 2 x 2 block of H is updated once,
+//     B <- J_s^H B J_t, and mirrored (6 W^3 FMA per sweep for H, not 12), and a block or
+//     column pair whose rotations were skipped is left alone;
+//   * given two W x W scratch matrices (s1, s2), the first sweeps run in FP32 on a scaled
+//     copy kept in V's storage.  Their eigenvectors, orthonormalised to FP64 by one cubic
+//     Newton-Schulz step V (15/8 - 10/8 G + 3/8 G^2), G = V^H V, turn H into V^H H V with an
+//     off-diagonal part of ~1e-6, from which the FP64 sweeps -- the same rotations and the
+//     same convergence test -- need two instead of seven to ten.  14 W^3 FMA for that against
+//     12 W^3 per sweep.
+// Measured on a GB300 at the Loewdin step of 1000 matrices of W = 32: see k_lowdin.
 // ----------------------------------------------------------------------------
-__device__ __noinline__ static int cta_jacobi(double2* H, double2* V, int W, int max_sweeps, double* red,
-                          double* rc, double2* rse, int* rp, int* rq, double skip_rel = 0.0) {
-  const int WW = W * W;
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) {
-    V[e] = cmk((e % W) == (e / W) ? 1.0 : 0.0, 0.0);
-  }
+struct JacF2 {
+  float x, y;
+};
+
+template <class R, class R2>
+__device__ __forceinline__ R2 jac_mk(R x, R y) {
+  R2 r;
+  r.x = x;
+  r.y = y;
+  return r;
+}
+// c a - conj(s) b  and  s a + c b
+template <class R, class R2>
+__device__ __forceinline__ R2 jac_p(R c, R2 s, R2 a, R2 b) {
+  return jac_mk<R, R2>(c * a.x - (s.x * b.x + s.y * b.y), c * a.y - (s.x * b.y - s.y * b.x));
+}
+template <class R, class R2>
+__device__ __forceinline__ R2 jac_q(R c, R2 s, R2 a, R2 b) {
+  return jac_mk<R, R2>(c * b.x + (s.x * a.x - s.y * a.y), c * b.y + (s.x * a.y + s.y * a.x));
+}
+template <class R2>
+__device__ __forceinline__ R2 jac_conj(R2 a) {
+  R2 r;
+  r.x = a.x;
+  r.y = -a.y;
+  return r;
+}
+
+// element e of the upper triangle i <= j, counted down the columns: e = j (j + 1) / 2 + i
+// (consecutive threads take consecutive elements, so no warp idles on the lower triangle)
+__device__ __forceinline__ void tri_index(int e, int& i, int& j) {
+  j = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+  while (j * (j + 1) / 2 > e) --j;
+  while ((j + 1) * (j + 2) / 2 <= e) ++j;
+  i = e - j * (j + 1) / 2;
+}
+
+// One sweep of rotations over all pairs of H, applied to V; pairs with |H_pq| <= tiny or
+// |H_pq|^2 <= thr are skipped.  Returns how many pairs this thread rotated.
+template <class R, class R2>
+__device__ __forceinline__ int jac_sweep(R2* H, R2* V, int W, R thr, R tiny, R* rc, R2* rse, int* rp, int* rq) {
   const int n = (W + 1) & ~1;     // even number of players (one dummy when W is odd)
   const int npair = n / 2;
-  __syncthreads();
-  for (int sweep = 0; sweep <= max_sweeps; ++sweep) {
-    double off = 0.0, fro = 0.0;
-    for (int e = threadIdx.x; e < WW; e += blockDim.x) {
-      const double a = cabs2(H[e]);
-      fro += a;
-      if ((e % W) != (e / W)) off += a;
+  const int nblk = npair * (npair - 1) / 2;
+  int rotated = 0;
+  for (int r = 0; r < n - 1; ++r) {
+    for (int t = threadIdx.x; t < npair; t += blockDim.x) {
+      int p, q;
+      if (t == 0) {
+        p = r;
+        q = n - 1;
+      } else {
+        p = r + t;
+        if (p >= n - 1) p -= n - 1;
+        q = r - t;
+        if (q < 0) q += n - 1;
+      }
+      if (p > q) {
+        const int x = p;
+        p = q;
+        q = x;
+      }
+      R c = R(1);
+      R2 se = jac_mk<R, R2>(R(0), R(0));
+      int live = 0;
+      if (q < W) {
+        const R2 b = H[q * W + p];
+        const R b2 = b.x * b.x + b.y * b.y;
+        const R ab = sqrt(b2);
+        if (ab > tiny && b2 > thr) {
+          live = 1;
+          ++rotated;
+          const R a = H[p * W + p].x, d = H[q * W + q].x;
+          const R th = (d - a) / (R(2) * ab);
+          const R tt = (th >= R(0) ? R(1) : R(-1)) / (fabs(th) + sqrt(R(1) + th * th));
+          c = R(1) / sqrt(R(1) + tt * tt);
+          const R s = tt * c / ab;
+          se = jac_mk<R, R2>(s * b.x, s * b.y);
+          // the pair's own block: diag(a - t |b|, d + t |b|)
+          H[p * W + p] = jac_mk<R, R2>(a - tt * ab, R(0));
+          H[q * W + q] = jac_mk<R, R2>(d + tt * ab, R(0));
+          H[q * W + p] = H[p * W + q] = jac_mk<R, R2>(R(0), R(0));
+        }
+      }
+      rp[t] = p;
+      rq[t] = live ? q : (q < W ? q + 0x10000 : 0x20000);   // bit 16: no rotation; bit 17: dummy
+      rc[t] = c;
+      rse[t] = se;
     }
-    off = block_sum(off, red);
-    fro = block_sum(fro, red);
-    if (off <= 1.0e-30 * fro || off == 0.0) return sweep;
-    if (sweep == max_sweeps) break;
-    const double thr = skip_rel * fro;
-    int rotated = 0;
-    for (int r = 0; r < n - 1; ++r) {
-      for (int t = threadIdx.x; t < npair; t += blockDim.x) {
-        int p, q;
-        if (t == 0) {
-          p = r;
-          q = n - 1;
-        } else {
-          p = (r + t) % (n - 1);
-          q = (r - t + (n - 1)) % (n - 1);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nblk + W * npair; e += blockDim.x) {
+      if (e < nblk) {
+        int s, t;   // block (s, t), s < t
+        tri_index(e, s, t);
+        ++t;
+        const int qsx = rq[s], qtx = rq[t];
+        if (qsx >= 0x10000 && qtx >= 0x10000) continue;
+        const bool ds = (qsx & 0x20000) != 0, dt = (qtx & 0x20000) != 0;
+        const int ps = rp[s], pt = rp[t], qs = ds ? ps : (qsx & 0xFFFF), qt = dt ? pt : (qtx & 0xFFFF);
+        const R cs = rc[s], ct = rc[t];
+        const R2 ss = rse[s], st = rse[t];
+        // (a dummy's partner repeats its own element; its rotation is the identity and its
+        // results are not stored)
+        const R2 b11 = H[pt * W + ps], b12 = H[qt * W + ps], b21 = H[pt * W + qs], b22 = H[qt * W + qs];
+        const R2 x11 = jac_p(ct, st, b11, b12), x12 = jac_q(ct, st, b11, b12);
+        const R2 x21 = jac_p(ct, st, b21, b22), x22 = jac_q(ct, st, b21, b22);
+        // rows by J_s^H: c x_p - s x_q and conj(s) x_p + c x_q
+        const R2 sc = jac_conj(ss);
+        const R2 y11 = jac_p(cs, sc, x11, x21), y21 = jac_q(cs, sc, x11, x21);
+        const R2 y12 = jac_p(cs, sc, x12, x22), y22 = jac_q(cs, sc, x12, x22);
+        H[pt * W + ps] = y11;
+        H[ps * W + pt] = jac_conj(y11);
+        if (!dt) {
+          H[qt * W + ps] = y12;
+          H[ps * W + qt] = jac_conj(y12);
         }
-        if (p > q) {
-          const int x = p;
-          p = q;
-          q = x;
-        }
-        double c = 1.0;
-        double2 se = cmk(0, 0);
-        if (q < W) {
-          const double2 b = H[q * W + p];
-          const double ab = sqrt(cabs2(b));
-          if (ab > 1.0e-300 && (skip_rel == 0.0 || ab * ab > thr)) {
-            ++rotated;
-            const double a = H[p * W + p].x, d = H[q * W + q].x;
-            const double th = (d - a) / (2.0 * ab);
-            const double tt = (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(1.0 + th * th));
-            c = 1.0 / sqrt(1.0 + tt * tt);
-            const double s = tt * c;
-            se = cmk(s * b.x / ab, s * b.y / ab);
+        if (!ds) {
+          H[pt * W + qs] = y21;
+          H[qs * W + pt] = jac_conj(y21);
+          if (!dt) {
+            H[qt * W + qs] = y22;
+            H[qs * W + qt] = jac_conj(y22);
           }
         }
-        rp[t] = p;
-        rq[t] = q;
-        rc[t] = c;
-        rse[t] = se;
+      } else {
+        // columns of V: V <- V J
+        const int i = (e - nblk) % W, t = (e - nblk) / W;
+        const int q = rq[t];
+        if (q >= 0x10000) continue;
+        const int p = rp[t];
+        const R2 vp = V[p * W + i], vq = V[q * W + i];
+        V[p * W + i] = jac_p(rc[t], rse[t], vp, vq);
+        V[q * W + i] = jac_q(rc[t], rse[t], vp, vq);
       }
-      __syncthreads();
-      // columns: H <- H J, V <- V J
-      for (int e = threadIdx.x; e < W * npair; e += blockDim.x) {
-        const int i = e % W, t = e / W;
-        const int p = rp[t], q = rq[t];
-        if (q >= W) continue;
-        const double c = rc[t];
-        const double2 se = rse[t];
-        const double2 hp = H[p * W + i], hq = H[q * W + i];
-        // (HJ)_ip = c H_ip - conj(se) H_iq ; (HJ)_iq = se H_ip + c H_iq
-        H[p * W + i] = csub(cscale(hp, c), cmul(cconj(se), hq));
-        H[q * W + i] = cadd(cmul(se, hp), cscale(hq, c));
-        const double2 vp = V[p * W + i], vq = V[q * W + i];
-        V[p * W + i] = csub(cscale(vp, c), cmul(cconj(se), vq));
-        V[q * W + i] = cadd(cmul(se, vp), cscale(vq, c));
+    }
+    __syncthreads();
+  }
+  return rotated;
+}
+
+// C = op(A) B (W x W, column-major), the upper triangle only and mirrored when HERM
+template <bool CA, bool HERM>
+__device__ __forceinline__ void jac_mm(double2* C, const double2* A, const double2* B, int W) {
+  const int items = HERM ? W * (W + 1) / 2 : W * W;
+  for (int e = threadIdx.x; e < items; e += blockDim.x) {
+    int i, j;
+    if (HERM) tri_index(e, i, j);
+    else i = e % W, j = e / W;
+    double2 acc = cmk(0, 0);
+#pragma unroll 4
+    for (int l = 0; l < W; ++l) {
+      if (CA) cfmac(acc, A[i * W + l], B[j * W + l]);
+      else cfma(acc, A[l * W + i], B[j * W + l]);
+    }
+    if (HERM && i == j) acc.y = 0.0;
+    C[j * W + i] = acc;
+    if (HERM && i < j) C[i * W + j] = cconj(acc);
+  }
+}
+
+// The FP32 stage: eigenvectors of H to ~1e-6, made orthonormal to FP64 in V, and H <- V^H H V.
+// The copy is shifted by the mean of the diagonal and scaled by the norm of what is left, so
+// that FP32 resolves the eigenvalues' spread (A^H A of a nearly unitary A is close to I).
+__device__ __forceinline__ void jac_fp32_stage(double2* H, double2* V, int W, double mean, double spread, double* red,
+                                               double* rc, double2* rse, int* rp, int* rq, double2* s1,
+                                               double2* s2) {
+  const int WW = W * W;
+  JacF2* Hf = reinterpret_cast<JacF2*>(V);
+  JacF2* Vf = Hf + WW;
+  const double sc = 1.0 / sqrt(spread);
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) {
+    const double2 h = H[e];
+    const bool d = (e % W) == (e / W);
+    Hf[e].x = (float)((d ? h.x - mean : h.x) * sc);
+    Hf[e].y = d ? 0.0f : (float)(h.y * sc);
+    Vf[e].x = d ? 1.0f : 0.0f;
+    Vf[e].y = 0.0f;
+  }
+  __syncthreads();
+  // until a sweep rotates no pair above 1e-7 of the norm (a dozen sweeps at most: what is
+  // left is the FP64 sweeps' work)
+  for (int sweep = 0; sweep < 12; ++sweep) {
+    const int rot = jac_sweep<float, JacF2>(Hf, Vf, W, 1.0e-14f, 1.0e-30f, reinterpret_cast<float*>(rc),
+                                            reinterpret_cast<JacF2*>(rse), rp, rq);
+    if (block_sum((double)rot, red) == 0.0) break;
+  }
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) s1[e] = cmk((double)Vf[e].x, (double)Vf[e].y);
+  __syncthreads();
+  jac_mm<true, true>(V, s1, s1, W);      // G
+  __syncthreads();
+  jac_mm<false, true>(s2, V, V, W);      // G^2
+  __syncthreads();
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) {
+    const double2 g = V[e], g2 = s2[e];
+    const double d = (e % W) == (e / W) ? 1.875 : 0.0;
+    V[e] = cmk(d - 1.25 * g.x + 0.375 * g2.x, 0.375 * g2.y - 1.25 * g.y);
+  }
+  __syncthreads();
+  jac_mm<false, false>(s2, s1, V, W);
+  __syncthreads();
+  jac_mm<false, false>(s1, H, s2, W);
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) V[e] = s2[e];
+  __syncthreads();
+  jac_mm<true, true>(H, s2, s1, W);
+  __syncthreads();
+}
+
+__device__ __noinline__ static int cta_jacobi(double2* H, double2* V, int W, int max_sweeps, double* red,
+                          double* rc, double2* rse, int* rp, int* rq, double skip_rel = 0.0,
+                          double2* s1 = nullptr, double2* s2 = nullptr) {
+  const int WW = W * W;
+  // With the FP32 stage the last sweep starts from a part that may sit anywhere below the
+  // plain criterion, where a solve from H itself overshoots it by orders: it is held to
+  // 1e-33 instead, and its rotations below 1e-17.5 of the norm are left out.
+  const double conv = s1 != nullptr && skip_rel == 0.0 ? 1.0e-33 : 1.0e-30;
+  const double skip = s1 != nullptr && skip_rel == 0.0 ? 1.0e-35 : skip_rel;
+  bool started = false;
+  __syncthreads();
+  for (int sweep = 0; sweep <= max_sweeps; ++sweep) {
+    double off = 0.0, dia = 0.0, tr = 0.0;
+    for (int e = threadIdx.x; e < WW; e += blockDim.x) {
+      const double a = cabs2(H[e]);
+      if ((e % W) != (e / W)) {
+        off += a;
+      } else {
+        dia += a;
+        tr += H[e].x;
       }
-      __syncthreads();
-      // rows: H <- J^H H
-      for (int e = threadIdx.x; e < W * npair; e += blockDim.x) {
-        const int j = e % W, t = e / W;
-        const int p = rp[t], q = rq[t];
-        if (q >= W) continue;
-        const double c = rc[t];
-        const double2 se = rse[t];
-        const double2 hp = H[j * W + p], hq = H[j * W + q];
-        // (J^H H)_pj = c H_pj - se H_qj ; (J^H H)_qj = conj(se) H_pj + c H_qj
-        H[j * W + p] = csub(cscale(hp, c), cmul(se, hq));
-        H[j * W + q] = cadd(cmul(cconj(se), hp), cscale(hq, c));
+    }
+    off = block_sum(off, red);
+    dia = block_sum(dia, red);
+    const double fro = off + dia;
+    if (!started) {
+      started = true;
+      const double mean = block_sum(tr, red) / (double)W;
+      const double spread = off + fmax(dia - (double)W * mean * mean, 0.0);
+      // (a matrix whose off-diagonal part is at 1e-5 already is where the FP32 stage ends;
+      // extreme or non-finite norms keep to FP64)
+      if (s1 != nullptr && W >= 6 && off > 1.0e-10 * spread && off > 1.0e-26 * fro && spread > 1.0e-200 &&
+          fro < 1.0e200) {
+        jac_fp32_stage(H, V, W, mean, spread, red, rc, rse, rp, rq, s1, s2);
+        --sweep;
+        continue;
       }
+      for (int e = threadIdx.x; e < WW; e += blockDim.x) V[e] = cmk((e % W) == (e / W) ? 1.0 : 0.0, 0.0);
       __syncthreads();
     }
-    if (skip_rel > 0.0 && block_sum((double)rotated, red) == 0.0) return sweep + 1;
+    if (off <= conv * fro || off == 0.0) return sweep;
+    if (sweep == max_sweeps) break;
+    const int rotated = jac_sweep<double, double2>(H, V, W, skip * fro, 1.0e-300, rc, rse, rp, rq);
+    if (skip > 0.0 && block_sum((double)rotated, red) == 0.0) return sweep + 1;
   }
   return -1;
 }
