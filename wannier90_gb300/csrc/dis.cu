@@ -26,6 +26,7 @@
 
 #include "cta.cuh"
 #include "dis.h"
+#include "polar.h"
 
 namespace w90g {
 
@@ -76,6 +77,7 @@ struct DisDev {
   const double2* sym_db;
   double2* sym_ws;
   int* sym_status;
+  const int* pstat;      // [k] kPolarDone where k_oz_polar has formed this kernel's polar factor; null: never
 };
 
 constexpr int kDisSymWs = 16;
@@ -200,7 +202,13 @@ __global__ void __launch_bounds__(256) k_dis_project(DisDev D) {
   __syncthreads();
   for (int e = threadIdx.x; e < nb * W; e += blockDim.x) Ak[e] = ws[e];
   __syncthreads();
-  cta_polar(ws + 5 * NN, nb, Ak, nb, n, W, ws + NN, ws + 2 * NN, ws + 3 * NN, ws + 4 * NN, sh.js(), &sh.flag);
+  // (k_oz_polar, run before, leaves its result in the same place)
+  if (D.pstat && D.pstat[k] == kPolarDone) {
+    if (threadIdx.x == 0) sh.flag = 0;
+    __syncthreads();
+  } else {
+    cta_polar(ws + 5 * NN, nb, Ak, nb, n, W, ws + NN, ws + 2 * NN, ws + 3 * NN, ws + 4 * NN, sh.js(), &sh.flag);
+  }
   for (int e = threadIdx.x; e < nb * W; e += blockDim.x) {
     const int i = e % nb;
     Uk[e] = (i < n) ? ws[5 * NN + e] : cmk(0, 0);
@@ -476,6 +484,14 @@ __global__ void __launch_bounds__(256) k_dis_gauge(DisDev D, int cur) {
   if (threadIdx.x == 0 && sw < 0) D.status[k] = 2;
 }
 
+// ---- U_opt^H A into the k's workspace, for k_oz_polar
+__global__ void __launch_bounds__(256) k_dis_ua(DisDev D, int cur) {
+  const int k = blockIdx.x;
+  const int nb = D.nb, W = D.W;
+  cta_zgemm(D.ws + (size_t)k * kWs * nb * nb, W, D.U[cur] + (size_t)k * nb * W, nb, true, D.A + (size_t)k * nb * W, nb,
+            false, W, W, D.ndim[k]);
+}
+
 // ---- internal_find_u (:531-698): U0 = polar factor of U_opt^H A
 __global__ void __launch_bounds__(256) k_dis_findu(DisDev D, int cur) {
   __shared__ DisShared sh;
@@ -485,6 +501,7 @@ __global__ void __launch_bounds__(256) k_dis_findu(DisDev D, int cur) {
   double2* ws = D.ws + (size_t)k * kWs * NN;
   const double2* Uk = D.U[cur] + (size_t)k * nb * W;
   const double2* Ak = D.A + (size_t)k * nb * W;
+  if (D.pstat && D.pstat[k] == kPolarDone) return;
   cta_zgemm(ws, W, Uk, nb, true, Ak, nb, false, W, W, n);
   __syncthreads();
   cta_polar(D.U0 + (size_t)k * W * W, W, ws, W, W, W, ws + NN, ws + 2 * NN, ws + 3 * NN, ws + 4 * NN, sh.js(), &sh.flag);
@@ -978,7 +995,7 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
                o_zin = take((size_t)K * NN * 16), o_zout = take((size_t)K * NN * 16),
                o_uw = take((size_t)K * W * W * 16), o_m0 = take((size_t)K * B * W * W * 16),
                o_ws = take((size_t)K * kWs * NN * 16), o_wk1 = take(K * 8), o_wk = take(K * 8),
-               o_st = take(K * 4), o_vz = take((size_t)K * NN * 16), o_sw = take(4);
+               o_st = take(K * 4), o_ps = take(K * 4), o_vz = take((size_t)K * NN * 16), o_sw = take(4);
   // symmetry tables: ik, moff, mem, goff, grp, status; slot matrices; workspace
   std::vector<int> sym_ints;
   if (nir > 0) {
@@ -1055,6 +1072,7 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
     D.wk1 = (double*)(a + o_wk1);
     D.wk = (double*)(a + o_wk);
     D.status = (int*)(a + o_st);
+    D.pstat = (const int*)(a + o_ps);
     D.Vz = (double2*)(a + o_vz);
     D.max_sweeps = (int*)(a + o_sw);
     D.sym_nir = nir;
@@ -1091,6 +1109,24 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   DIS_CHECK(cudaMemcpyAsync(D.U[0], s.A, (size_t)K * nb * W * 16, in_kind, st));
   DIS_CHECK(cudaMemsetAsync(D.status, 0, K * 4, st));
   DIS_CHECK(cudaMemsetAsync(D.max_sweeps, 0, 4, st));
+  // The polar factors on the tensor cores first (k_oz_polar; from 9 bands on, as in the
+  // projection of an isolated group); the kernels after it take what it left alone.
+  {
+    PolarArgs a{};
+    a.x = D.U[0];
+    a.ldx = a.ldq = a.qrows = nb;
+    a.strideX = (size_t)nb * W;
+    a.q = D.ws + 5 * NN;
+    a.strideQ = a.strideW = kWs * NN;
+    a.rows = D.ndim;
+    a.row0 = D.nfirst;
+    a.cols = W;
+    a.n = *std::max_element(ndim.begin(), ndim.end());
+    a.work = D.ws + NN;
+    a.status = (int*)D.pstat;
+    if (a.n >= 9) DIS_CHECK(launch(kDisProject, [&] { oz_polar_launch(a, K, st); }));
+    else DIS_CHECK(cudaMemsetAsync((void*)D.pstat, 0, K * 4, st));
+  }
   DIS_CHECK(launch(kDisProject, [&] { k_dis_project<<<K, 256, 0, st>>>(D); }));
   if (any_froz) DIS_CHECK(launch(kDisFroz, [&] { k_dis_froz<<<K, 256, 0, st>>>(D); }));
   DIS_CHECK(cudaMemcpyAsync(status.data(), D.status, K * 4, cudaMemcpyDeviceToHost, st));
@@ -1154,6 +1190,20 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   }
   // the subspace-Hamiltonian gauge is kept out in the symmetry-adapted mode (:2675)
   if (nir == 0) DIS_CHECK(launch(kDisGauge, [&] { k_dis_gauge<<<K, 256, 0, st>>>(D, cur); }));
+  if (W >= 9) {
+    PolarArgs a{};
+    a.x = D.ws;
+    a.ldx = a.ldq = a.qrows = a.cols = a.n = W;
+    a.strideX = a.strideW = kWs * NN;
+    a.q = D.U0;
+    a.strideQ = (size_t)W * W;
+    a.work = D.ws + NN;
+    a.status = (int*)D.pstat;
+    DIS_CHECK(launch(kDisFindU, [&] { k_dis_ua<<<K, 256, 0, st>>>(D, cur); }));
+    DIS_CHECK(launch(kDisFindU, [&] { oz_polar_launch(a, K, st); }));
+  } else {
+    DIS_CHECK(cudaMemsetAsync((void*)D.pstat, 0, K * 4, st));
+  }
   DIS_CHECK(launch(kDisFindU, [&] { k_dis_findu<<<K, 256, 0, st>>>(D, cur); }));
   // symmetric initial U with d = D (sitesym_replace_d_matrix_band, :237, :688-692)
   if (nir > 0) DIS_CHECK(launch(kDisSym, [&] { k_dis_sym_u<<<nir, 256, 0, st>>>(D, cur, 1); }));

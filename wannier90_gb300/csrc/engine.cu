@@ -15,6 +15,7 @@
 #include <sstream>
 
 #include "engine.h"
+#include "polar.h"
 
 namespace w90g {
 
@@ -63,6 +64,7 @@ namespace {
 constexpr size_t kAlign = 256;
 size_t align_up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 constexpr int kTileW = 32;
+constexpr int kPolarMinW = 9;   // projection on the tensor cores from this width on (see project)
 
 #define W90G_CHECK(call)                                                          \
   do {                                                                            \
@@ -583,6 +585,22 @@ int Engine::project(std::string& err) {
   const int ws = std::max(maxW_small_, 1);
   const WorkMap wmk{d_offs_k_, nprob()};
   const WorkMap wmkb{d_offs_kb_, nprob()};
+  // The polar factors on the tensor cores from num_wann 9 on (project of 1000 k: W = 9 and
+  // above; narrower ones fill little of a 128-row tile and their FP64 form is the faster one);
+  // k_lowdin takes what is left.  Work: the second M buffer, which the projection does not use.
+  W90G_CHECK(cudaMemsetAsync(d_status_, 0, n_k_ * sizeof(int), st));
+  if (nprob() == 1 && specs_[0].W >= kPolarMinW && specs_[0].W <= kPolarMaxN && specs_[0].B >= kPolarMats) {
+    const size_t W = specs_[0].W, WW = W * W;
+    PolarArgs a{};
+    a.x = a.q = hprobs_[0].U[0];
+    a.ldx = a.ldq = a.qrows = a.cols = a.n = (int)W;
+    a.strideX = a.strideQ = WW;
+    a.work = hprobs_[0].M[1];
+    a.strideW = kPolarMats * WW;
+    a.status = d_status_;
+    W90G_CHECK(oz_polar_launch(a, n_k_, st));
+    launches_ += 1;
+  }
   k_lowdin<<<n_k_, 256, 4 * ws * ws * 16, st>>>(dprobs_, wmk, d_status_);
   W90G_CHECK(cudaGetLastError());
   launches_ += 1;

@@ -15,6 +15,7 @@
 // precomputed, exp(X) by an optimised Taylor scheme instead of an eigensolver) and keep
 // W <= 32 operands in shared memory.
 #include "cta.cuh"
+#include "polar.h"
 
 namespace w90g {
 
@@ -1193,10 +1194,15 @@ __global__ void k_log_init(const Problem* __restrict__ probs) {
 // ----------------------------------------------------------------------------
 // k_lowdin: overlap_project's U(k) = Z V^dagger from A(k) = Z S V^dagger
 // (src/overlap.F90:842-860), computed as U = A (A^H A)^{-1/2} = A V L^{-1/2} V^H with the
-// Jacobi eigenpairs (V, L) of A^H A: the same unitary polar factor for full-rank A.
+// Jacobi eigenpairs (V, L) of A^H A: the same unitary polar factor for full-rank A.  The
+// eigenpairs carry the square of A's condition number; the two steps after them take it back
+// to the condition number itself: one Newton-Schulz step (U unitary again), then U <- U (I + X)
+// with X anti-Hermitian from X H + H X = H1 - H1^H, H1 = U^H A (the polar factor is the U
+// that makes H1 Hermitian), solved in the eigenbasis, where H = L^{1/2}.
 // Input A(k) in U[cur](k) (the reference reads A into u_matrix, src/wannier_prog.F90:523-529);
 // output U overwrites it.  One CTA (256 threads) per (problem, k).
-// Status per k: 0 ok, 1 rank deficient, 2 Jacobi not converged.
+// Status per k: 0 ok, 1 rank deficient, 2 Jacobi not converged.  A matrix whose status is
+// kPolarDone on entry has been finished by k_oz_polar.
 // ----------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_lowdin(const Problem* __restrict__ probs, WorkMap wm,
                                                 int* __restrict__ status) {
@@ -1205,6 +1211,8 @@ __global__ void __launch_bounds__(256) k_lowdin(const Problem* __restrict__ prob
   __shared__ double rc[128];
   __shared__ double2 rse[128];
   __shared__ int rp[128], rq[128];
+  __shared__ double s_h[256];
+  if (status[blockIdx.x] == kPolarDone) return;
   int k;
   const int p = locate(wm, blockIdx.x, k);
   const Problem& P = probs[p];
@@ -1214,34 +1222,60 @@ __global__ void __launch_bounds__(256) k_lowdin(const Problem* __restrict__ prob
   double2* Uk = P.U[P.st->cur] + (size_t)k * WW;
   for (int e = threadIdx.x; e < WW; e += blockDim.x) A[e] = Uk[e];
   __syncthreads();
-  cta_gemm<true>(S, W, A, W, A, W, W);
-  __syncthreads();
-  const int sweeps = cta_jacobi(S, V, W, 60, red, rc, rse, rp, rq);
-  // V' = V diag(lambda^{-1/2}) into T
+  jac_mm<true, true>(S, A, A, W);
+  // A is scratch of the eigensolver, and read again afterwards
+  const int sweeps = cta_jacobi(S, V, W, 60, red, rc, rse, rp, rq, 0.0, A, T);
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) A[e] = Uk[e];
   __shared__ int bad;
   if (threadIdx.x == 0) bad = (sweeps < 0) ? 2 : 0;
   __syncthreads();
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) {
-    const int j = e / W;
+  for (int j = threadIdx.x; j < W; j += blockDim.x) {
     const double l = S[j * W + j].x;
     if (!(l > 0.0)) bad = 1;
-    T[e] = cscale(V[e], 1.0 / sqrt(l));
+    s_h[j] = sqrt(l);
   }
+  __syncthreads();
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) T[e] = cscale(V[e], 1.0 / s_h[e / W]);
   __syncthreads();
   cta_gemm<false>(S, W, A, W, T, W, W);      // S <- A V L^{-1/2}
   __syncthreads();
-  // U = S V^H : compute via (V S^H)^H  -> use conj-transposed product with A := V
-  // U_ij = sum_l S_il conj(V_jl)
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) {
-    const int i = e % W, j = e / W;
-    double2 acc = cmk(0, 0);
-    for (int l = 0; l < W; ++l) {
-      const double2 s = S[l * W + i];
-      const double2 v = V[l * W + j];
-      acc = cadd(acc, cmulc(s, v));
+  // C = X V^H
+  auto mul_vh = [&](double2* C, const double2* X) {
+    for (int e = threadIdx.x; e < WW; e += blockDim.x) {
+      const int i = e % W, j = e / W;
+      double2 acc = cmk(0, 0);
+      for (int l = 0; l < W; ++l) acc = cadd(acc, cmulc(X[l * W + i], V[l * W + j]));
+      C[e] = acc;
     }
-    Uk[e] = acc;
-  }
+  };
+  mul_vh(T, S);
+  __syncthreads();
+  // Newton-Schulz: U (3 I - U^H U) / 2
+  jac_mm<true, true>(S, T, T, W);
+  __syncthreads();
+  for (int e = threadIdx.x; e < WW; e += blockDim.x)
+    S[e] = cmk(((e % W) == (e / W) ? 1.5 : 0.0) - 0.5 * S[e].x, -0.5 * S[e].y);
+  __syncthreads();
+  cta_gemm<false>(Uk, W, T, W, S, W, W);
+  __syncthreads();
+  // the anti-Hermitian part of H1 = U^H A, twice: K = H1 - H1^H; X = V [(V^H K V)_ij / (h_i + h_j)] V^H
+  cta_gemm<true>(S, W, Uk, W, A, W, W);
+  __syncthreads();
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) T[e] = csub(S[e], cconj(S[(e % W) * W + e / W]));
+  __syncthreads();
+  cta_gemm<false>(S, W, T, W, V, W, W);
+  __syncthreads();
+  cta_gemm<true>(T, W, V, W, S, W, W);
+  __syncthreads();
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) T[e] = cscale(T[e], 1.0 / (s_h[e % W] + s_h[e / W]));
+  __syncthreads();
+  cta_gemm<false>(S, W, V, W, T, W, W);
+  __syncthreads();
+  mul_vh(T, S);
+  __syncthreads();
+  cta_gemm<false>(S, W, Uk, W, T, W, W);
+  __syncthreads();
+  for (int e = threadIdx.x; e < WW; e += blockDim.x) Uk[e] = cadd(Uk[e], S[e]);
   if (threadIdx.x == 0) status[blockIdx.x] = bad;
 }
 
