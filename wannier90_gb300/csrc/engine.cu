@@ -43,6 +43,11 @@ __global__ void k_phases(const Problem* probs, int mode);
 __global__ void k_sym_grad(const Problem* probs, WorkMap wm);
 __global__ void k_sym_dir(const Problem* probs, WorkMap wm);
 __global__ void k_sym_u(const Problem* probs, WorkMap wm);
+cudaError_t oz3_launch(int wp, const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, cudaStream_t s);
+cudaError_t oz3_preslice_launch(int wp, const Problem* probs, WorkMap wm, int ngroups, int tmax, cudaStream_t s);
+cudaError_t oz3_set_attributes(int wp);
+void oz3_bytes(int W, int K, int B, size_t out[4]);
+int oz3_tiles(int W, int B);
 cudaError_t oz2_launch(int wp, int step, const Problem* probs, WorkMap wm, int which, int ngroups,
                        cudaStream_t s);
 cudaError_t oz2_set_attributes(int wp);
@@ -227,7 +232,14 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
     z.ub2 = align_up(d);
     z.ub2e = align_up(e);
   }
-  if (wp) {
+  if (wp > 32) {
+    size_t b[4];
+    oz3_bytes((int)W, (int)K, (int)B, b);
+    z.m0s = align_up(b[0]);
+    z.m0e = align_up(b[1]);
+    z.ub2 = align_up(b[2]);
+    z.ub2e = align_up(b[3]);
+  } else if (wp) {
     size_t d = 0, e = 0;
     oz_preslice_bytes(wp, (int)K, (int)B, &d, &e);
     z.m0s = align_up(d);
@@ -465,7 +477,12 @@ int Engine::alloc(std::string& err) {
   for (const auto& s : specs_) tensor_exp_ = tensor_exp_ && s.tensor_exp;
   pipe_ = tensor_wp_ != 0 && tensor_wp_ <= 32;
   for (const auto& s : specs_) pipe_ = pipe_ && s.mupdate_pipe;
-  if (tensor_wp_) W90G_CHECK(pipe_ ? oz2_set_attributes(tensor_wp_) : oz_set_attributes(tensor_wp_));
+  tiles3_ = 0;
+  if (tensor_wp_ > 32)
+    for (const auto& s : specs_) tiles3_ = std::max(tiles3_, oz3_tiles(s.W, s.B));
+  if (tensor_wp_)
+    W90G_CHECK(tiles3_ ? oz3_set_attributes(tensor_wp_)
+                       : (pipe_ ? oz2_set_attributes(tensor_wp_) : oz_set_attributes(tensor_wp_)));
   exp_smem_ = tensor_exp_ && tensor_wp_ == 32;
   for (const auto& s : specs_) exp_smem_ = exp_smem_ && s.exp_smem;
   if (tensor_exp_) W90G_CHECK(oz_exp_set_attributes(tensor_wp_, exp_smem_ ? 1 : 0));
@@ -669,8 +686,9 @@ int Engine::prepare_tensor(cudaStream_t st, std::string& err) {
   k_frob0<<<n_kb_, 128, 0, st>>>(dprobs_, wmkb);
   W90G_CHECK(cudaGetLastError());
   // step 1's A operand (the entry overlaps) in digit planes, once per solve
-  W90G_CHECK(pipe_ ? oz2_preslice_launch(tensor_wp_, dprobs_, wmk, n_k_, st)
-                  : oz_preslice_launch(tensor_wp_, dprobs_, wmk, n_k_, st));
+  W90G_CHECK(tiles3_ ? oz3_preslice_launch(tensor_wp_, dprobs_, wmk, n_k_, tiles3_, st)
+                    : (pipe_ ? oz2_preslice_launch(tensor_wp_, dprobs_, wmk, n_k_, st)
+                             : oz_preslice_launch(tensor_wp_, dprobs_, wmk, n_k_, st)));
   launches_ += 3;
   return 0;
 }
@@ -679,7 +697,9 @@ void Engine::launch_mupdate(cudaStream_t s, int which) {
   const int np = nprob();
   const WorkMap wmk{d_offs_k_, np};
   const WorkMap wmkb{d_offs_kb_, np};
-  if (pipe_) {
+  if (tiles3_) {
+    oz3_launch(tensor_wp_, dprobs_, wmk, which, n_k_, tiles3_, s);
+  } else if (pipe_) {
     oz2_launch(tensor_wp_, 1, dprobs_, wmk, which, n_k_, s);
     oz2_launch(tensor_wp_, 2, dprobs_, wmk, which, n_k_, s);
   } else if (tensor_wp_) {
@@ -766,7 +786,7 @@ int Engine::advance(int n, int* d_flag, std::string& err) {
   n = std::min(n, max_iter_ - launched_iters_);
   for (int i = 0; i < n; ++i) W90G_CHECK(cudaGraphLaunch(graph_exec_, st));
   // grad, search, 2 x (exp, M update, 2 spread passes), step, end (+ 2 precond)
-  launches_ += (10LL + 2 * (tensor_wp_ ? 2 : 1) + (pc_tiles_ ? 2 : 0) + (guide_w_ ? 1 : 0) + (n_ir_ ? 2 : 0)) *
+  launches_ += (10LL + 2 * (tiles3_ ? 3 : (tensor_wp_ ? 2 : 1)) + (pc_tiles_ ? 2 : 0) + (guide_w_ ? 1 : 0) + (n_ir_ ? 2 : 0)) *
                 std::max(n, 0);
   launched_iters_ += std::max(n, 0);
   if (d_flag) {

@@ -28,13 +28,11 @@
 // Every wait is bounded (W90G_SPIN_LIMIT tries) and also gives up when another role has
 // failed; a failed CTA then waits (W90G_DRAIN_LIMIT) for the MMAs it issued and the bulk
 // copies in flight before it frees tensor memory, and reports error 2 for the problem.
-#include "oz.cuh"
+#include "oz_pipe.cuh"
 
 namespace w90g {
 
 namespace {
-
-constexpr int kDynBudget = 232448 - 5120;                 // opt-in smem minus static use and slack
 
 // Warp roles per step: 16 epilogue warps (4 per TMEM lane quarter) share the exact
 // recombination; the producer is split into an A producer, which fills the ring of K-step
@@ -77,44 +75,6 @@ struct MU2 {
   static_assert(NS >= 2, "shared memory for at least two A stages");
   static constexpr size_t BYTES = (size_t)NS * STAGE + 2 * (size_t)B_BYTES + 1024;
 };
-
-// element (r, q) of a 128 x 16 K-major stage plane (canonical layout, no swizzle):
-// core matrices of 8 rows x 8 K (16 B rows), LBO 128 B along K, SBO 256 B along rows
-__device__ __forceinline__ uint32_t stage_off(int r, int q) {
-  return (uint32_t)((r >> 3) * 256 + (q >> 3) * 128 + (r & 7) * 16 + (q & 7) * 2);
-}
-
-__device__ __forceinline__ void bar_named(int id, int n) {
-  asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(n) : "memory");
-}
-
-// bounded wait that also stops when another role reported a failure (*bad != 0)
-__device__ __forceinline__ bool mbar_wait_role(uint32_t addr, uint32_t parity, volatile int* bad) {
-  for (int it = 0; it < W90G_SPIN_LIMIT; ++it) {
-    if (mbar_try(addr, parity)) return true;
-    if ((it & 63) == 63 && *bad) return false;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(b)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" :: "r"(smem_u32(b)) : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* b) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-               :: "r"(smem_u32(b)) : "memory");
-}
-
-// the group's skip predicate, read alike by every role (nothing writes it during the kernel)
-__device__ __forceinline__ bool group_active(const Problem& P, int which) {
-  const CtrlState* st = P.st;
-  return !st->done && !(which == 1 && !st->do_second);
-}
 
 template <int WP>
 __device__ __forceinline__ int ntiles_of(int B) {
@@ -698,17 +658,6 @@ __global__ void __launch_bounds__(256) k_oz_preslice2(const Problem* __restrict_
 
 // ---- host side ----------------------------------------------------------------------
 namespace {
-
-int sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) !=
-                                                  cudaSuccess || n <= 0)
-      n = 148;
-  }
-  return n;
-}
 
 template <int WP>
 cudaError_t launch2_wp(int step, const Problem* probs, WorkMap wm, int which, int ngroups, cudaStream_t s) {

@@ -421,8 +421,6 @@ cudaError_t oz_preslice_launch(int wp, const Problem* probs, WorkMap wm, int gri
     case 8: k_oz_preslice<8><<<grid, 256, 0, s>>>(probs, wm); break;
     case 16: k_oz_preslice<16><<<grid, 256, 0, s>>>(probs, wm); break;
     case 32: k_oz_preslice<32><<<grid, 256, 0, s>>>(probs, wm); break;
-    case 64: k_oz_preslice<64><<<grid, 256, 0, s>>>(probs, wm); break;
-    case 128: k_oz_preslice<128><<<grid, 256, 0, s>>>(probs, wm); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -444,8 +442,7 @@ cudaError_t oz_launch(int wp, int step, const Problem* probs, WorkMap wm, int wh
     case 8: return oz_launch_wp<8>(step, probs, wm, which, grid, s);
     case 16: return oz_launch_wp<16>(step, probs, wm, which, grid, s);
     case 32: return oz_launch_wp<32>(step, probs, wm, which, grid, s);
-    case 64: return oz_launch_wp<64>(step, probs, wm, which, grid, s);
-    default: return oz_launch_wp<128>(step, probs, wm, which, grid, s);
+    default: return cudaErrorInvalidValue;
   }
 }
 
@@ -462,18 +459,7 @@ cudaError_t oz_set_attributes(int wp) {
     case 8: return oz_attr_wp<8>();
     case 16: return oz_attr_wp<16>();
     case 32: return oz_attr_wp<32>();
-    case 64: return oz_attr_wp<64>();
-    default: return oz_attr_wp<128>();
-  }
-}
-
-size_t oz_smem_bytes(int wp) {
-  switch (wp) {
-    case 8: return TileSmem<8>::BYTES;
-    case 16: return TileSmem<16>::BYTES;
-    case 32: return TileSmem<32>::BYTES;
-    case 64: return TileSmem<64>::BYTES;
-    default: return TileSmem<128>::BYTES;
+    default: return cudaErrorInvalidValue;
   }
 }
 
