@@ -36,7 +36,6 @@ __global__ void k_all_done(const Problem* probs, int nprob, int* out);
 __global__ void k_fp64_peak(double* out, int iters, double seed);
 __global__ void k_u_final(const Problem* probs, WorkMap wm);
 __global__ void k_u_identity(const Problem* probs, WorkMap wm);
-__global__ void k_frob0(const Problem* probs, WorkMap wm);
 __global__ void k_precond(const Problem* probs, int dir);
 __global__ void k_phases(const Problem* probs, int mode);
 // kernels (k_sitesym.cu)
@@ -193,6 +192,17 @@ int choose_tensor_wp(const std::vector<ProblemSpec>& specs) {
   return wmax <= 8 ? 8 : (wmax <= 16 ? 16 : (wmax <= 32 ? 32 : (wmax <= 64 ? 64 : 128)));
 }
 
+// chunks of the spread passes: at most 64 blocks each, and down to 16 while that gives every SM
+// one (64 alone left 100 of the SMs idle on 3072 blocks of num_wann 128: 55 us against 20)
+int omega_chunks(const ProblemSpec& s) {
+  const int KB = s.K * s.B;
+  return std::max((KB + 63) / 64, std::min((KB + 15) / 16, 152));
+}
+
+// partial off-diagonal sums per (k,b) that the tensor M update's epilogue writes: one per column
+// group, and for num_wann > 32 per 32-row piece of the block (k_mupdate3.cu)
+int odn_of(int W) { return W <= 32 ? 4 : 4 * (W / 32 + 2); }
+
 struct Sizes {
   size_t M, U, KWW, work, tbuf, diag, offd, gpart, cen, log, logc, nn, bk, wb, st, op1, op2, m0, u0, inv, fr;
   size_t m0s, m0e, zexp, ub2, ub2e;
@@ -222,7 +232,7 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
   z.m0 = wp ? align_up(K * B * WW * 16) : 0;
   z.u0 = wp ? align_up(K * WW * 16) : 0;
   z.inv = wp ? align_up(K * B * 4) : 0;
-  z.fr = wp ? align_up(K * B * 8) : 0;
+  z.fr = wp ? align_up(K * B * odn_of(s.W) * 8) : 0;
   z.m0s = z.m0e = 0;
   z.zexp = (wp && wp <= 32) ? align_up(K * B * W * 4) : 0;
   z.ub2 = z.ub2e = 0;
@@ -255,7 +265,7 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
   z.bk = align_up(K * B * 3 * 8);
   z.wb = align_up(B * 8);
   z.st = align_up(sizeof(CtrlState));
-  const size_t nch = (K * B + 63) / 64;
+  const size_t nch = omega_chunks(s);
   z.op1 = align_up(nch * (4 * W + 2) * 8);
   z.op2 = align_up(nch * 8);
   z.pkr = z.pr2 = z.pgr = z.pgp = z.ppart = 0;
@@ -329,7 +339,7 @@ int Engine::alloc(std::string& err) {
     offs_k[p + 1] = offs_k[p] + s.K;
     offs_kb[p + 1] = offs_kb[p] + s.K * s.B;
     offs_grad[p + 1] = offs_grad[p] + s.K * nt * nt;
-    offs_chunk[p + 1] = offs_chunk[p] + (s.K * s.B + 63) / 64;
+    offs_chunk[p + 1] = offs_chunk[p] + omega_chunks(s);
     offs_ir[p + 1] = offs_ir[p] + s.sym_nir;
     if (s.W <= 32) maxW_small_ = std::max(maxW_small_, s.W);
     max_iter_ = std::max(max_iter_, s.ctl.num_iter);
@@ -394,7 +404,8 @@ int Engine::alloc(std::string& err) {
     int* inv = z.inv ? (int*)take(z.inv) : nullptr;
     P.inv_nnlist = inv;
     P.tensor = tensor_wp_ ? 1 : 0;
-    P.frob0 = z.fr ? (double*)take(z.fr) : nullptr;
+    P.odpart = z.fr ? (double*)take(z.fr) : nullptr;
+    P.odn = odn_of(s.W);
     P.m0s = z.m0s ? (unsigned char*)take(z.m0s) : nullptr;
     P.m0s_exp = z.m0e ? (int*)take(z.m0e) : nullptr;
     P.zexp = z.zexp ? (int*)take(z.zexp) : nullptr;
@@ -410,7 +421,7 @@ int Engine::alloc(std::string& err) {
     }
     P.opart1 = (double*)take(z.op1);
     P.opart2 = (double*)take(z.op2);
-    P.nchunk = (s.K * s.B + 63) / 64;
+    P.nchunk = omega_chunks(s);
     P.ctl = s.ctl;
     W90G_CHECK(cudaMemcpyAsync(nn, s.nnlist.data(), s.nnlist.size() * sizeof(int), cudaMemcpyHostToDevice, stream()));
     W90G_CHECK(cudaMemcpyAsync(bk, s.bk.data(), s.bk.size() * sizeof(double), cudaMemcpyHostToDevice, stream()));
@@ -681,15 +692,13 @@ int Engine::prepare_tensor(cudaStream_t st, std::string& err) {
     W90G_CHECK(cudaMemcpyAsync(hprobs_[p].U0, hprobs_[p].U[0], (size_t)s.K * WW * 16, cudaMemcpyDeviceToDevice, st));
   }
   const WorkMap wmk{d_offs_k_, nprob()};
-  const WorkMap wmkb{d_offs_kb_, nprob()};
   k_u_identity<<<n_k_, 256, 0, st>>>(dprobs_, wmk);
-  k_frob0<<<n_kb_, 128, 0, st>>>(dprobs_, wmkb);
   W90G_CHECK(cudaGetLastError());
   // step 1's A operand (the entry overlaps) in digit planes, once per solve
   W90G_CHECK(tiles3_ ? oz3_preslice_launch(tensor_wp_, dprobs_, wmk, n_k_, tiles3_, st)
                     : (pipe_ ? oz2_preslice_launch(tensor_wp_, dprobs_, wmk, n_k_, st)
                              : oz_preslice_launch(tensor_wp_, dprobs_, wmk, n_k_, st)));
-  launches_ += 3;
+  launches_ += 2;
   return 0;
 }
 

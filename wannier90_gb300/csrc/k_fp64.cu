@@ -97,13 +97,20 @@ __global__ void k_mdiag(const Problem* __restrict__ probs, WorkMap wm) {
 }
 
 // ----------------------------------------------------------------------------
-// wann_omega (src/wannierise.F90:1979-2284) as a deterministic three-pass reduction
-// over chunks of kOmegaChunk (k,b) blocks:
+// wann_omega (src/wannierise.F90:1979-2284) as a deterministic two-pass reduction over
+// nchunk chunks of consecutive (k,b) blocks (at most kOmegaChunk each; the engine makes as many
+// chunks of at least 16 blocks as the chip has SMs):
 //   p1: per chunk  P_n = sum wb b ln_n (3W), q_n = sum wb (1 - |M_nn|^2 + ln_n^2) (W),
-//       sum wb offd, and (first pass only) sum wb (W - sum|M|^2)
-//   p2: rave = -(1/K) sum_chunks P (same fixed order in every CTA), then the chunk's
-//       part of sum wb (ln_n + b.rave_n)^2
-//   p3: one CTA per problem: totals, centres, spreads, Omega terms.
+//       sum wb offd, and (first pass only) sum wb (W - sum|M|^2); the last CTA: totals, centres,
+//       spreads;
+//   p2: the chunk's part of sum wb (ln_n + b.rave_n)^2; the last CTA: the Omega terms.
+// Both are latency bound: a few FP64 operations per statistic, so what counts is the chain of
+// barriers and dependent loads.  The four sums of p1 meet in shared memory behind one barrier,
+// the off-diagonal sum takes all threads, and a last CTA reads the chunk partials sixteen loads
+// at a time into four accumulators.
+// On the tensor path the off-diagonal sums come from the M update's epilogue (odpart), summed
+// there directly: |M0|_F^2 minus the diagonal, which they replace, cancels to ~1e-14 of num_wann
+// and near a minimum hid the trial step's change from the parabola.
 // Selective localisation (slwf_num = s > 0, :2144-2211): p1's off-diagonal slot holds
 // sum over n < s of wb (1 - |M_nn|^2 + lambda ln_n^2) (Omega_IOD) and its Omega_I slot
 // sum over n < s of 2 wb lambda ln_n (b.c_n) (the k-sum of Omega_nu); p2 sums over n < s
@@ -145,7 +152,8 @@ __global__ void __launch_bounds__(256) k_omega_p1(const Problem* __restrict__ pr
   if (omega_skip(st, slot)) return;
   const int W = P.W, B = P.B;
   const int KB = P.K * B;
-  const int kb0 = ch * kOmegaChunk, kb1 = min(KB, kb0 + kOmegaChunk);
+  const int per = (KB + P.nchunk - 1) / P.nchunk;
+  const int kb0 = ch * per, kb1 = min(KB, kb0 + per);
   const int t = threadIdx.x;
   const int nsub = blockDim.x / W;           // W <= 256
   const int n = t % W, sub = t / W;
@@ -161,6 +169,7 @@ __global__ void __launch_bounds__(256) k_omega_p1(const Problem* __restrict__ pr
     c2 = P.slwf_c[2 * W + n];
   }
   if (act) {
+#pragma unroll 4
     for (int kb = kb0 + sub; kb < kb1; kb += nsub) {
       const double w = P.wb[kb % B];
       const double l = P.diag_ln[(size_t)kb * W + n];
@@ -179,16 +188,16 @@ __global__ void __launch_bounds__(256) k_omega_p1(const Problem* __restrict__ pr
     }
   }
   double* out = P.opart1 + (size_t)ch * (4 * W + 2);
-  const double vals[4] = {r0, r1, r2, q};
-  for (int c = 0; c < 4; ++c) {
-    red[t] = act ? vals[c] : 0.0;
-    __syncthreads();
-    if (t < W) {
-      double sacc = 0.0;
-      for (int u = 0; u < nsub; ++u) sacc += red[u * W + t];
-      out[c * W + t] = sacc;
-    }
-    __syncthreads();
+  __shared__ double s_sum[4][256];
+  s_sum[0][t] = act ? r0 : 0.0;
+  s_sum[1][t] = act ? r1 : 0.0;
+  s_sum[2][t] = act ? r2 : 0.0;
+  s_sum[3][t] = act ? q : 0.0;
+  __syncthreads();
+  for (int i = t; i < 4 * W; i += blockDim.x) {
+    double sacc = 0.0;
+    for (int u = 0; u < nsub; ++u) sacc += s_sum[i / W][u * W + i % W];
+    out[i] = sacc;
   }
   if (P.slwf_num > 0) {
     // Omega_IOD in the off-diagonal slot, the k-sum of Omega_nu in the Omega_I slot
@@ -200,43 +209,51 @@ __global__ void __launch_bounds__(256) k_omega_p1(const Problem* __restrict__ pr
     }
   } else {
     const bool first = (slot == 2) && st->first_pass;
+    const bool parts = P.tensor && slot < 2;   // partials of the tensor M update's epilogue
     double od = 0.0, oi = 0.0;
-    for (int kb = kb0 + t; kb < kb1; kb += blockDim.x) {
+    // tpk threads share one block (k,b)
+    int tpk = 1;
+    while (2 * tpk * per <= (int)blockDim.x && tpk < 32) tpk *= 2;
+    const int sl = t % tpk;
+    for (int kb = kb0 + t / tpk; kb < kb1; kb += blockDim.x / tpk) {
       const double w = P.wb[kb % B];
-      double o;
-      if (P.tensor && slot < 2) {
-        // tensor path: |M(k,b)|_F^2 is invariant under the unitary rotation, so the
-        // off-diagonal sum is |M0(k,b)|_F^2 minus the diagonal (src/wannierise.F90:2214-2258)
-        double sd = 0.0;
-        for (int m = 0; m < W; ++m) sd += P.diag_abs2[(size_t)kb * W + m];
-        o = P.frob0[kb] - sd;
-      } else {
+      double o = 0.0;
+      if (parts) {
+        for (int i = sl; i < P.odn; i += tpk) o += P.odpart[(size_t)kb * P.odn + i];
+      } else if (sl == 0) {
         o = P.offd[kb];
       }
       od += w * o;
       if (first) {
         double sd = 0.0;
-        for (int m = 0; m < W; ++m) sd += P.diag_abs2[(size_t)kb * W + m];
-        oi += w * ((double)W - (o + sd));
+        for (int m = sl; m < W; m += tpk) sd += P.diag_abs2[(size_t)kb * W + m];
+        oi += w * ((sl == 0 ? (double)W : 0.0) - (o + sd));
       }
     }
     od = block_sum(od, red);
-    oi = block_sum(oi, red);
+    if (first) oi = block_sum(oi, red);
     if (t == 0) {
       out[4 * W] = od;
       out[4 * W + 1] = oi;
     }
   }
   if (!last_chunk_cta(&st->omega_arrive[0], P.nchunk)) return;
-  // ---- the last CTA: every chunk sum in chunk order on its own thread -- rave (3W) into
+  // ---- the last CTA: every chunk sum on its own thread, in a fixed order -- rave (3W) into
   // the slot's centres, r^2 (W) into its spreads, the Omega_OD and Omega_I totals (2)
   double* cen = P.centres + (size_t)slot * 4 * W;
   const int stride = 4 * W + 2;
   __shared__ double s_rave[3 * 256];
   __shared__ double s_q[256];
   for (int i = t; i < 4 * W + 2; i += blockDim.x) {
-    double sacc = 0.0;
-    for (int c = 0; c < P.nchunk; ++c) sacc += __ldcg(P.opart1 + (size_t)c * stride + i);
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* src = P.opart1 + i;
+    int c = 0;
+#pragma unroll 4
+    for (; c + 4 <= P.nchunk; c += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a[u] += __ldcg(src + (size_t)(c + u) * stride);
+    for (; c < P.nchunk; ++c) a[0] += __ldcg(src + (size_t)c * stride);
+    const double sacc = (a[0] + a[1]) + (a[2] + a[3]);
     if (i < 3 * W) s_rave[i] = -sacc / (double)P.K;
     else if (i < 4 * W) s_q[i - 3 * W] = sacc;
     else st->omega_tot[i - 4 * W] = sacc;
@@ -261,7 +278,8 @@ __global__ void __launch_bounds__(256) k_omega_p2(const Problem* __restrict__ pr
   if (omega_skip(st, slot)) return;
   const int W = P.W, B = P.B, K = P.K;
   const int KB = K * B;
-  const int kb0 = ch * kOmegaChunk, kb1 = min(KB, kb0 + kOmegaChunk);
+  const int per = (KB + P.nchunk - 1) / P.nchunk;
+  const int kb0 = ch * per, kb1 = min(KB, kb0 + per);
   const int t = threadIdx.x;
   const int nsub = blockDim.x / W;
   const int n = t % W, sub = t / W;
@@ -271,6 +289,7 @@ __global__ void __launch_bounds__(256) k_omega_p2(const Problem* __restrict__ pr
   // selective localisation: Omega_D over the objective WFs only
   if (sub < nsub && (P.slwf_num == 0 || n < P.slwf_num)) {
     const double x0 = cen[n], x1 = cen[W + n], x2 = cen[2 * W + n];
+#pragma unroll 4
     for (int kb = kb0 + sub; kb < kb1; kb += nsub) {
       const double w = P.wb[kb % B];
       const double* bv = P.bk + (size_t)kb * 3;
@@ -281,10 +300,11 @@ __global__ void __launch_bounds__(256) k_omega_p2(const Problem* __restrict__ pr
   dd = block_sum(dd, red);
   if (t == 0) P.opart2[ch] = dd;
   if (!last_chunk_cta(&st->omega_arrive[1], P.nchunk)) return;
-  // ---- the last CTA: the Omega_D total in chunk order, then the spread of the slot
+  // ---- the last CTA: the Omega_D total, then the spread of the slot
+  double acc = 0.0;
+  for (int c = t; c < P.nchunk; c += blockDim.x) acc += __ldcg(P.opart2 + c);
+  acc = block_sum(acc, red);
   if (t == 0) {
-    double acc = 0.0;
-    for (int c = 0; c < P.nchunk; ++c) acc += __ldcg(P.opart2 + c);
     const double od = st->omega_tot[0], oi = st->omega_tot[1], dsum = acc;
     Spread sp;
     if (P.slwf_num > 0) {
@@ -1451,22 +1471,6 @@ __global__ void __launch_bounds__(256) k_u_final(const Problem* __restrict__ pro
   cta_gemm<false>(sC, W, sA, W, sR, W, W);
   __syncthreads();
   for (int e = threadIdx.x; e < WW; e += blockDim.x) R[e] = sC[e];
-}
-
-// ----------------------------------------------------------------------------
-// k_frob0: |M0(k,b)|_F^2 per block (tensor path, once per solve).  One CTA per (k,b).
-// ----------------------------------------------------------------------------
-__global__ void k_frob0(const Problem* __restrict__ probs, WorkMap wm) {
-  __shared__ double red[128];
-  int kb;
-  const int p = locate(wm, blockIdx.x, kb);
-  const Problem& P = probs[p];
-  const int W = P.W;
-  const double2* Mb = P.M0 + (size_t)kb * W * W;
-  double acc = 0.0;
-  for (int e = threadIdx.x; e < W * W; e += blockDim.x) acc += cabs2(Mb[e]);
-  acc = block_sum(acc, red);
-  if (threadIdx.x == 0) P.frob0[kb] = acc;
 }
 
 }  // namespace w90g

@@ -1,6 +1,6 @@
 // Tensor-core M update for num_wann <= 32, pipelined: M(k,b) = U(k)^H M0(k,b) U(k+b).
 //
-// The arithmetic is k_tensor.cu's (real embedding, 7 signed 7-bit FP16 digits per
+// The arithmetic is k_tensor.cu's (real embedding, 7 signed 8-bit FP16 digits per
 // operand, the 28 digit pairs of the 7 diagonals accumulated exactly in FP32 TMEM
 // columns, exact int64 recombination), so results are bitwise those of k_oz_mupdate;
 // only the schedule differs.  One persistent CTA per SM walks the work units
@@ -79,20 +79,6 @@ struct MU2 {
 template <int WP>
 __device__ __forceinline__ int ntiles_of(int B) {
   return (B * WP + kTileRows - 1) / kTileRows;
-}
-
-// S = sum_d D_d 2^(7(6-d)) of the 7 diagonal accumulators dd[0], dd[stride], ... (exact
-// integers |D_d| < 2^22 held in FP32), exactly.  b_d = bits(D_d + 1.5 * 2^23) = D_d +
-// 0x4B400000, and S = 2^21 H + L with H = sum_{d<=3} D_d 2^(7(3-d)), L = sum_{d>=4}
-// D_d 2^(7(6-d)): each a sum of widened 32 x 32-bit products with the bias folded into
-// one constant.  The same integer as the Horner form (acc << 7) + D_d of k_tensor.cu.
-__device__ __forceinline__ long long recombine7_exact(const uint32_t* dd, int stride) {
-  long long b[kDiag];
-#pragma unroll
-  for (int d = 0; d < kDiag; ++d) b[d] = (long long)__float_as_int(__uint_as_float(dd[d * stride]) + 12582912.0f);
-  const long long H = b[0] * (1LL << 21) + b[1] * (1LL << 14) + b[2] * 128LL + b[3] - 0x4B400000LL * 2113665LL;
-  const long long L = b[4] * (1LL << 14) + b[5] * 128LL + b[6] - 0x4B400000LL * 16513LL;
-  return H * (1LL << 21) + L;
 }
 
 }  // namespace
@@ -250,7 +236,7 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
               const int it = pa + j * R::PAT;
               if (it < R::AITEMS) {
                 uint32_t w[kS][4];
-                pack_digits7(w, av[j], zex[j], false);
+                slice_run8_h(w, av[j], zex[j]);
                 const uint32_t o = stage_off(it % kTileRows, 8 * (it / kTileRows));
 #pragma unroll
                 for (int t = 0; t < kS; ++t)
@@ -349,11 +335,11 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
           v[i] = 0.0;
           if (cc < W && mm < W) {
             const double2 u = Ug[(size_t)cc * W + mm];
-            v[i] = part == 0 ? u.x : -u.y;     // step 1: B = conj(U)
+            v[i] = part == 0 ? u.x : u.y;
           }
         }
         uint32_t w[kS][4];
-        pack_digits7(w, v, ec, false);
+        slice_run8_h(w, v, ec);
         const int k_re = g8 * 16, k_im = k_re + 8;   // K positions of Re / Im of m = 8 g8 ..
         if (part == 0) {
           const uint32_t o_rr = kmaj_off(cc, k_re, KC), o_ii = kmaj_off(CW + cc, k_im, KC);
@@ -369,21 +355,19 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
             }
           }
         } else {
-          // B_i = -Im U (step 1) to (N im, K re) -- for step 2 (B_i = Im U) the same digits
-          // go to (N re, K im) -- and -B_i = Im U to (N re, K im), for step 2 to (N im, K re)
+          // step 1 (B = conj(U)): B_i = -Im U to (N im, K re) and -B_i = Im U to (N re, K im);
+          // step 2's image the other way round
           const uint32_t o_ir = kmaj_off(CW + cc, k_re, KC), o_ri = kmaj_off(cc, k_im, KC);
 #pragma unroll
           for (int t = 0; t < kS; ++t) {
             const uint4 q = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
-            *(uint4*)(dB + (size_t)t * L::B_PLANE + o_ir) = q;
-            if (gB) *(uint4*)(gB + (size_t)t * L::B_PLANE + o_ri) = q;
-          }
-          pack_digits7(w, v, ec, true);
-#pragma unroll
-          for (int t = 0; t < kS; ++t) {   // the digits of the negated values
-            const uint4 q = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
+            const uint4 n = make_uint4(f16x2_neg(w[t][0]), f16x2_neg(w[t][1]), f16x2_neg(w[t][2]), f16x2_neg(w[t][3]));
             *(uint4*)(dB + (size_t)t * L::B_PLANE + o_ri) = q;
-            if (gB) *(uint4*)(gB + (size_t)t * L::B_PLANE + o_ir) = q;
+            *(uint4*)(dB + (size_t)t * L::B_PLANE + o_ir) = n;
+            if (gB) {
+              *(uint4*)(gB + (size_t)t * L::B_PLANE + o_ir) = q;
+              *(uint4*)(gB + (size_t)t * L::B_PLANE + o_ri) = n;
+            }
           }
         }
       }
@@ -528,7 +512,7 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
         for (int j = 0; j < CPG; ++j) ecol[j] = s_colexp[bb][jbeg + j];
         if (tile == ntiles - 1) mbar_arrive(&b_empty[bb]);   // colexp read: B may be replaced
         const uint32_t acc = tmem + (uint32_t)(a * L::ACC_COLS);
-        double dre = 0.0, dim = 0.0;
+        double dre = 0.0, dim = 0.0, od = 0.0;
         bool has_diag = false;
 #pragma unroll 1
         for (int j0 = jbeg; j0 < jbeg + CPG; j0 += 2) {
@@ -547,8 +531,8 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
           for (int j = 0; j < 2; ++j) {
             const int c = j0 + j;   // complex output column
             const int e = erow + ecol[c - jbeg];
-            const double re = int64_scaled_to_double(recombine7_exact(&q[0][j], 2), e - 56);
-            const double im = int64_scaled_to_double(recombine7_exact(&s2[0][j], 2), e - 56);
+            const double re = int64_scaled_to_double(recombine8_exact<KC>(&q[0][j], 2), e - 56);
+            const double im = int64_scaled_to_double(recombine8_exact<KC>(&s2[0][j], 2), e - 56);
             if (STEP == 1) {
               // step 2's row scale of row c of Z(k,b): the largest |re|, |im| over this
               // block's rows rr, i.e. over its WP lanes (segmented max; zero rows add 0).
@@ -570,12 +554,21 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
                 dre = re;
                 dim = im;
                 has_diag = true;
+              } else {
+                od = fma(re, re, od);
+                od = fma(im, im, od);
               }
             }
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive(&acc_empty[a]);
+        if (STEP == 2) {
+          // the block's off-diagonal sum over this warp's columns: its WP lanes
+#pragma unroll
+          for (int o = 1; o < WP && o < 32; o <<= 1) od += __shfl_xor_sync(0xffffffffu, od, o);
+          if (rr == 0 && bi < B) P.odpart[(size_t)kb_out * 4 + cg] = od;
+        }
         if (STEP == 2 && has_diag) {
           P.diag_ln[(size_t)kb_out * W + rr] = guided_ln(P, (size_t)kb_out * W + rr, make_double2(dre, dim));
           P.diag_abs2[(size_t)kb_out * W + rr] = dre * dre + dim * dim;
@@ -634,23 +627,23 @@ __global__ void __launch_bounds__(256) k_oz_preslice2(const Problem* __restrict_
     if (tid < kTileRows) P.m0s_exp[((size_t)g * ntiles + tile) * kTileRows + tid] = s_rowexp[tid];
     for (int ks = 0; ks < KSTEPS; ++ks) {
       unsigned char* dst = P.m0s + (((size_t)g * ntiles + tile) * KSTEPS + ks) * (size_t)L::STAGE;
-      for (int e = tid; e < kTileRows * 8; e += blockDim.x) {
-        const int r = e >> 3, l = e & 7;
-        const int row = tile * kTileRows + r;
-        const int bi = row / WP, rr = row % WP;
-        const int m = ks * 8 + l;
-        double2 a = make_double2(0.0, 0.0);
-        if (bi < B && rr < W && m < W) a = P.M0[((size_t)g * B + bi) * WW + (size_t)rr * W + m];
-        int xr[kS], xi[kS];
-        digits7(scaled_int(a.x, s_rowexp[r]), xr);
-        digits7(scaled_int(a.y, s_rowexp[r]), xi);
-        const uint32_t o = stage_off(r, l);
+      // a thread slices one part of a row's 8 complex: one 16-byte core row per plane
+      const int r = tid % kTileRows, part = tid / kTileRows;
+      const int row = tile * kTileRows + r, bi = row / WP, rr = row % WP;
+      double v[8];
 #pragma unroll
-        for (int t = 0; t < kS; ++t) {
-          *(uint16_t*)(dst + (size_t)t * L::PLANE + o) = int_to_f16(xr[t]);
-          *(uint16_t*)(dst + (size_t)t * L::PLANE + o + 128) = int_to_f16(xi[t]);
-        }
+      for (int i = 0; i < 8; ++i) {
+        const int m = ks * 8 + i;
+        v[i] = 0.0;
+        if (bi < B && rr < W && m < W)
+          v[i] = ((const double*)(P.M0 + ((size_t)g * B + bi) * WW + (size_t)rr * W + m))[part];
       }
+      uint32_t w[kS][4];
+      slice_run8_h(w, v, s_rowexp[r]);
+      const uint32_t o = stage_off(r, 8 * part);
+#pragma unroll
+      for (int t = 0; t < kS; ++t)
+        *(uint4*)(dst + (size_t)t * L::PLANE + o) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
     }
     __syncthreads();
   }

@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
       }
       double2* dst = (STEP == 1 ? P.tbuf : P.M[cur ^ 1]) + kb * WW + rr;
       const int* ecol = P.ub2_exp + (size_t)g * W;
+      double od = 0.0;   // step 2: |M_mn|^2 off the diagonal, this row and column group
       for (int nc = 0; nc < G.nch; ++nc) {
         if (!await(&acc_full, (uint32_t)useq & 1, p)) {
           ok = false;
@@ -399,10 +400,15 @@ __global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
               double im = recombine3<EIGHT>(&s2[0][j], 2, e);
               if (STEP == 1) im = -im;          // the product is conj(Z)
               dst[(size_t)c * W] = make_double2(re, im);
-              if (STEP == 2 && c == rr) {
-                dre = re;
-                dim = im;
-                has_diag = true;
+              if (STEP == 2) {
+                if (c == rr) {
+                  dre = re;
+                  dim = im;
+                  has_diag = true;
+                } else {
+                  od = fma(re, re, od);
+                  od = fma(im, im, od);
+                }
               }
             }
           }
@@ -414,6 +420,25 @@ __global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
           P.diag_abs2[kb * W + rr] = dre * dre + dim * dim;
         }
         ++useq;
+      }
+      if (STEP == 2 && ok) {
+        // The off-diagonal sums of the warp's 32 rows, which lie in one block or two (num_wann >
+        // 32): piece (row / 32 - first row of the block / 32) of the block and column group cg.
+        // The warp with a block's last row clears the pieces its position leaves unused.
+        const int row0 = tile * kTileRows + wq * 32, b0 = row0 / W;
+        for (int b = b0; b <= b0 + 1 && b < P.B; ++b) {
+          double x = valid && bi == b ? od : 0.0;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+          const int first = b * W / 32, last = (b * W + W - 1) / 32;
+          if (row0 + 31 < b * W) break;
+          if (lane == 0) {
+            double* dp = P.odpart + (size_t)P.inv_nnlist[(size_t)g * P.B + b] * P.odn + cg;
+            dp[(row0 / 32 - first) * 4] = x;
+            if (row0 / 32 == last)
+              for (int i = last - first + 1; i < P.odn / 4; ++i) dp[i * 4] = 0.0;
+          }
+        }
       }
       ++tseq;
     }

@@ -1,16 +1,17 @@
-// Tensor-core M update: M(k,b) = U(k)^H M0(k,b) U(k+b) with FP64-level accuracy from
+// Tensor-core M update: M(k,b) = U(k)^H M0(k,b) U(k+b) with FP64 accuracy from
 // FP16 tcgen05 MMAs (Ozaki-style exact slicing).
 //
 // Every complex product is computed through its real embedding
 //     [C_r C_i] = [A_r A_i] [[B_r, B_i], [-B_i, B_r]]      (K = N = 2*WP real)
 // Each operand is scaled per row (A) / per column (B) by a power of two and split into
-// S = 7 signed 7-bit digits (x_1 in [-128,128], x_t in [-64,63] for t > 1), each an exact
-// FP16 value (built two at a time by a packed FP16 subtraction, pack_digits7).  For every digit pair (t,u) with t+u <= S-1 (0-based) the MMA A^(t) B^(u)
-// over the K = 2*WP reduction is exact in the FP32 accumulator (every partial sum is an
-// integer below 2^22), so the pairs of one diagonal d = t+u share one TMEM accumulator.
-// The epilogue recombines the 7 diagonals exactly in int64 and rounds once to FP64.
-// Truncation error: ~2^-49 relative to (row scale x column scale) per product term.
-// Widths up to 128 are handled by chunking K and N in 32-complex-column pieces.
+// S = 7 signed 8-bit digits (|x| <= 128), each an exact FP16 value (built two at a time by a
+// packed FP16 subtraction, slice_run8_h).  For every digit pair (t,u) with t+u <= S-1 (0-based)
+// the MMA A^(t) B^(u) over the K = 2*WP <= 64 reduction is exact in the FP32 accumulator (every
+// partial sum is an integer below 2^23), so the pairs of one diagonal d = t+u share one TMEM
+// accumulator.  The epilogue recombines the 7 diagonals in int64 and rounds once to FP64.
+// Error: the digit pairs left out, ~2^-53 of (row scale x column scale).  (7-bit digits, whose
+// error is 2^-48, cost the same MMAs and more slicing.)  num_wann <= 32 here; the pipelined form
+// of the same arithmetic is k_mupdate2.cu, wider problems take k_mupdate3.cu.
 //
 // The product is batched as tall-skinny GEMMs (B*WP rows sharing one WP x WP operand):
 //   step 1 (group k):  rows (b, n):  Z(k,b)^T = M0(k,b)^T conj(U(k))   -> Z row-major
@@ -22,24 +23,6 @@
 #include "oz.cuh"
 
 namespace w90g {
-
-// Digit scheme: 7 signed 7-bit digits (49 bits).  (8-bit digits give 56 bits for the
-// same 28 MMAs but their wider exact recombination made the update 20% slower; the
-// update's ~2^-49 error stays far below what the line search resolves.)
-template <int WP>
-__device__ __forceinline__ void split_digits(double v, int e, int x[kS]) {
-  digits7(scaled_int(v, e), x);
-}
-
-// value of the 7 FP32 diagonal accumulators dd[0], dd[stride], ... for row / column
-// exponents summing to escale
-template <int WP>
-__device__ __forceinline__ double recombine_digits(const uint32_t* dd, int stride, int escale) {
-  long long acc = float_to_int_exact(__uint_as_float(dd[0]));
-#pragma unroll
-  for (int d = 1; d < kDiag; ++d) acc = (acc << 7) + float_to_int_exact(__uint_as_float(dd[d * stride]));
-  return int64_scaled_to_double(acc, escale - 56);
-}
 
 // Row exponents of A tile `tile` (2 threads per row, all 256 threads of the CTA).
 template <int WP, class AElem>
@@ -78,7 +61,7 @@ __device__ __forceinline__ void a_slice_chunk(unsigned char* dst, int tile, int 
       v[i] = part == 0 ? a.x : a.y;
     }
     uint32_t w[kS][4];
-    pack_digits7(w, v, rowexp[r], false);
+    slice_run8_h(w, v, rowexp[r]);
     const uint32_t o = kmaj_off(r, part * CW + lg * 8, KC);
 #pragma unroll
     for (int t = 0; t < kS; ++t)
@@ -169,12 +152,18 @@ __global__ void __launch_bounds__(256, 1) k_oz_mupdate(const Problem* __restrict
         v[i] = 0.0;
         if (cc < W && mm < W) {
           const double2 u = Ug[(size_t)cc * W + mm];
-          const double br = u.x, bi = (STEP == 1) ? -u.y : u.y;
-          v[i] = (kre && nre) ? br : (kre ? bi : (nre ? -bi : br));   // [B_r B_i; -B_i B_r]
+          v[i] = kre == nre ? u.x : u.y;    // [B_r B_i; -B_i B_r], the sign below
         }
       }
       uint32_t w[kS][4];
-      pack_digits7(w, v, s_colexp[cc < WP ? cc : 0], false);
+      slice_run8_h(w, v, s_colexp[cc < WP ? cc : 0]);
+      // (B = conj(U) in step 1, U in step 2; the digits are always Im U's, negated where needed)
+      if (STEP == 1 ? (kre && !nre) : (!kre && nre)) {
+#pragma unroll
+        for (int t = 0; t < kS; ++t)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) w[t][i] = f16x2_neg(w[t][i]);
+      }
       const uint32_t off = kmaj_off(n, kk0, KC);
 #pragma unroll
       for (int t = 0; t < kS; ++t)
@@ -313,7 +302,7 @@ __global__ void __launch_bounds__(256, 1) k_oz_mupdate(const Problem* __restrict
         int kb_out = 0;
         if (STEP == 2 && bi < B) kb_out = P.inv_nnlist[(size_t)g * B + bi];
         const int jbeg = half * (CW / 2), jend = jbeg + CW / 2;
-        double dre = 0.0, dim = 0.0;
+        double dre = 0.0, dim = 0.0, od[2] = {0.0, 0.0};   // od: per quarter of the columns
         bool has_diag = false;
 #pragma unroll 1
         for (int j0 = jbeg; j0 < jend; j0 += 4) {
@@ -333,10 +322,9 @@ __global__ void __launch_bounds__(256, 1) k_oz_mupdate(const Problem* __restrict
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int c = nc * CW + j0 + j;   // complex output column
-            // S = sum_d D_d 2^(7(6-d)) by Horner in int64 (exact, |S| < 2^63)
             const int ecol = s_colexp[c < WP ? c : 0];
-            const double re = recombine_digits<WP>(&q[0][j], 4, erow + ecol);
-            const double im = recombine_digits<WP>(&s4[0][j], 4, erow + ecol);
+            const double re = int64_scaled_to_double(recombine8_exact<KC>(&q[0][j], 4), erow + ecol - 56);
+            const double im = int64_scaled_to_double(recombine8_exact<KC>(&s4[0][j], 4), erow + ecol - 56);
             if (valid && c < W) {
               if (STEP == 1) {
                 // Z(k,b) row-major: element (j=c, n=rr) at c*W + rr
@@ -348,14 +336,26 @@ __global__ void __launch_bounds__(256, 1) k_oz_mupdate(const Problem* __restrict
                   dre = re;
                   dim = im;
                   has_diag = true;
+                } else {
+                  double& acc = (j0 + j - jbeg) < CW / 4 ? od[0] : od[1];
+                  acc = fma(re, re, acc);
+                  acc = fma(im, im, acc);
                 }
               }
             }
           }
         }
+        if (STEP == 2) {
+          // the block's off-diagonal sums over its WP lanes, as k_oz_mupdate2 forms them
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int o = 1; o < WP && o < 32; o <<= 1) od[h] += __shfl_xor_sync(0xffffffffu, od[h], o);
+            if (rr == 0 && bi < B) P.odpart[(size_t)kb_out * 4 + half * 2 + h] = od[h];
+          }
+        }
         if (STEP == 2 && has_diag) {
-          // diagonal statistics (once per row); the off-diagonal sum follows from the
-          // invariant |M(k,b)|_F^2 = |M0(k,b)|_F^2 in the spread pass
+          // diagonal statistics (once per row)
           P.diag_ln[(size_t)kb_out * W + rr] = guided_ln(P, (size_t)kb_out * W + rr, make_double2(dre, dim));
           P.diag_abs2[(size_t)kb_out * W + rr] = dre * dre + dim * dim;
         }

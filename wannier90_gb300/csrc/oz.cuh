@@ -194,6 +194,38 @@ __device__ __forceinline__ void pack_digits7(uint32_t (&w)[kS][4], const double 
   }
 }
 
+// The seven 8-bit digit planes of the 8 values scaled by 2^(55 - ex), as packed FP16
+// pairs: w[t][i / 2] holds digit t of values i (low half) and i + 1 -- the digits of
+// digits7x8, without its serial recoding.  With C = 128 (1 + 2^8 + ... + 2^40), byte t' of
+// N + C is digit 6 - t' plus 128 (adding 128 at every lower byte position turns the
+// centred digits into the plain bytes of N + C: x_6 = sext8(N mod 2^8) = byte0(N + 128) -
+// 128, and (N - x_6) / 2^8 = (N + 128) >> 8, so the next step repeats on N + 128 shifted),
+// and the top digit is (N + C) >> 48 (arithmetic), so b = digit + 128 lies in [0, 256].
+// With 0x6400 above it, b is the FP16 number 1024 + b: one byte permute, one mask and one
+// packed subtraction of 1152 give two digits.  Exact: FP16 holds the integers to 2048, and
+// the difference of two of them is rounded to itself.
+__device__ __forceinline__ void slice_run8_h(uint32_t (&w)[7][4], const double (&v)[8], int ex) {
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    const long long ma = scaled_int55(v[i], ex) + 0x808080808080LL;
+    const long long mb = scaled_int55(v[i + 1], ex) + 0x808080808080LL;
+    const uint32_t la = (uint32_t)ma, lb = (uint32_t)mb;
+    const uint32_t ha = (uint32_t)((unsigned long long)ma >> 32), hb = (uint32_t)((unsigned long long)mb >> 32);
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      const uint32_t bt = (uint32_t)(t & 3);
+      const uint32_t sel = bt | (bt << 4) | ((4u + bt) << 8) | ((4u + bt) << 12);
+      const uint32_t p = __byte_perm(t < 4 ? la : ha, t < 4 ? lb : hb, sel);
+      w[6 - t][i >> 1] = f16x2_sub((p & 0x00FF00FFu) | 0x64006400u, 0x64806480u);
+    }
+    const uint32_t ta = (uint32_t)((int)(ma >> 48) + 128), tb = (uint32_t)((int)(mb >> 48) + 128);
+    w[0][i >> 1] = f16x2_sub(ta | (tb << 16) | 0x64006400u, 0x64806480u);
+  }
+}
+
+// -x for both halves of a packed FP16 pair (a zero becomes -0, the same in every product)
+__device__ __forceinline__ uint32_t f16x2_neg(uint32_t w) { return w ^ 0x80008000u; }
+
 // exact integer value of an integer-valued float with |f| < 2^24
 __device__ __forceinline__ int float_to_int_exact24(float f) {
   return (fabsf(f) < 4194304.0f) ? float_to_int_exact(f) : __float2int_rn(f);
@@ -254,6 +286,25 @@ __device__ __forceinline__ double recombine7x8(const uint32_t* dd, int stride, i
 #pragma unroll
   for (int d = 5; d < 7; ++d) lo = (lo << 8) + float_to_int_exact24(__uint_as_float(dd[d * stride]));
   return int64_scaled_to_double(hi, sc + 24) + int64_scaled_to_double(lo, sc);
+}
+
+// S with C = S 2^(e-56) of the 7 diagonal accumulators dd[0], dd[stride], ... of an 8-bit-digit
+// product over K <= 64 real terms (the M update of num_wann <= 32; e the exponents' sum): D_0..D_3
+// at 2^(42-8d) plus (D_4 2^16 + D_5 2^8 + D_6) / 2^6 rounded, below 2^63 for any operands.  The last
+// bit weighs 2^(e-56); the digit pairs left out weigh ~2^(e-53).  |D_d| <= (d + 1) K 2^14 is below
+// 2^22, where the bits of D + 1.5 2^23 are D + 0x4B400000, except for d >= 4 with K = 64.
+template <int K>
+__device__ __forceinline__ long long recombine8_exact(const uint32_t* dd, int stride) {
+  static_assert(K <= 64, "8-bit digits: the int64 sum is sized for K <= 64");
+  int d[kDiag];
+#pragma unroll
+  for (int i = 0; i < kDiag; ++i) {
+    const float f = __uint_as_float(dd[i * stride]);
+    d[i] = (K <= 32 || i < 4) ? float_to_int_exact(f) : __float2int_rn(f);
+  }
+  const long long hi = (long long)d[0] * (1LL << 24) + (long long)d[1] * 65536 + ((long long)d[2] * 256 + d[3]);
+  const long long lo = (long long)d[4] * 65536 + ((long long)d[5] * 256 + d[6]);
+  return hi * (1LL << 18) + ((lo + 32) >> 6);
 }
 
 // Spin limits of the mbarrier waits.  A wait that runs out of W90G_SPIN_LIMIT tries makes

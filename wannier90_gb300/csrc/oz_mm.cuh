@@ -438,38 +438,6 @@ __device__ __forceinline__ void load_run8(double (&v)[8], const double2* base, s
   }
 }
 
-// The seven 8-bit digit planes of the 8 values scaled by 2^(55 - ex), as packed FP16
-// pairs: w[t][i / 2] holds digit t of values i (low half) and i + 1 -- the digits of
-// digits7x8, without its serial recoding.  With C = 128 (1 + 2^8 + ... + 2^40), byte t' of
-// N + C is digit 6 - t' plus 128 (adding 128 at every lower byte position turns the
-// centred digits into the plain bytes of N + C: x_6 = sext8(N mod 2^8) = byte0(N + 128) -
-// 128, and (N - x_6) / 2^8 = (N + 128) >> 8, so the next step repeats on N + 128 shifted),
-// and the top digit is (N + C) >> 48 (arithmetic), so b = digit + 128 lies in [0, 256].
-// With 0x6400 above it, b is the FP16 number 1024 + b: one byte permute, one mask and one
-// packed subtraction of 1152 give two digits.  Exact: FP16 holds the integers to 2048, and
-// the difference of two of them is rounded to itself.
-__device__ __forceinline__ void slice_run8_h(uint32_t (&w)[7][4], const double (&v)[8], int ex) {
-#pragma unroll
-  for (int i = 0; i < 8; i += 2) {
-    const long long ma = scaled_int55(v[i], ex) + 0x808080808080LL;
-    const long long mb = scaled_int55(v[i + 1], ex) + 0x808080808080LL;
-    const uint32_t la = (uint32_t)ma, lb = (uint32_t)mb;
-    const uint32_t ha = (uint32_t)((unsigned long long)ma >> 32), hb = (uint32_t)((unsigned long long)mb >> 32);
-#pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      const uint32_t bt = (uint32_t)(t & 3);
-      const uint32_t sel = bt | (bt << 4) | ((4u + bt) << 8) | ((4u + bt) << 12);
-      const uint32_t p = __byte_perm(t < 4 ? la : ha, t < 4 ? lb : hb, sel);
-      w[6 - t][i >> 1] = f16x2_sub((p & 0x00FF00FFu) | 0x64006400u, 0x64806480u);
-    }
-    const uint32_t ta = (uint32_t)((int)(ma >> 48) + 128), tb = (uint32_t)((int)(mb >> 48) + 128);
-    w[0][i >> 1] = f16x2_sub(ta | (tb << 16) | 0x64006400u, 0x64806480u);
-  }
-}
-
-// -x for both halves of a packed FP16 pair (a zero becomes -0, the same in every product)
-__device__ __forceinline__ uint32_t f16x2_neg(uint32_t w) { return w ^ 0x80008000u; }
-
 // C = A B, then the Epi.  num_wann <= 32 (staged accumulators): the epilogue applies the
 // Epi itself and writes ep.out only (C unused; ep.out may alias B, whose digits are in
 // shared memory before the MMAs run, but not A); WP = 64: C as in oz_cmm.
