@@ -205,14 +205,14 @@ int odn_of(int W) { return W <= 32 ? 4 : 4 * (W / 32 + 2); }
 
 struct Sizes {
   size_t M, U, KWW, work, tbuf, diag, offd, gpart, cen, log, logc, nn, bk, wb, st, op1, op2, m0, u0, inv, fr;
-  size_t m0s, m0e, zexp, ub2, ub2e;
+  size_t m0s, m0e, zexp, ub2, ub2e, einfo;
   size_t pkr, pr2, pgr, pgp, ppart;
   size_t gbka, gneigh, grg, gsheet, gcsheet;
   size_t slwf;
   size_t symi, symd, symw;
   size_t total() const {
     return 2 * M + 2 * U + 3 * KWW + work + tbuf + 2 * diag + offd + gpart + cen + log + logc + nn + bk + wb + st +
-           op1 + op2 + m0 + u0 + inv + fr + m0s + m0e + zexp + ub2 + ub2e + pkr + 2 * pr2 + pgr + pgp + ppart + gbka + gneigh + grg + gsheet +
+           op1 + op2 + m0 + u0 + inv + fr + m0s + m0e + zexp + ub2 + ub2e + einfo + pkr + 2 * pr2 + pgr + pgp + ppart + gbka + gneigh + grg + gsheet +
            gcsheet + slwf + symi + 2 * symd + symw;
   }
 };
@@ -226,8 +226,9 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
   z.M = align_up(K * B * WW * 16);
   z.U = align_up(K * WW * 16);
   z.KWW = align_up(K * WW * 16);
-  // exp workspace: FP64 kernels for W > 32; tensor exp keeps its matrices here for W > 16
-  z.work = (s.W > 32 || (wp && s.W > 16)) ? align_up(K * 6 * WW * 16) : 0;
+  // exp workspace: FP64 kernels for W > 32; the tensor exp keeps X and its powers here
+  z.work = (s.W > 32 || wp) ? align_up(K * 6 * WW * 16) : 0;
+  z.einfo = wp ? align_up(K * 8) : 0;
   z.tbuf = (s.W > 32 || wp) ? align_up(K * B * WW * 16) : 0;
   z.m0 = wp ? align_up(K * B * WW * 16) : 0;
   z.u0 = wp ? align_up(K * WW * 16) : 0;
@@ -387,6 +388,7 @@ int Engine::alloc(std::string& err) {
     P.D = (double2*)take(z.KWW);
     P.dU = (double2*)take(z.KWW);
     P.work = z.work ? (double2*)take(z.work) : nullptr;
+    P.expinfo = z.einfo ? (float*)take(z.einfo) : nullptr;
     P.tbuf = z.tbuf ? (double2*)take(z.tbuf) : nullptr;
     P.diag_ln = (double*)take(z.diag);
     P.diag_abs2 = (double*)take(z.diag);

@@ -1,14 +1,23 @@
-// Tensor-core rotation step: dU(k) = exp(s D(k)) and U(k) <- U(k) dU(k)
-// (internal_new_u_and_m, src/wannierise.F90:1655-1733) with every W x W complex
-// product on the tcgen05 tensor cores through exact slicing into BF16 / FP16 digits
-// (see k_tensor.cu).
+// Tensor-core rotation step: U(k) <- U(k) exp(s D(k)) (internal_new_u_and_m,
+// src/wannierise.F90:1655-1733) with every W x W complex product on the tcgen05 tensor cores
+// through exact slicing into FP16 / BF16 digits at 56-bit precision (oz_mm.cuh); norms and the
+// polynomials' linear combinations are FP64 (the norms' moduli FP32).
 //
-// The matrix function is the FP64 path's (k_exp_u in k_fp64.cu): scaling and squaring
-// of a Taylor polynomial evaluated by Paterson-Stockmeyer, degree and squarings chosen
-// per matrix from its 1-norm.  Scalar work (norms, the polynomial's linear combinations,
-// the Hermitian symmetrisation of the even powers) stays in FP64; only the products move
-// to the tensor pipe (oz_mm.cuh).  The exp chain (powers, Horner steps, up to ~10 squarings
-// that double any error) needs the 56-bit operands of those products.
+// The matrix function is a Taylor polynomial of degree 4, 8 or 12 of X 2^-js, squared js times.
+// What it costs is products (each: slice two operands, 28 to 36 digit-pair MMAs, recombine), so
+//   * the polynomials are evaluated with 2, 3 and 4 products (powers included) instead of
+//     Paterson-Stockmeyer's 3, 4 and 5:
+//       T4  = I + X + X^2 (1/2 + X/6 + X^2/24)
+//       T8  = I + X + y2 X^2 + (x3 X^2 + A) (x4 + x5 X + x6 X^2 + x7 A),  A = X^2 (x1 X + x2 X^2)
+//             (P. Bader, S. Blanes, F. Casas, Mathematics 7 (2019) 1174)
+//       T12 = I + X + c2 X^2 + c3 X^3 + (B2 + A) A,  A = a2 X^2 + a3 X^3 + B4^2, B2 and B4 cubics
+//             (their form; of its one-parameter family of solutions the one without constant
+//             and linear terms in A, so that nothing cancels against I);
+//   * the scaling follows sqrt(||X^2||_1), which bounds the 2-norm of the anti-Hermitian X and is
+//     half of ||X||_1 or less for a full W = 32 matrix: one squaring less on average;
+//   * the optimal step's X is a multiple of the trial step's, so its powers are the trial's: the
+//     factor f goes into the coefficients and the second exp starts after them.
+// Truncation: theta^(m+1) / (m+1)! <= 2^-53 at the 2-norm theta (||e^X||_2 = 1).
 //
 // One CTA (256 threads) per (problem, k).
 #include "oz_mm.cuh"
@@ -17,73 +26,36 @@ namespace w90g {
 
 namespace {
 
-// x 2^-j (sc = 2^-j): an exponent subtraction where the result is a normal number (the
-// product is exact there, so the bits are those of x * sc), else the FP64 multiply
-__device__ __forceinline__ double scale_pow2(double x, int j, double sc) {
-  const long long b = __double_as_longlong(x);
-  const int be = (int)((b >> 52) & 0x7FF);
-  if (be > j && be != 0x7FF) return __longlong_as_double(b - ((long long)j << 52));
-  return x * sc;
-}
+// T8: x1..x7, y2; T12: B2 (0..3), B4 (1..3), a2, a3, c2, c3.  T8 in closed form; T12 by Newton's
+// method on the 13 coefficient equations in 40 digits.
+constexpr double kT8x1 = 0.10836465678522780852, kT8x2 = 0.027091164196306952131, kT8x3 = 0.66666666666666666667,
+                 kT8x4 = 0.54676145797072405251, kT8x5 = 0.16112557339541759283, kT8x6 = 0.014090917158378207731,
+                 kT8x7 = 0.033792797010870504141, kT8y2 = 0.13549236135285063166;
+constexpr double kT12b0 = 5.0188519759285061501, kT12b1 = 1.3093238729699402869, kT12b2 = 0.15744598937135220317,
+                 kT12b3 = -0.0014710039978467423724, kT12e1 = 0.13181061013830184016,
+                 kT12e2 = 0.020278555405892590793, kT12e3 = 0.0067595184686308635978,
+                 kT12a2 = 0.020689394224651494005, kT12a3 = 0.012386729930502613689,
+                 kT12c2 = 0.30896527326341831812, kT12c3 = 0.027832075977002841435;
 
-// The number of halvings that bring v >= 0 to theta (a positive normal) or below, at most
-// 60: the count of the loop "while (v > theta && j < 60) { v *= 0.5; ++j; }" (halving is
-// exact), from the bits with integer ops only.  Non-negative doubles order like their bit
-// patterns; with v = mv 2^ev and theta = mt 2^et (mantissas in [1, 2)), v 2^-j <= theta
-// first holds at j = ev - et, or one later where mv > mt.  (0 for nan, where v > theta is
-// false; 60 for inf.)
-__device__ __forceinline__ int halvings(double v, double theta) {
-  constexpr long long kMant = 0x000FFFFFFFFFFFFFLL;
-  const long long vb = __double_as_longlong(v), tb = __double_as_longlong(theta);
-  if (vb <= tb) return 0;
-  if ((vb >> 52) == 0x7FF && (vb & kMant) != 0) return 0;
-  const int j = (int)(vb >> 52) - (int)(tb >> 52) + ((vb & kMant) > (tb & kMant) ? 1 : 0);
-  return j > 60 ? 60 : j;
-}
-
-// Degree m, block size pw and squarings js of exp(X) from its 1-norm, with the cost in
-// products (powers plus Horner steps, plus js): the FP64 path's table (k_exp_u), the
-// cheapest candidate after the halvings that bring the norm under its theta.
-struct ExpPlan {
-  int m, pw, js, cost;
-};
-__device__ const int kPlanM[5] = {4, 6, 8, 12, 16};
-__device__ const int kPlanP[5] = {4, 3, 4, 4, 4};
-__device__ const double kPlanTheta[5] = {1.6e-3, 1.68e-2, 6.6e-2, 0.32, 0.78};
-__device__ const int kPlanCost[5] = {3, 3, 4, 5, 6};
-
-__device__ __noinline__ ExpPlan exp_plan(double nrm) {
-  ExpPlan pl{16, 4, 0, 1 << 30};
-  for (int c = 0; c < 5; ++c) {
-    const int j = halvings(nrm, kPlanTheta[c]);
-    const int cost = kPlanCost[c] + j;
-    if (cost < pl.cost) pl = ExpPlan{kPlanM[c], kPlanP[c], j, cost};
+// degree m and squarings js of a 2-norm: the cheapest of T4 (2 products up to 1.6e-3), T8 (3 up
+// to 6.6e-2) and T12 (4 up to 0.32, one more per doubling); at most 60 squarings
+__device__ __forceinline__ void exp_plan(float rho, int& m, int& js) {
+  js = 0;
+  if (rho <= 1.6e-3f) {
+    m = 4;
+  } else if (rho <= 6.6e-2f) {
+    m = 8;
+  } else {
+    m = 12;
+    while (rho > 0.32f && js < 60) {
+      rho *= 0.5f;
+      ++js;
+    }
   }
-  return pl;
 }
 
-// Whether every norm within a relative 2^-14 of nrm gets the same halvings for every
-// candidate -- nrm finite and at least that far from each candidate's boundaries theta
-// 2^(j-1) and theta 2^j -- so that an estimate of the norm to that accuracy picks the plan
-// the exact norm picks.  (nrm < x 2^j compares the bits of nrm with those of x plus j in
-// the exponent field, x 2^j being a normal number here.)
-__device__ __noinline__ bool exp_plan_stable(double nrm) {
-  if (!(nrm < 1e300)) return false;
-  const long long nb = __double_as_longlong(nrm);
-  for (int c = 0; c < 5; ++c) {
-    const double th = kPlanTheta[c];
-    const int j = halvings(nrm, th);
-    const long long lo = __double_as_longlong(th * (1.0 - 0x1p-14)), hi = __double_as_longlong(th * (1.0 + 0x1p-14));
-    if (j < 60 && !(nb < lo + ((long long)j << 52))) return false;
-    if (j > 0 && !(nb > hi + ((long long)(j - 1) << 52))) return false;
-  }
-  return true;
-}
-
-// |re + i im| to a relative 2^-20 with no FP64 instruction: each part truncated to FP32
-// through its bits (0 below 2^-60, +inf above 2^60 or for inf / nan), then FP32 fma and
-// q rsqrt(q) (rsqrtf: 2 ulp).  A column sum of these (<= 128 terms, FP32) is within 2^-16
-// of the FP64 one.  (An infinite estimate gives a nan norm, which is never stable.)
+// |re + i im| in FP32 to a relative 2^-20 (0 below 2^-60, +inf above 2^60 or for inf / nan)
+// with no FP64 instruction: each part truncated through its bits, then fma and q rsqrt(q)
 __device__ __forceinline__ float abs_est(double2 v) {
   auto f32 = [](double x) -> float {
     const unsigned long long b = abs_bits(x);
@@ -97,12 +69,27 @@ __device__ __forceinline__ float abs_est(double2 v) {
   return q > 0.0f ? q * rsqrtf(q) : 0.0f;
 }
 
-__device__ const double kOzInvFact[17] = {
-    1.0, 1.0, 0.5, 1.6666666666666666e-01, 4.1666666666666664e-02, 8.3333333333333332e-03,
-    1.3888888888888889e-03, 1.9841269841269841e-04, 2.4801587301587302e-05,
-    2.7557319223985893e-06, 2.7557319223985888e-07, 2.5052108385441720e-08,
-    2.0876756987868100e-09, 1.6059043836821613e-10, 1.1470745597729725e-11,
-    7.6471637318198164e-13, 4.7794773323873853e-14};
+// c0 I + c1 X + c2 P2 + c3 P3 at element e, added by a product's epilogue
+struct PolyAdd {
+  static constexpr bool kActive = true;
+  const double2 *X, *P2, *P3;
+  double c0, c1, c2, c3;
+  int W;
+  __device__ double2 operator()(int e) const {
+    double2 v = cmk((e % W) == (e / W) ? c0 : 0.0, 0.0);
+    if (c1 != 0.0) {
+      const double2 x = X[e];
+      v = cmk(fma(x.x, c1, v.x), x.y * c1);
+    }
+    const double2 p = P2[e];
+    v = cmk(fma(p.x, c2, v.x), fma(p.y, c2, v.y));
+    if (c3 != 0.0) {
+      const double2 r = P3[e];
+      v = cmk(fma(r.x, c3, v.x), fma(r.y, c3, v.y));
+    }
+    return v;
+  }
+};
 
 }  // namespace
 
@@ -115,9 +102,9 @@ __global__ void __launch_bounds__(256, 2) k_oz_exp(const Problem* __restrict__ p
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_rowexp[WP], s_colexp[WP];
-  __shared__ unsigned s_key[6][2][WP];
+  __shared__ unsigned s_key[5][2][WP];
   __shared__ int s_bad;
-  __shared__ double red[256];
+  __shared__ float s_wmax[8];
 
   int k;
   const int p = locate(wm, blockIdx.x, k);
@@ -138,213 +125,198 @@ __global__ void __launch_bounds__(256, 2) k_oz_exp(const Problem* __restrict__ p
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_bad = 0;
   }
-  // FP64 matrices: shared memory for WP <= 32, else the per-k workspace (6 W^2)
-  double2* mats = E::MATS_IN_SMEM ? (double2*)(base + E::REGION)
-                                  : (P.work + (size_t)k * 6 * WW);
-  double2 *X = mats, *Y2 = mats + WW, *Y3 = mats + 2 * WW, *Y4 = mats + 3 * WW, *R = mats + 4 * WW,
-          *T = mats + 5 * WW;
-  double2* Dk = P.D + (size_t)k * WW;
-  const double s = (which == 0) ? st->s_trial : st->s_second;
-  // scale records of X, Y2, Y3, Y4, R, T (see Rec).  The powers are exactly Hermitian or
-  // anti-Hermitian (|re| and |im| of element (i, j) are those of (j, i)), so row i and
-  // column i of their records are the same maximum: one array serves both.
-  Rec rX{s_key[0][0], s_key[0][1]}, rY2{s_key[1][0], s_key[1][0]}, rY3{s_key[2][0], s_key[2][0]},
-      rY4{s_key[3][0], s_key[3][0]}, rR{s_key[4][0], s_key[4][1]}, rT{s_key[5][0], s_key[5][1]};
+  // the matrices: shared memory for WP <= 16 (32 on request), else the per-k workspace (6 W^2),
+  // whose first three -- X and its powers -- the optimal step's launch finds there
+  double2* kept = P.work + (size_t)k * 6 * WW;
+  double2* mats = E::MATS_IN_SMEM ? (double2*)(base + E::REGION) : kept;
+  double2 *X = mats, *P2 = mats + WW, *P3 = mats + 2 * WW, *Z = mats + 3 * WW, *A = mats + 4 * WW,
+          *L = mats + 5 * WW;
+  float* info = P.expinfo + (size_t)k * 2;   // sqrt(||X^2||_1) of the trial step; 1 when P3 is there
+  // scale records (see Rec).  The powers are exactly Hermitian or anti-Hermitian (|re| and |im| of
+  // element (i, j) are those of (j, i)), so row i and column i of their records are the same
+  // maximum: one array serves both.
+  Rec rX{s_key[0][0], s_key[0][0]}, rP2{s_key[0][1], s_key[0][1]}, rZ{s_key[2][0], s_key[2][1]},
+      rA{s_key[3][0], s_key[3][1]}, rL{s_key[4][0], s_key[4][1]};
+  const Rec norec{nullptr, nullptr};
+  const NoAdd none;
   rec_clear(rX, WP);
-  // ---- X = s D (the trial step first forms D = coefG G + coefD D_prev; in the
-  // symmetry-adapted mode k_sym_dir has formed D already) and estimates of the moduli
-  // |X_ij| into shared scratch.  num_wann <= 32: X stays in registers (element tid + 256 i
-  // in slot i) until it is scaled below.
-  constexpr bool XREG = WP <= 32;
-  constexpr int NE = XREG ? (WP * WP + 255) / 256 : 1;
-  double2 xr[NE];
-  // the digit region is free before the first product: |X_ij| estimates, then (where the
-  // exact norm is needed, once the estimates are summed) the exact moduli in its place
-  float* absf = (float*)base;
-  double* absx = (double*)base;
-  const bool form_d = (which == 0 && P.sym_nir == 0);
-  const double cg = st->coefG, cd = st->coefD;
-  const double2* Gk = form_d ? (st->use_gp ? P.pc_gp : P.G) + (size_t)k * WW : nullptr;
-  // (each product and the sum rounded on its own, as the oracle forms D: no contraction
-  // into an FMA, whose choice of product would follow the code's shape)
-  auto form_x = [&](int e) -> double2 {
-    double2 d = Dk[e];
-    if (form_d) {
-      const double2 g = Gk[e];
-      d = cmk(__dadd_rn(__dmul_rn(g.x, cg), __dmul_rn(d.x, cd)), __dadd_rn(__dmul_rn(g.y, cg), __dmul_rn(d.y, cd)));
-      Dk[e] = d;
-    }
-    const double2 x = cscale(d, s);
-    absf[e] = abs_est(x);
-    return x;
-  };
-  if (XREG) {
-#pragma unroll
-    for (int i = 0; i < NE; ++i) {
-      const int e = tid + 256 * i;
-      if (e < WW) xr[i] = form_x(e);
-    }
-  } else {
-#pragma unroll 4
-    for (int e = tid; e < WW; e += 256) X[e] = form_x(e);
-  }
+  rec_clear(rP2, WP);
+  rec_clear(rZ, WP);
+  rec_clear(rL, WP);
   __syncthreads();
   OzCtx cx{base, base + E::SB_OFFSET, tmem_slot, smem_u32(&mbar), 0u, s_rowexp, s_colexp, &s_bad};
-
-  // ---- degree / squarings from the 1-norm (the FP64 path's table and choice, exp_plan).
-  // The plan depends on the norm only through which side of each theta 2^j it lies, so
-  // the FP32 estimate decides wherever it is clearly inside one interval
-  // (exp_plan_stable); else the exact FP64 norm is formed -- moduli, then each column
-  // summed in row order -- as the FP64 path forms it.  One thread plans, all read it.
-  __shared__ float s_wmax[8];
-  __shared__ int s_plan[5];
-  {
-    float colmax = 0.0f;
+  bool ok = true;
+  float rho;
+  double f = 1.0;
+  bool have3 = false;
+  int nprod = 0;
+  if (which == 0) {
+    // ---- X = s D (first D = coefG G + coefD D_prev; in the symmetry-adapted mode k_sym_dir has
+    // formed D already).  Each product and the sum rounded on its own, as the oracle forms D:
+    // no contraction into an FMA, whose choice of product would follow the code's shape.
+    double2* Dk = P.D + (size_t)k * WW;
+    const double s = st->s_trial;
+    const bool form_d = P.sym_nir == 0;
+    const double cg = st->coefG, cd = st->coefD;
+    const double2* Gk = form_d ? (st->use_gp ? P.pc_gp : P.G) + (size_t)k * WW : nullptr;
+#pragma unroll 4
+    for (int e = tid; e < WW; e += 256) {
+      double2 d = Dk[e];
+      if (form_d) {
+        const double2 g = Gk[e];
+        d = cmk(__dadd_rn(__dmul_rn(g.x, cg), __dmul_rn(d.x, cd)), __dadd_rn(__dmul_rn(g.y, cg), __dmul_rn(d.y, cd)));
+        Dk[e] = d;
+      }
+      const double2 x = cscale(d, s);
+      X[e] = x;
+      rec_add(rX, e % W, e / W, x);
+    }
+    __syncthreads();
+    ok = E::mm(cx, P2, X, rX.row, X, rX.col, W, Epi{P2, 1, rP2}, none);
+    ++nprod;
+    // ---- sqrt(||X^2||_1) from FP32 moduli (their sums are within 2^-16; 2^-10 on top)
+    float* absf = (float*)base;   // the digit region is free between products
+    for (int e = tid; e < WW; e += 256) absf[e] = abs_est(P2[e]);
+    __syncthreads();
+    float cmax = 0.0f;
     for (int j = tid; j < W; j += 256) {
       float a = 0.0f;
       for (int i = 0; i < W; ++i) a += absf[(size_t)j * W + i];
-      colmax = fmaxf(colmax, a);
+      cmax = fmaxf(cmax, a);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) colmax = fmaxf(colmax, __shfl_xor_sync(0xffffffffu, colmax, o));
-    if ((tid & 31) == 0) s_wmax[warp] = colmax;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float nf = 0.0f;
-    for (int w = 0; w < 8; ++w) nf = fmaxf(nf, s_wmax[w]);
-    const bool stable = exp_plan_stable((double)nf);
-    const ExpPlan pl = exp_plan((double)nf);
-    s_plan[0] = pl.m;
-    s_plan[1] = pl.pw;
-    s_plan[2] = pl.js;
-    s_plan[3] = stable ? 0 : 1;
-    s_plan[4] = pl.cost;
-  }
-  __syncthreads();
-  if (s_plan[3]) {
-    auto exact_abs = [&](int e, double2 x) { absx[e] = sqrt(cabs2(x)); };
-    if (XREG) {
-#pragma unroll
-      for (int i = 0; i < NE; ++i) {
-        const int e = tid + 256 * i;
-        if (e < WW) exact_abs(e, xr[i]);
-      }
-    } else {
-      for (int e = tid; e < WW; e += 256) exact_abs(e, X[e]);
-    }
+    for (int o = 16; o > 0; o >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+    if ((tid & 31) == 0) s_wmax[warp] = cmax;
     __syncthreads();
-    double colmax = 0.0;
-    for (int j = tid; j < W; j += 256) {
-      double a = 0.0;
-      for (int i = 0; i < W; ++i) a += absx[(size_t)j * W + i];
-      colmax = fmax(colmax, a);
-    }
-    __syncthreads();
-    const double nrm = cta_max(colmax, red);
-    if (tid == 0) {
-      const ExpPlan pl = exp_plan(nrm);
-      s_plan[0] = pl.m;
-      s_plan[1] = pl.pw;
-      s_plan[2] = pl.js;
-      s_plan[4] = pl.cost;
-    }
-    __syncthreads();
-  }
-  const int m = s_plan[0], pw = s_plan[1], js = s_plan[2];
-  const double sc = ldexp(1.0, -js);
-  auto scale_x = [&](int e, double2 x) {
-    const double2 v = make_double2(scale_pow2(x.x, js, sc), scale_pow2(x.y, js, sc));
-    X[e] = v;
-    rec_add(rX, e % W, e / W, v);
-  };
-  if (XREG) {
-#pragma unroll
-    for (int i = 0; i < NE; ++i) {
-      const int e = tid + 256 * i;
-      if (e < WW) scale_x(e, xr[i]);
-    }
+    cmax = 0.0f;
+    for (int w = 0; w < 8; ++w) cmax = fmaxf(cmax, s_wmax[w]);
+    rho = sqrtf(cmax * 1.001f);
   } else {
-#pragma unroll 4
-    for (int e = tid; e < WW; e += 256) scale_x(e, X[e]);
+    f = st->s_second / st->s_trial;
+    rho = info[0] * fabsf((float)f) * 1.0001f;
+    have3 = info[1] != 0.0f;
   }
-  __syncthreads();
-  const NoAdd none;
-  // powers, exactly Hermitian (even) / anti-Hermitian (odd) as the FP64 path forms them
-  bool ok = E::mm(cx, Y2, X, rX.row, X, rX.col, W, Epi{Y2, 1, rY2}, none);
-  if (ok) ok = E::mm(cx, Y3, Y2, rY2.row, X, rX.col, W, Epi{Y3, -1, rY3}, none);
-  if (ok && pw >= 4) ok = E::mm(cx, Y4, Y2, rY2.row, Y2, rY2.col, W, Epi{Y4, 1, rY4}, none);
-  const double2* Yp = (pw == 4) ? Y4 : Y3;
-  const Rec rYp = (pw == 4) ? rY4 : rY3;
-  const int nblk = (m + pw) / pw;
-  // block q of the polynomial, sum_r c_{pw q + r} X^r (X^0 = I), one FMA per term and part
-  // (the FP64 pipe runs at 1/64 of FP32 on this chip: these elementwise terms are a large
-  // part of the chain's FP64 work)
-  auto blk = [&](int q, int e) -> double2 {
-    const int i = e % W, j = e / W;
-    double2 v = cmk(0.0, 0.0);
-    for (int r = 0; r < pw; ++r) {
-      const int deg = pw * q + r;
-      if (deg > m) break;
-      const double c = kOzInvFact[deg];
-      if (r == 0) {
-        if (i == j) v.x += c;
-      } else {
-        const double2 y = (r == 1) ? X[e] : ((r == 2) ? Y2[e] : Y3[e]);
-        v = cmk(fma(y.x, c, v.x), fma(y.y, c, v.y));
+  int m, js;
+  exp_plan(rho, m, js);
+  f *= ldexp(1.0, -js);
+  if (which == 1) {
+    // the powers kept by the trial step, with the records of those that enter a product
+    const bool need = m < 12 || !have3;
+    if (E::MATS_IN_SMEM || need)
+      for (int e = tid; e < WW; e += 256) {
+        const double2 x = kept[e], q = kept[WW + e];
+        if (E::MATS_IN_SMEM) {
+          X[e] = x;
+          P2[e] = q;
+          if (have3) P3[e] = kept[2 * WW + e];
+        }
+        if (need) {
+          rec_add(rX, e % W, e / W, x);
+          rec_add(rP2, e % W, e / W, q);
+        }
       }
+    __syncthreads();
+  }
+  const double f2 = f * f, f3 = f2 * f;
+  double2* Ex = Z;     // where the polynomial ends up
+  Rec rE = rZ;
+  if (m == 4) {
+    // E = P2 [f^2 (1/2 + f X / 6 + f^2 P2 / 24)] + I + f X
+    for (int e = tid; e < WW; e += 256) {
+      const double2 x = X[e], q = P2[e];
+      const double d = (e % W) == (e / W) ? 0.5 * f2 : 0.0;
+      const double2 z = cmk(fma(q.x, f2 * f2 / 24.0, fma(x.x, f3 / 6.0, d)), fma(q.y, f2 * f2 / 24.0, x.y * (f3 / 6.0)));
+      L[e] = z;
+      rec_add(rL, e % W, e / W, z);
     }
-    return v;
-  };
-  int q = nblk - 1;
-  rec_clear(rR, WP);
-  __syncthreads();
-  if (pw * q == m) {
-    const double cm = kOzInvFact[m];
-    #pragma unroll 4
-    for (int e = tid; e < WW; e += blockDim.x) {
-      const double2 b = blk(q - 1, e), y = Yp[e];
-      const double2 v = cmk(fma(y.x, cm, b.x), fma(y.y, cm, b.y));
-      R[e] = v;
-      rec_add(rR, e % W, e / W, v);
+    __syncthreads();
+    if (ok) ok = E::mm(cx, Z, P2, rP2.row, L, rL.col, W, Epi{Z, 0, rZ}, PolyAdd{X, P2, P3, 1.0, f, 0.0, 0.0, W});
+    nprod += 1;
+  } else if (m == 8) {
+    for (int e = tid; e < WW; e += 256) {
+      const double2 x = X[e], q = P2[e];
+      const double2 z = cmk(fma(q.x, kT8x2 * f2 * f2, x.x * (kT8x1 * f3)), fma(q.y, kT8x2 * f2 * f2, x.y * (kT8x1 * f3)));
+      L[e] = z;
+      rec_add(rL, e % W, e / W, z);
     }
-    q -= 1;
+    __syncthreads();
+    if (ok) ok = E::mm(cx, A, P2, rP2.row, L, rL.col, W, Epi{A, 0, norec}, none);
+    rec_clear(rL, WP);
+    rec_clear(rA, WP);
+    __syncthreads();
+    // left factor into L, right factor over A
+    for (int e = tid; e < WW; e += 256) {
+      const double2 x = X[e], q = P2[e], a = A[e];
+      const double d = (e % W) == (e / W) ? kT8x4 : 0.0;
+      const double2 l = cmk(fma(q.x, kT8x3 * f2, a.x), fma(q.y, kT8x3 * f2, a.y));
+      const double2 r = cmk(fma(a.x, kT8x7, fma(q.x, kT8x6 * f2, fma(x.x, kT8x5 * f, d))),
+                            fma(a.y, kT8x7, fma(q.y, kT8x6 * f2, x.y * (kT8x5 * f))));
+      L[e] = l;
+      A[e] = r;
+      rec_add(rL, e % W, e / W, l);
+      rec_add(rA, e % W, e / W, r);
+    }
+    __syncthreads();
+    if (ok) ok = E::mm(cx, Z, L, rL.row, A, rA.col, W, Epi{Z, 0, rZ}, PolyAdd{X, P2, P3, 1.0, f, kT8y2 * f2, 0.0, W});
+    nprod += 2;
   } else {
-    #pragma unroll 4
-    for (int e = tid; e < WW; e += blockDim.x) {
-      const double2 v = blk(q, e);
-      R[e] = v;
-      rec_add(rR, e % W, e / W, v);
+    if (!have3) {
+      if (ok) ok = E::mm(cx, P3, P2, rP2.row, X, rX.col, W, Epi{P3, -1, norec}, none);
+      ++nprod;
+      have3 = true;
     }
+    for (int e = tid; e < WW; e += 256) {
+      const double2 x = X[e], q = P2[e], r = P3[e];
+      const double2 z = cmk(fma(r.x, kT12e3 * f3, fma(q.x, kT12e2 * f2, x.x * (kT12e1 * f))),
+                            fma(r.y, kT12e3 * f3, fma(q.y, kT12e2 * f2, x.y * (kT12e1 * f))));
+      Z[e] = z;
+      rec_add(rZ, e % W, e / W, z);
+    }
+    __syncthreads();
+    if (ok) ok = E::mm(cx, A, Z, rZ.row, Z, rZ.col, W, Epi{A, 0, rA}, PolyAdd{X, P2, P3, 0.0, 0.0, kT12a2 * f2, kT12a3 * f3, W});
+    for (int e = tid; e < WW; e += 256) {
+      const double2 x = X[e], q = P2[e], r = P3[e], a = A[e];
+      const double d = (e % W) == (e / W) ? kT12b0 : 0.0;
+      const double2 l = cmk(a.x + fma(r.x, kT12b3 * f3, fma(q.x, kT12b2 * f2, fma(x.x, kT12b1 * f, d))),
+                            a.y + fma(r.y, kT12b3 * f3, fma(q.y, kT12b2 * f2, x.y * (kT12b1 * f))));
+      L[e] = l;
+      rec_add(rL, e % W, e / W, l);
+    }
+    __syncthreads();
+    if (ok)
+      ok = E::mm(cx, Z, L, rL.row, A, rA.col, W, Epi{Z, 0, rZ}, PolyAdd{X, P2, P3, 1.0, f, kT12c2 * f2, kT12c3 * f3, W});
+    nprod += 2;
   }
-  __syncthreads();
-  // Horner steps R <- Yp R + block q (the product's epilogue adds the block)
-  for (q = q - 1; q >= 0 && ok; --q) {
-    const HornerAdd<decltype(blk)> hadd{&blk, q};
-    ok = E::mm(cx, T, Yp, rYp.row, R, rR.col, W, Epi{R, 0, rR}, hadd);
-  }
-  double2* a = R;
-  double2* b = T;
-  Rec ra = rR, rb = rT;
+  // ---- squarings, between Z and A
+  double2* other = A;
+  Rec ro = rA;
   for (int sq = 0; sq < js && ok; ++sq) {
-    ok = E::mm(cx, b, a, ra.row, a, ra.col, W, Epi{b, 0, rb}, none);
-    double2* tmp = a;
-    a = b;
-    b = tmp;
-    const Rec rt = ra;
-    ra = rb;
-    rb = rt;
+    ok = E::mm(cx, other, Ex, rE.row, Ex, rE.col, W, Epi{other, 0, ro}, none);
+    double2* t = Ex;
+    Ex = other;
+    other = t;
+    const Rec rt = rE;
+    rE = ro;
+    ro = rt;
   }
-  // dU = exp(s D);  U[cur^1] = U[cur] dU
-  double2* dUk = P.dU + (size_t)k * WW;
-  #pragma unroll 4
-  for (int e = tid; e < WW; e += blockDim.x) dUk[e] = a[e];
-  __syncthreads();
+  // ---- U[cur^1] = U[cur] exp(s D)
   const int cur = st->cur;
   double2* Unew = P.U[cur ^ 1] + (size_t)k * WW;
-  if (ok) ok = E::mm(cx, Unew, P.U[cur] + (size_t)k * WW, nullptr, a, ra.col, W, Epi{Unew, 0, Rec{nullptr, nullptr}},
-                     none);
-  if (tid == 0) atomicAdd(&st->exp_products, (double)s_plan[4] + 1.0);   // the plan's cost, + U dU
+  if (ok) ok = E::mm(cx, Unew, P.U[cur] + (size_t)k * WW, nullptr, Ex, rE.col, W, Epi{Unew, 0, norec}, none);
+  if (which == 0) {
+    // for the optimal step
+    if (E::MATS_IN_SMEM)
+      for (int e = tid; e < WW; e += 256) {
+        kept[e] = X[e];
+        kept[WW + e] = P2[e];
+        if (have3) kept[2 * WW + e] = P3[e];
+      }
+    if (tid == 0) {
+      info[0] = rho;
+      info[1] = have3 ? 1.0f : 0.0f;
+    }
+  }
+  if (tid == 0) atomicAdd(&st->exp_products, (double)(nprod + js) + 1.0);   // and U exp(s D)
   if (!ok && tid == 0) {
     st->error = 2;
     st->done = 1;

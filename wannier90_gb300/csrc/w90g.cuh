@@ -119,7 +119,8 @@ struct Problem {
   double2* G;
   double2* D;
   double2* dU;
-  double2* work;        // exp / eig workspace (W > 32): 6*W*W per k
+  double2* work;        // exp / eig workspace (W > 32, or the tensor exp): 6*W*W per k
+  float* expinfo;       // tensor exp: [k][2] norm and state of the trial step's powers, for the optimal step
   double2* tbuf;        // M-update intermediate (W > 32): W*W per (k,b)
   const int* nnlist;    // [k][b] 0-based
   const double* bk;     // [k][b][3]
