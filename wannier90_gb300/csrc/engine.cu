@@ -192,11 +192,12 @@ int choose_tensor_wp(const std::vector<ProblemSpec>& specs) {
   return wmax <= 8 ? 8 : (wmax <= 16 ? 16 : (wmax <= 32 ? 32 : (wmax <= 64 ? 64 : 128)));
 }
 
-// chunks of the spread passes: at most 64 blocks each, and down to 16 while that gives every SM
-// one (64 alone left 100 of the SMs idle on 3072 blocks of num_wann 128: 55 us against 20)
+// chunks of the spread passes: 64 blocks (k,b) each, and from 512 blocks on down to 16 while that
+// gives every SM one (64 alone left 100 of the SMs idle on 3072 blocks of num_wann 128)
 int omega_chunks(const ProblemSpec& s) {
   const int KB = s.K * s.B;
-  return std::max((KB + 63) / 64, std::min((KB + 15) / 16, 152));
+  const int n = (KB + 63) / 64;
+  return KB < 512 ? n : std::max(n, std::min((KB + 15) / 16, 152));
 }
 
 // partial off-diagonal sums per (k,b) that the tensor M update's epilogue writes: one per column
@@ -205,14 +206,14 @@ int odn_of(int W) { return W <= 32 ? 4 : 4 * (W / 32 + 2); }
 
 struct Sizes {
   size_t M, U, KWW, work, tbuf, diag, offd, gpart, cen, log, logc, nn, bk, wb, st, op1, op2, m0, u0, inv, fr;
-  size_t m0s, m0e, zexp, ub2, ub2e, einfo;
+  size_t m0s, m0e, zexp, ub2, ub2e, einfo, odp;
   size_t pkr, pr2, pgr, pgp, ppart;
   size_t gbka, gneigh, grg, gsheet, gcsheet;
   size_t slwf;
   size_t symi, symd, symw;
   size_t total() const {
     return 2 * M + 2 * U + 3 * KWW + work + tbuf + 2 * diag + offd + gpart + cen + log + logc + nn + bk + wb + st +
-           op1 + op2 + m0 + u0 + inv + fr + m0s + m0e + zexp + ub2 + ub2e + einfo + pkr + 2 * pr2 + pgr + pgp + ppart + gbka + gneigh + grg + gsheet +
+           op1 + op2 + m0 + u0 + inv + fr + m0s + m0e + zexp + ub2 + ub2e + einfo + odp + pkr + 2 * pr2 + pgr + pgp + ppart + gbka + gneigh + grg + gsheet +
            gcsheet + slwf + symi + 2 * symd + symw;
   }
 };
@@ -233,7 +234,8 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
   z.m0 = wp ? align_up(K * B * WW * 16) : 0;
   z.u0 = wp ? align_up(K * WW * 16) : 0;
   z.inv = wp ? align_up(K * B * 4) : 0;
-  z.fr = wp ? align_up(K * B * odn_of(s.W) * 8) : 0;
+  z.odp = wp ? align_up(K * B * odn_of(s.W) * 8) : 0;
+  z.fr = wp ? align_up(K * B * 8) : 0;
   z.m0s = z.m0e = 0;
   z.zexp = (wp && wp <= 32) ? align_up(K * B * W * 4) : 0;
   z.ub2 = z.ub2e = 0;
@@ -406,7 +408,8 @@ int Engine::alloc(std::string& err) {
     int* inv = z.inv ? (int*)take(z.inv) : nullptr;
     P.inv_nnlist = inv;
     P.tensor = tensor_wp_ ? 1 : 0;
-    P.odpart = z.fr ? (double*)take(z.fr) : nullptr;
+    P.frob0 = z.fr ? (double*)take(z.fr) : nullptr;
+    P.odpart = z.odp ? (double*)take(z.odp) : nullptr;
     P.odn = odn_of(s.W);
     P.m0s = z.m0s ? (unsigned char*)take(z.m0s) : nullptr;
     P.m0s_exp = z.m0e ? (int*)take(z.m0e) : nullptr;

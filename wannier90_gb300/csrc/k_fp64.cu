@@ -65,12 +65,18 @@ __device__ void cta_gemm(double2* __restrict__ C, int ldc, const double2* __rest
 // Per-block statistics of one M(k,b): Im ln M_nn, |M_nn|^2, sum_{m!=n}|M_mn|^2.
 // (the quantities wann_omega reads, src/wannierise.F90:2034-2043, :2076-2090, :2241-2258)
 __device__ void block_stats(const double2* Mb, int ld, int W, double* ln_out, double* abs2_out,
-                            double* offd_out, double* red, const Problem* P = nullptr, size_t kb = 0) {
-  double off = 0.0;
+                            double* offd_out, double* red, const Problem* P = nullptr, size_t kb = 0,
+                            double* fro_out = nullptr) {
+  double off = 0.0, fro = 0.0;
   for (int e = threadIdx.x; e < W * W; e += blockDim.x) {
     const int m = e % W, n = e / W;
     const double2 v = Mb[n * ld + m];
     if (m != n) off += cabs2(v);
+    if (fro_out) fro += cabs2(v);
+  }
+  if (fro_out) {
+    fro = block_sum(fro, red);
+    if (threadIdx.x == 0) *fro_out = fro;
   }
   for (int n = threadIdx.x; n < W; n += blockDim.x) {
     const double2 d = Mb[n * ld + n];
@@ -93,7 +99,7 @@ __global__ void k_mdiag(const Problem* __restrict__ probs, WorkMap wm) {
   const int W = P.W;
   const double2* Mb = P.M[P.st->cur] + (size_t)local * W * W;
   block_stats(Mb, W, W, P.diag_ln + (size_t)local * W, P.diag_abs2 + (size_t)local * W,
-              P.offd + local, red, &P, (size_t)local);
+              P.offd + local, red, &P, (size_t)local, P.frob0 ? P.frob0 + local : nullptr);
 }
 
 // ----------------------------------------------------------------------------
@@ -109,8 +115,12 @@ __global__ void k_mdiag(const Problem* __restrict__ probs, WorkMap wm) {
 // the off-diagonal sum takes all threads, and a last CTA reads the chunk partials sixteen loads
 // at a time into four accumulators.
 // On the tensor path the off-diagonal sums come from the M update's epilogue (odpart), summed
-// there directly: |M0|_F^2 minus the diagonal, which they replace, cancels to ~1e-14 of num_wann
-// and near a minimum hid the trial step's change from the parabola.
+// there directly.  |M0|_F^2 minus the diagonal, the invariant form used before, cancels to ~1e-14 of
+// num_wann and near a minimum hid the trial step's change from the parabola (1000 k, num_wann 32,
+// 1e-12 window: refused steps, Omega 5e-8 after 3107 iterations; with the direct sum 8e-11).  Only
+// the first trial step still takes the invariant form: the first step length is the one quantity
+// that its offset against the entry overlaps' direct sum moves by more than rounding, and with it
+// the whole trajectory, which so stays the earlier one.
 // Selective localisation (slwf_num = s > 0, :2144-2211): p1's off-diagonal slot holds
 // sum over n < s of wb (1 - |M_nn|^2 + lambda ln_n^2) (Omega_IOD) and its Omega_I slot
 // sum over n < s of 2 wb lambda ln_n (b.c_n) (the k-sum of Omega_nu); p2 sums over n < s
@@ -210,24 +220,42 @@ __global__ void __launch_bounds__(256) k_omega_p1(const Problem* __restrict__ pr
   } else {
     const bool first = (slot == 2) && st->first_pass;
     const bool parts = P.tensor && slot < 2;   // partials of the tensor M update's epilogue
+    const bool inv = parts && slot == 0 && st->iter == 0;
     double od = 0.0, oi = 0.0;
-    // tpk threads share one block (k,b)
-    int tpk = 1;
-    while (2 * tpk * per <= (int)blockDim.x && tpk < 32) tpk *= 2;
-    const int sl = t % tpk;
-    for (int kb = kb0 + t / tpk; kb < kb1; kb += blockDim.x / tpk) {
-      const double w = P.wb[kb % B];
-      double o = 0.0;
-      if (parts) {
-        for (int i = sl; i < P.odn; i += tpk) o += P.odpart[(size_t)kb * P.odn + i];
-      } else if (sl == 0) {
-        o = P.offd[kb];
+    if (parts) {
+      // tpk threads share one block (k,b); per <= 64 blocks take one round
+      int tpk = 1;
+      while (2 * tpk * per <= (int)blockDim.x && tpk < 32) tpk *= 2;
+      const int sl = t % tpk, kb = kb0 + t / tpk;
+      const bool in = kb < kb1 && t / tpk < per;
+      const double w = in ? P.wb[kb % B] : 0.0;
+      double o = 0.0, sd = 0.0;
+      if (in) {
+        if (!inv)
+          for (int i = sl; i < P.odn; i += tpk) o += P.odpart[(size_t)kb * P.odn + i];
+        else
+          for (int m = sl; m < W; m += tpk) sd += P.diag_abs2[(size_t)kb * W + m];
       }
-      od += w * o;
-      if (first) {
-        double sd = 0.0;
-        for (int m = sl; m < W; m += tpk) sd += P.diag_abs2[(size_t)kb * W + m];
-        oi += w * ((sl == 0 ? (double)W : 0.0) - (o + sd));
+      if (inv) {
+        __syncthreads();   // s_sum's sums are out
+        s_sum[0][t] = sd;
+        __syncthreads();
+        if (in && sl == 0) {
+          for (int i = 1; i < tpk; ++i) sd += s_sum[0][t + i];
+          o = P.frob0[kb] - sd;
+        }
+      }
+      od = w * o;
+    } else {
+      for (int kb = kb0 + t; kb < kb1; kb += blockDim.x) {
+        const double w = P.wb[kb % B];
+        const double o = P.offd[kb];
+        od += w * o;
+        if (first) {
+          double sd = 0.0;
+          for (int m = 0; m < W; ++m) sd += P.diag_abs2[(size_t)kb * W + m];
+          oi += w * ((double)W - (o + sd));
+        }
       }
     }
     od = block_sum(od, red);

@@ -1,6 +1,6 @@
 // Tensor-core M update for num_wann <= 32, pipelined: M(k,b) = U(k)^H M0(k,b) U(k+b).
 //
-// The arithmetic is k_tensor.cu's (real embedding, 7 signed 8-bit FP16 digits per
+// The arithmetic is k_tensor.cu's (real embedding, 7 signed 7-bit FP16 digits per
 // operand, the 28 digit pairs of the 7 diagonals accumulated exactly in FP32 TMEM
 // columns, exact int64 recombination), so results are bitwise those of k_oz_mupdate;
 // only the schedule differs.  One persistent CTA per SM walks the work units
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
               const int it = pa + j * R::PAT;
               if (it < R::AITEMS) {
                 uint32_t w[kS][4];
-                slice_run8_h(w, av[j], zex[j]);
+                pack_digits7(w, av[j], zex[j], false);
                 const uint32_t o = stage_off(it % kTileRows, 8 * (it / kTileRows));
 #pragma unroll
                 for (int t = 0; t < kS; ++t)
@@ -335,11 +335,11 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
           v[i] = 0.0;
           if (cc < W && mm < W) {
             const double2 u = Ug[(size_t)cc * W + mm];
-            v[i] = part == 0 ? u.x : u.y;
+            v[i] = part == 0 ? u.x : -u.y;     // step 1: B = conj(U)
           }
         }
         uint32_t w[kS][4];
-        slice_run8_h(w, v, ec);
+        pack_digits7(w, v, ec, false);
         const int k_re = g8 * 16, k_im = k_re + 8;   // K positions of Re / Im of m = 8 g8 ..
         if (part == 0) {
           const uint32_t o_rr = kmaj_off(cc, k_re, KC), o_ii = kmaj_off(CW + cc, k_im, KC);
@@ -355,19 +355,21 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
             }
           }
         } else {
-          // step 1 (B = conj(U)): B_i = -Im U to (N im, K re) and -B_i = Im U to (N re, K im);
-          // step 2's image the other way round
+          // B_i = -Im U (step 1) to (N im, K re) -- for step 2 (B_i = Im U) the same digits
+          // go to (N re, K im) -- and -B_i = Im U to (N re, K im), for step 2 to (N im, K re)
           const uint32_t o_ir = kmaj_off(CW + cc, k_re, KC), o_ri = kmaj_off(cc, k_im, KC);
 #pragma unroll
           for (int t = 0; t < kS; ++t) {
             const uint4 q = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
-            const uint4 n = make_uint4(f16x2_neg(w[t][0]), f16x2_neg(w[t][1]), f16x2_neg(w[t][2]), f16x2_neg(w[t][3]));
+            *(uint4*)(dB + (size_t)t * L::B_PLANE + o_ir) = q;
+            if (gB) *(uint4*)(gB + (size_t)t * L::B_PLANE + o_ri) = q;
+          }
+          pack_digits7(w, v, ec, true);
+#pragma unroll
+          for (int t = 0; t < kS; ++t) {   // the digits of the negated values
+            const uint4 q = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
             *(uint4*)(dB + (size_t)t * L::B_PLANE + o_ri) = q;
-            *(uint4*)(dB + (size_t)t * L::B_PLANE + o_ir) = n;
-            if (gB) {
-              *(uint4*)(gB + (size_t)t * L::B_PLANE + o_ir) = q;
-              *(uint4*)(gB + (size_t)t * L::B_PLANE + o_ri) = n;
-            }
+            if (gB) *(uint4*)(gB + (size_t)t * L::B_PLANE + o_ir) = q;
           }
         }
       }
@@ -531,8 +533,8 @@ __global__ void __launch_bounds__(Roles<STEP>::THREADS, 1)
           for (int j = 0; j < 2; ++j) {
             const int c = j0 + j;   // complex output column
             const int e = erow + ecol[c - jbeg];
-            const double re = int64_scaled_to_double(recombine8_exact<KC>(&q[0][j], 2), e - 56);
-            const double im = int64_scaled_to_double(recombine8_exact<KC>(&s2[0][j], 2), e - 56);
+            const double re = int64_scaled_to_double(recombine7_exact(&q[0][j], 2), e - 56);
+            const double im = int64_scaled_to_double(recombine7_exact(&s2[0][j], 2), e - 56);
             if (STEP == 1) {
               // step 2's row scale of row c of Z(k,b): the largest |re|, |im| over this
               // block's rows rr, i.e. over its WP lanes (segmented max; zero rows add 0).
@@ -639,7 +641,7 @@ __global__ void __launch_bounds__(256) k_oz_preslice2(const Problem* __restrict_
           v[i] = ((const double*)(P.M0 + ((size_t)g * B + bi) * WW + (size_t)rr * W + m))[part];
       }
       uint32_t w[kS][4];
-      slice_run8_h(w, v, s_rowexp[r]);
+      pack_digits7(w, v, s_rowexp[r], false);
       const uint32_t o = stage_off(r, 8 * part);
 #pragma unroll
       for (int t = 0; t < kS; ++t)

@@ -1,17 +1,17 @@
-// Tensor-core M update: M(k,b) = U(k)^H M0(k,b) U(k+b) with FP64 accuracy from
+// Tensor-core M update: M(k,b) = U(k)^H M0(k,b) U(k+b) with FP64-level accuracy from
 // FP16 tcgen05 MMAs (Ozaki-style exact slicing).
 //
 // Every complex product is computed through its real embedding
 //     [C_r C_i] = [A_r A_i] [[B_r, B_i], [-B_i, B_r]]      (K = N = 2*WP real)
 // Each operand is scaled per row (A) / per column (B) by a power of two and split into
-// S = 7 signed 8-bit digits (|x| <= 128), each an exact FP16 value (built two at a time by a
-// packed FP16 subtraction, slice_run8_h).  For every digit pair (t,u) with t+u <= S-1 (0-based)
-// the MMA A^(t) B^(u) over the K = 2*WP <= 64 reduction is exact in the FP32 accumulator (every
-// partial sum is an integer below 2^23), so the pairs of one diagonal d = t+u share one TMEM
-// accumulator.  The epilogue recombines the 7 diagonals in int64 and rounds once to FP64.
-// Error: the digit pairs left out, ~2^-53 of (row scale x column scale).  (7-bit digits, whose
-// error is 2^-48, cost the same MMAs and more slicing.)  num_wann <= 32 here; the pipelined form
-// of the same arithmetic is k_mupdate2.cu, wider problems take k_mupdate3.cu.
+// S = 7 signed 7-bit digits (x_1 in [-128,128], x_t in [-64,63] for t > 1), each an exact
+// FP16 value (built two at a time by a packed FP16 subtraction, pack_digits7).  For every digit
+// pair (t,u) with t+u <= S-1 (0-based) the MMA A^(t) B^(u) over the K = 2*WP <= 64 reduction is
+// exact in the FP32 accumulator (every partial sum is an integer below 2^22), so the pairs of one
+// diagonal d = t+u share one TMEM accumulator.  The epilogue recombines the 7 diagonals exactly in
+// int64 and rounds once to FP64.  Truncation error: ~2^-49 of (row scale x column scale).
+// num_wann <= 32 here; the pipelined form of the same arithmetic is k_mupdate2.cu, wider problems
+// take k_mupdate3.cu.
 //
 // The product is batched as tall-skinny GEMMs (B*WP rows sharing one WP x WP operand):
 //   step 1 (group k):  rows (b, n):  Z(k,b)^T = M0(k,b)^T conj(U(k))   -> Z row-major
@@ -61,7 +61,7 @@ __device__ __forceinline__ void a_slice_chunk(unsigned char* dst, int tile, int 
       v[i] = part == 0 ? a.x : a.y;
     }
     uint32_t w[kS][4];
-    slice_run8_h(w, v, rowexp[r]);
+    pack_digits7(w, v, rowexp[r], false);
     const uint32_t o = kmaj_off(r, part * CW + lg * 8, KC);
 #pragma unroll
     for (int t = 0; t < kS; ++t)
@@ -152,18 +152,12 @@ __global__ void __launch_bounds__(256, 1) k_oz_mupdate(const Problem* __restrict
         v[i] = 0.0;
         if (cc < W && mm < W) {
           const double2 u = Ug[(size_t)cc * W + mm];
-          v[i] = kre == nre ? u.x : u.y;    // [B_r B_i; -B_i B_r], the sign below
+          const double br = u.x, bi = (STEP == 1) ? -u.y : u.y;
+          v[i] = (kre && nre) ? br : (kre ? bi : (nre ? -bi : br));   // [B_r B_i; -B_i B_r]
         }
       }
       uint32_t w[kS][4];
-      slice_run8_h(w, v, s_colexp[cc < WP ? cc : 0]);
-      // (B = conj(U) in step 1, U in step 2; the digits are always Im U's, negated where needed)
-      if (STEP == 1 ? (kre && !nre) : (!kre && nre)) {
-#pragma unroll
-        for (int t = 0; t < kS; ++t)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) w[t][i] = f16x2_neg(w[t][i]);
-      }
+      pack_digits7(w, v, s_colexp[cc < WP ? cc : 0], false);
       const uint32_t off = kmaj_off(n, kk0, KC);
 #pragma unroll
       for (int t = 0; t < kS; ++t)
@@ -323,8 +317,8 @@ __global__ void __launch_bounds__(256, 1) k_oz_mupdate(const Problem* __restrict
           for (int j = 0; j < 4; ++j) {
             const int c = nc * CW + j0 + j;   // complex output column
             const int ecol = s_colexp[c < WP ? c : 0];
-            const double re = int64_scaled_to_double(recombine8_exact<KC>(&q[0][j], 4), erow + ecol - 56);
-            const double im = int64_scaled_to_double(recombine8_exact<KC>(&s4[0][j], 4), erow + ecol - 56);
+            const double re = int64_scaled_to_double(recombine7_exact(&q[0][j], 4), erow + ecol - 56);
+            const double im = int64_scaled_to_double(recombine7_exact(&s4[0][j], 4), erow + ecol - 56);
             if (valid && c < W) {
               if (STEP == 1) {
                 // Z(k,b) row-major: element (j=c, n=rr) at c*W + rr

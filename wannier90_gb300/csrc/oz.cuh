@@ -288,23 +288,18 @@ __device__ __forceinline__ double recombine7x8(const uint32_t* dd, int stride, i
   return int64_scaled_to_double(hi, sc + 24) + int64_scaled_to_double(lo, sc);
 }
 
-// S with C = S 2^(e-56) of the 7 diagonal accumulators dd[0], dd[stride], ... of an 8-bit-digit
-// product over K <= 64 real terms (the M update of num_wann <= 32; e the exponents' sum): D_0..D_3
-// at 2^(42-8d) plus (D_4 2^16 + D_5 2^8 + D_6) / 2^6 rounded, below 2^63 for any operands.  The last
-// bit weighs 2^(e-56); the digit pairs left out weigh ~2^(e-53).  |D_d| <= (d + 1) K 2^14 is below
-// 2^22, where the bits of D + 1.5 2^23 are D + 0x4B400000, except for d >= 4 with K = 64.
-template <int K>
-__device__ __forceinline__ long long recombine8_exact(const uint32_t* dd, int stride) {
-  static_assert(K <= 64, "8-bit digits: the int64 sum is sized for K <= 64");
-  int d[kDiag];
+// S = sum_d D_d 2^(7(6-d)) of the 7 diagonal accumulators dd[0], dd[stride], ... (exact
+// integers |D_d| < 2^22 held in FP32), exactly.  b_d = bits(D_d + 1.5 * 2^23) = D_d +
+// 0x4B400000, and S = 2^21 H + L with H = sum_{d<=3} D_d 2^(7(3-d)), L = sum_{d>=4}
+// D_d 2^(7(6-d)): each a sum of widened 32 x 32-bit products with the bias folded into
+// one constant.
+__device__ __forceinline__ long long recombine7_exact(const uint32_t* dd, int stride) {
+  long long b[kDiag];
 #pragma unroll
-  for (int i = 0; i < kDiag; ++i) {
-    const float f = __uint_as_float(dd[i * stride]);
-    d[i] = (K <= 32 || i < 4) ? float_to_int_exact(f) : __float2int_rn(f);
-  }
-  const long long hi = (long long)d[0] * (1LL << 24) + (long long)d[1] * 65536 + ((long long)d[2] * 256 + d[3]);
-  const long long lo = (long long)d[4] * 65536 + ((long long)d[5] * 256 + d[6]);
-  return hi * (1LL << 18) + ((lo + 32) >> 6);
+  for (int d = 0; d < kDiag; ++d) b[d] = (long long)__float_as_int(__uint_as_float(dd[d * stride]) + 12582912.0f);
+  const long long H = b[0] * (1LL << 21) + b[1] * (1LL << 14) + b[2] * 128LL + b[3] - 0x4B400000LL * 2113665LL;
+  const long long L = b[4] * (1LL << 14) + b[5] * 128LL + b[6] - 0x4B400000LL * 16513LL;
+  return H * (1LL << 21) + L;
 }
 
 // Spin limits of the mbarrier waits.  A wait that runs out of W90G_SPIN_LIMIT tries makes
