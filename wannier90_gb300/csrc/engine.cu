@@ -24,6 +24,7 @@ __global__ void k_mdiag(const Problem* probs, WorkMap wm);
 __global__ void k_omega_p1(const Problem* probs, WorkMap wm, int slot);
 __global__ void k_omega_p2(const Problem* probs, WorkMap wm, int slot);
 __global__ void k_grad(const Problem* probs, WorkMap wm);
+__global__ void k_grad_search(const Problem* probs, WorkMap wm);
 __global__ void k_ctrl_search(const Problem* probs);
 __global__ void k_exp_u(const Problem* probs, WorkMap wm, int which);
 __global__ void k_m_update(const Problem* probs, WorkMap wm, int mode, int which);
@@ -68,6 +69,7 @@ namespace {
 constexpr size_t kAlign = 256;
 size_t align_up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 constexpr int kTileW = 32;
+constexpr int kOmegaFused = 16, kOmegaOneCta = 3072;   // as in k_fp64.cu
 constexpr int kPolarMinW = 9;   // projection on the tensor cores from this width on (see project)
 
 #define W90G_CHECK(call)                                                          \
@@ -351,6 +353,8 @@ int Engine::alloc(std::string& err) {
   n_kb_ = offs_kb[np];
   n_grad_ = offs_grad[np];
   n_chunk_ = offs_chunk[np];
+  omega_two_ = false;
+  for (const auto& s : specs_) omega_two_ = omega_two_ || s.K * s.B * s.W > kOmegaOneCta;
   n_ir_ = offs_ir[np];
   total += header_bytes(np, n_k_);
   if (async_alloc_) W90G_CHECK(cudaMallocAsync(&arena_, total, stream()));
@@ -683,7 +687,7 @@ void Engine::launch_omega(cudaStream_t s, int slot) {
   const int np = nprob();
   const WorkMap wmc{d_offs_chunk_, np};
   k_omega_p1<<<n_chunk_, 256, 0, s>>>(dprobs_, wmc, slot);
-  k_omega_p2<<<n_chunk_, 256, 0, s>>>(dprobs_, wmc, slot);
+  if (!(slot & kOmegaFused) || omega_two_) k_omega_p2<<<n_chunk_, 256, 0, s>>>(dprobs_, wmc, slot);
 }
 
 // tensor path: keep the entry M and U, iterate on R = U0^H U starting from identity
@@ -742,22 +746,25 @@ void Engine::launch_iteration(cudaStream_t s) {
   const WorkMap wmkb{d_offs_kb_, np};
   const WorkMap wmg{d_offs_grad_, np};
   if (guide_w_) k_phases<<<dim3(guide_w_, np), 256, 0, s>>>(dprobs_, 1);
-  k_grad<<<n_grad_, 256, 0, s>>>(dprobs_, wmg);
-  if (n_ir_) k_sym_grad<<<n_ir_, 256, 0, s>>>(dprobs_, WorkMap{d_offs_ir_, np});
-  if (pc_tiles_) {
-    k_precond<<<dim3(pc_tiles_, np), 256, 0, s>>>(dprobs_, 0);
-    k_precond<<<dim3(pc_tiles_, np), 256, 0, s>>>(dprobs_, 1);
+  if (n_ir_ || pc_tiles_) {
+    k_grad<<<n_grad_, 256, 0, s>>>(dprobs_, wmg);
+    if (n_ir_) k_sym_grad<<<n_ir_, 256, 0, s>>>(dprobs_, WorkMap{d_offs_ir_, np});
+    if (pc_tiles_) {
+      k_precond<<<dim3(pc_tiles_, np), 256, 0, s>>>(dprobs_, 0);
+      k_precond<<<dim3(pc_tiles_, np), 256, 0, s>>>(dprobs_, 1);
+    }
+    k_ctrl_search<<<np, 256, 0, s>>>(dprobs_);
+    if (n_ir_) k_sym_dir<<<n_ir_, 256, 0, s>>>(dprobs_, WorkMap{d_offs_ir_, np});
+  } else {
+    k_grad_search<<<n_grad_, 256, 0, s>>>(dprobs_, wmg);
   }
-  k_ctrl_search<<<np, 256, 0, s>>>(dprobs_);
-  if (n_ir_) k_sym_dir<<<n_ir_, 256, 0, s>>>(dprobs_, WorkMap{d_offs_ir_, np});
+  // (k_ctrl_step and k_ctrl_end run in the spread passes' last CTAs)
   launch_exp(s, 0);
   launch_mupdate(s, 0);
-  launch_omega(s, 0);
-  k_ctrl_step<<<(np + 127) / 128, 128, 0, s>>>(dprobs_, np);
+  launch_omega(s, kOmegaFused);
   launch_exp(s, 1);
   launch_mupdate(s, 1);
-  launch_omega(s, 1);
-  k_ctrl_end<<<np, 128, 0, s>>>(dprobs_);
+  launch_omega(s, kOmegaFused + 1);
 }
 
 int Engine::begin(std::string& err) {
@@ -799,9 +806,11 @@ int Engine::advance(int n, int* d_flag, std::string& err) {
   cudaStream_t st = stream();
   n = std::min(n, max_iter_ - launched_iters_);
   for (int i = 0; i < n; ++i) W90G_CHECK(cudaGraphLaunch(graph_exec_, st));
-  // grad, search, 2 x (exp, M update, 2 spread passes), step, end (+ 2 precond)
-  launches_ += (10LL + 2 * (tiles3_ ? 3 : (tensor_wp_ ? 2 : 1)) + (pc_tiles_ ? 2 : 0) + (guide_w_ ? 1 : 0) + (n_ir_ ? 2 : 0)) *
-                std::max(n, 0);
+  // grad (with the search), 2 x (exp, M update, 1 or 2 spread passes); precond: 2 and the search;
+  // symmetry: 2 and the search
+  launches_ += (1LL + 2 * (1 + (tiles3_ ? 3 : (tensor_wp_ ? 2 : 1)) + (omega_two_ ? 2 : 1)) + (pc_tiles_ ? 2 : 0) +
+                (n_ir_ ? 2 : 0) + (pc_tiles_ || n_ir_ ? 1 : 0) + (guide_w_ ? 1 : 0)) *
+               std::max(n, 0);
   launched_iters_ += std::max(n, 0);
   if (d_flag) {
     // every problem done (converged or out of iterations) -> *d_flag = 1

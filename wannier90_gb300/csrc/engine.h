@@ -139,6 +139,7 @@ class Engine {
   int guide_w_ = 0;      // > 0: some problem uses guiding centres; CTAs per problem of k_phases
   int maxW_small_ = 0;   // largest W <= 32 in the batch (shared-memory kernels)
   int tiles3_ = 0;           // num_wann > 32 on the tensor path: 128-row tiles of the largest group
+  bool omega_two_ = false;   // some problem needs the spread's second pass as a launch of its own
   int tensor_wp_ = 0;    // > 0: tensor M update with padded width 8..128 for the whole batch
   bool tensor_exp_ = false;  // exp(s D) on the tensor cores (k_oz_exp)
   bool pipe_ = false;        // tensor M update by the pipelined kernel (tensor_wp_ <= 32)

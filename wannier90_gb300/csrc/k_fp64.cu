@@ -26,10 +26,23 @@ constexpr int kSmemW = 32;   // W <= kSmemW: all per-matrix operands live in sha
 // ----------------------------------------------------------------------------
 // C = op(A) * B for W x W column-major matrices (generic pointers: shared or global).
 // CA: op(A) = A^H (A read as conj(A[i*lda+l])), else op(A) = A.
-// Each thread computes a 2x2 micro-tile of C.  C must not alias A or B.
+// C must not alias A or B.  W <= kSmemW (operands in shared memory): one element per thread.  The
+// FP64 pipe takes 17 cycles per warp instruction whatever its active lanes, so the 2 x 2 micro-tiles
+// that wider matrices use (fewer loads per FMA) cost a 4 x 4 product four times and an 8 x 8 one
+// twice the instructions; the sums over l are the same.
 template <bool CA>
 __device__ void cta_gemm(double2* __restrict__ C, int ldc, const double2* __restrict__ A, int lda,
                          const double2* __restrict__ B, int ldb, int W) {
+  if (W <= kSmemW) {
+    for (int e = threadIdx.x; e < W * W; e += blockDim.x) {
+      const int i = e % W, j = e / W;
+      double2 c = cmk(0, 0);
+#pragma unroll 4
+      for (int l = 0; l < W; ++l) cfma(c, CA ? cconj(A[i * lda + l]) : A[l * lda + i], B[j * ldb + l]);
+      C[j * ldc + i] = c;
+    }
+    return;
+  }
   const int nb = (W + 1) >> 1;
   for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {
     const int i0 = (t % nb) * 2, j0 = (t / nb) * 2;
@@ -103,6 +116,122 @@ __global__ void k_mdiag(const Problem* __restrict__ probs, WorkMap wm) {
 }
 
 // ----------------------------------------------------------------------------
+// k_ctrl_step: internal_optimal_step (src/wannierise.F90:1528-1596).  One thread per problem.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ void ctrl_step(const Problem& P) {
+  CtrlState* st = P.st;
+  const Control& c = P.ctl;
+  if (c.lfixstep) {
+    st->lquad = 0;
+    st->do_second = 0;
+    return;
+  }
+  const double trial = st->slot[0].om_tot, cur = st->wann.om_tot;
+  double fac = trial - cur, shift;
+  if (fabs(fac) > 2.2250738585072014e-308) {   // tiny(1.0_dp)
+    fac = 1.0 / fac;
+    shift = 1.0;
+  } else {
+    fac = 1.0e6;
+    shift = fac * trial - fac * cur;
+  }
+  const double eqb = fac * st->doda0;
+  const double eqa = shift - eqb * c.trial_step;
+  int lquad;
+  double alphamin, falphamin;
+  if (fabs(eqa / (fac * cur)) > 2.220446049250313e-16) {
+    lquad = 1;
+    alphamin = -0.5 * eqb / eqa * (c.trial_step * c.trial_step);
+    falphamin = cur - 0.25 * eqb * eqb / (fac * eqa) * (c.trial_step * c.trial_step);
+  } else {
+    lquad = 0;
+    alphamin = c.trial_step;
+    falphamin = trial;
+  }
+  if (st->doda0 * alphamin > 0.0) {
+    lquad = 0;
+    alphamin = c.trial_step;
+    falphamin = trial;
+  }
+  st->lquad = lquad;
+  st->alphamin = alphamin;
+  st->falphamin = falphamin;
+  st->do_second = lquad;
+  st->s_second = alphamin / (4.0 * P.wbtot);
+}
+
+__global__ void k_ctrl_step(const Problem* __restrict__ probs, int nprob) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < nprob && !probs[p].st->done) ctrl_step(probs[p]);
+}
+
+// ----------------------------------------------------------------------------
+// k_ctrl_end: spread bookkeeping, log line, convergence (internal_test_convergence,
+// src/wannierise.F90:1076-1164), buffer flip.  One CTA (128 threads) per problem.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ void ctrl_end(const Problem& P) {
+  CtrlState* st = P.st;
+  const int W = P.W;
+  const int acc = st->do_second ? 1 : 0;
+  // accepted centres -> slot 2
+  const double* src = P.centres + (size_t)acc * 4 * W;
+  double* dst = P.centres + (size_t)2 * 4 * W;
+  double* lgc = P.log_centres + (size_t)(st->iter + 1) * 4 * W;
+  for (int i = threadIdx.x; i < 4 * W; i += blockDim.x) {
+    dst[i] = src[i];
+    lgc[i] = src[i];
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const Control& c = P.ctl;
+  st->old = st->wann;
+  st->wann = st->slot[acc];
+  st->cur ^= 1;
+  const int iter = st->iter + 1;
+  st->iter = iter;
+  double* lg = P.log + (size_t)iter * kLogStride;
+  lg[0] = iter;
+  lg[1] = st->wann.om_tot - st->old.om_tot;
+  lg[2] = sqrt(fabs(st->gcnorm1));
+  lg[3] = st->wann.om_tot;
+  lg[4] = st->wann.om_d;
+  lg[5] = st->wann.om_od;
+  lg[6] = st->lquad;
+  lg[7] = st->alphamin;
+  unsigned long long tns;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(tns));
+  lg[8] = (double)tns;
+  lg[9] = st->wann.om_nu;
+  if (c.conv_window > 1) {
+    const double delta = st->wann.om_tot - st->old.om_tot;
+    const int cw = c.conv_window;
+    if (iter <= cw) {
+      st->history[iter - 1] = delta;
+    } else {
+      for (int j = 0; j < cw - 1; ++j) st->history[j] = st->history[j + 1];
+      st->history[cw - 1] = delta;
+    }
+    st->conv_count += 1;
+    if (st->conv_count >= cw) {
+      bool ok = true;
+      for (int j = 0; j < cw; ++j)
+        if (fabs(st->history[j]) > c.conv_tol) ok = false;
+      if (ok) st->lconverged = 1;   // conv_noise_amp > 0 is rejected on the host
+    }
+  }
+  if (st->lconverged || iter >= c.num_iter) st->done = 1;
+  if (!isfinite(st->wann.om_tot)) {
+    st->error = 1;
+    st->done = 1;
+  }
+}
+
+__global__ void k_ctrl_end(const Problem* __restrict__ probs) {
+  const Problem& P = probs[blockIdx.x];
+  if (!P.st->done) ctrl_end(P);
+}
+
+// ----------------------------------------------------------------------------
 // wann_omega (src/wannierise.F90:1979-2284) as a deterministic two-pass reduction over
 // nchunk chunks of consecutive (k,b) blocks (at most kOmegaChunk each; the engine makes as many
 // chunks of at least 16 blocks as the chip has SMs):
@@ -145,6 +274,69 @@ __device__ __forceinline__ bool last_chunk_cta(unsigned* arrive, int nchunk) {
   return last;
 }
 
+// kOmegaFused in a pass's slot: the last CTA of the trial's and of the optimal step's second pass
+// goes on with k_ctrl_step and k_ctrl_end, and the first pass of a problem of at most kOmegaOneCta
+// statistics (k,b,n) also does the second's work in its last CTA: one SM's FP64 pipe takes ~4 ns
+// for each, a launch of its own 8 to 10 us.
+constexpr int kOmegaFused = 16, kOmegaOneCta = 3072;
+__device__ __forceinline__ bool omega_one(const Problem& P, int slot) {
+  return (slot & kOmegaFused) != 0 && P.K * P.B * P.W <= kOmegaOneCta;
+}
+
+// the slot's spread from the Omega_D sum (one thread)
+__device__ __forceinline__ void omega_final(const Problem& P, int slot, double dsum) {
+  CtrlState* st = P.st;
+  const int K = P.K;
+  const double od = st->omega_tot[0], oi = st->omega_tot[1];
+  Spread sp;
+  if (P.slwf_num > 0) {
+    // Omega_tot = Omega_IOD + Omega_D + Omega_nu (Omega_I is never formed); om_od
+    // carries Omega_IOD + Omega_nu, what the reference prints as O_IOD
+    const double iod = od / (double)K;
+    sp.om_nu = oi / (double)K + P.slwf_nu0;
+    sp.om_i = 0.0;
+    sp.om_d = (1.0 - P.slwf_lambda) * dsum / (double)K;
+    sp.om_od = iod + sp.om_nu;
+    sp.om_tot = iod + sp.om_d + sp.om_nu;
+  } else {
+    if ((slot == 2) && st->first_pass) {
+      st->om_invariant = oi / (double)K;
+      st->first_pass = 0;
+    }
+    sp.om_i = st->om_invariant;
+    sp.om_d = dsum / (double)K;
+    sp.om_od = od / (double)K;
+    sp.om_tot = sp.om_i + sp.om_d + sp.om_od;
+    sp.om_nu = 0.0;
+  }
+  if (slot == 2) st->wann = sp;
+  else st->slot[slot] = sp;
+  if (!isfinite(sp.om_tot)) {
+    st->error = 1;
+    st->done = 1;
+  }
+}
+
+// sum wb (ln_n + b.rave_n)^2 of this thread's part of the blocks [kb0, kb1)
+__device__ __forceinline__ double omega_dd(const Problem& P, const double* cen, int kb0, int kb1) {
+  const int W = P.W, B = P.B;
+  const int t = threadIdx.x, nsub = blockDim.x / W;
+  const int n = t % W, sub = t / W;
+  double dd = 0.0;
+  // selective localisation: Omega_D over the objective WFs only
+  if (sub < nsub && (P.slwf_num == 0 || n < P.slwf_num)) {
+    const double x0 = cen[n], x1 = cen[W + n], x2 = cen[2 * W + n];
+#pragma unroll 4
+    for (int kb = kb0 + sub; kb < kb1; kb += nsub) {
+      const double w = P.wb[kb % B];
+      const double* bv = P.bk + (size_t)kb * 3;
+      const double l = P.diag_ln[(size_t)kb * W + n] + (bv[0] * x0 + bv[1] * x1 + bv[2] * x2);
+      dd = fma(w * l, l, dd);
+    }
+  }
+  return dd;
+}
+
 __device__ __forceinline__ bool omega_skip(const CtrlState* st, int slot) {
   if (slot < 2) {
     if (st->done) return true;
@@ -159,7 +351,12 @@ __global__ void __launch_bounds__(256) k_omega_p1(const Problem* __restrict__ pr
   const int p = locate(wm, blockIdx.x, ch);
   const Problem& P = probs[p];
   CtrlState* st = P.st;
-  if (omega_skip(st, slot)) return;
+  const bool one = omega_one(P, slot);
+  slot &= kOmegaFused - 1;
+  if (omega_skip(st, slot)) {
+    if (one && slot == 1 && ch == 0 && !st->done) ctrl_end(P);
+    return;
+  }
   const int W = P.W, B = P.B;
   const int KB = P.K * B;
   const int per = (KB + P.nchunk - 1) / P.nchunk;
@@ -295,6 +492,18 @@ __global__ void __launch_bounds__(256) k_omega_p1(const Problem* __restrict__ pr
     cen[3 * W + i] = s_q[i] / (double)P.K - (x0 * x0 + x1 * x1 + x2 * x2);
   }
   if (t == 0) st->omega_arrive[0] = 0u;
+  if (!one) return;
+  // ---- few statistics: the second pass here
+  __syncthreads();
+  const double acc = block_sum(omega_dd(P, cen, 0, KB), red);
+  if (t == 0) {
+    omega_final(P, slot, acc);
+    if (slot == 0 && !st->done) ctrl_step(P);
+  }
+  if (slot == 1) {
+    __syncthreads();
+    if (!st->done) ctrl_end(P);
+  }
 }
 
 __global__ void __launch_bounds__(256) k_omega_p2(const Problem* __restrict__ probs, WorkMap wm, int slot) {
@@ -303,65 +512,31 @@ __global__ void __launch_bounds__(256) k_omega_p2(const Problem* __restrict__ pr
   const int p = locate(wm, blockIdx.x, ch);
   const Problem& P = probs[p];
   CtrlState* st = P.st;
-  if (omega_skip(st, slot)) return;
-  const int W = P.W, B = P.B, K = P.K;
-  const int KB = K * B;
-  const int per = (KB + P.nchunk - 1) / P.nchunk;
-  const int kb0 = ch * per, kb1 = min(KB, kb0 + per);
-  const int t = threadIdx.x;
-  const int nsub = blockDim.x / W;
-  const int n = t % W, sub = t / W;
-  // rave from pass 1's last CTA (the slot's centres)
-  const double* cen = P.centres + (size_t)slot * 4 * W;
-  double dd = 0.0;
-  // selective localisation: Omega_D over the objective WFs only
-  if (sub < nsub && (P.slwf_num == 0 || n < P.slwf_num)) {
-    const double x0 = cen[n], x1 = cen[W + n], x2 = cen[2 * W + n];
-#pragma unroll 4
-    for (int kb = kb0 + sub; kb < kb1; kb += nsub) {
-      const double w = P.wb[kb % B];
-      const double* bv = P.bk + (size_t)kb * 3;
-      const double l = P.diag_ln[(size_t)kb * W + n] + (bv[0] * x0 + bv[1] * x1 + bv[2] * x2);
-      dd = fma(w * l, l, dd);
-    }
+  const bool fused = (slot & kOmegaFused) != 0;
+  if (omega_one(P, slot)) return;   // done by the first pass
+  slot &= kOmegaFused - 1;
+  if (omega_skip(st, slot)) {
+    if (fused && slot == 1 && ch == 0 && !st->done) ctrl_end(P);
+    return;
   }
-  dd = block_sum(dd, red);
-  if (t == 0) P.opart2[ch] = dd;
+  const int KB = P.K * P.B;
+  const int per = (KB + P.nchunk - 1) / P.nchunk;
+  // rave from pass 1's last CTA (the slot's centres)
+  const double dd = block_sum(omega_dd(P, P.centres + (size_t)slot * 4 * P.W, ch * per, min(KB, (ch + 1) * per)), red);
+  if (threadIdx.x == 0) P.opart2[ch] = dd;
   if (!last_chunk_cta(&st->omega_arrive[1], P.nchunk)) return;
   // ---- the last CTA: the Omega_D total, then the spread of the slot
   double acc = 0.0;
-  for (int c = t; c < P.nchunk; c += blockDim.x) acc += __ldcg(P.opart2 + c);
+  for (int c = threadIdx.x; c < P.nchunk; c += blockDim.x) acc += __ldcg(P.opart2 + c);
   acc = block_sum(acc, red);
-  if (t == 0) {
-    const double od = st->omega_tot[0], oi = st->omega_tot[1], dsum = acc;
-    Spread sp;
-    if (P.slwf_num > 0) {
-      // Omega_tot = Omega_IOD + Omega_D + Omega_nu (Omega_I is never formed); om_od
-      // carries Omega_IOD + Omega_nu, what the reference prints as O_IOD
-      const double iod = od / (double)K;
-      sp.om_nu = oi / (double)K + P.slwf_nu0;
-      sp.om_i = 0.0;
-      sp.om_d = (1.0 - P.slwf_lambda) * dsum / (double)K;
-      sp.om_od = iod + sp.om_nu;
-      sp.om_tot = iod + sp.om_d + sp.om_nu;
-    } else {
-      if ((slot == 2) && st->first_pass) {
-        st->om_invariant = oi / (double)K;
-        st->first_pass = 0;
-      }
-      sp.om_i = st->om_invariant;
-      sp.om_d = dsum / (double)K;
-      sp.om_od = od / (double)K;
-      sp.om_tot = sp.om_i + sp.om_d + sp.om_od;
-      sp.om_nu = 0.0;
-    }
-    if (slot == 2) st->wann = sp;
-    else st->slot[slot] = sp;
-    if (!isfinite(sp.om_tot)) {
-      st->error = 1;
-      st->done = 1;
-    }
+  if (threadIdx.x == 0) {
+    omega_final(P, slot, acc);
     st->omega_arrive[1] = 0u;
+    if (fused && slot == 0 && !st->done) ctrl_step(P);
+  }
+  if (fused && slot == 1) {
+    __syncthreads();
+    if (!st->done) ctrl_end(P);
   }
 }
 
@@ -413,7 +588,10 @@ __device__ __forceinline__ bool grad_q(const Problem& P, double w, double l, dou
 // G on both; a CTA with ti > tj only clears its partial slots.
 constexpr int kGradBC = 8;   // b values whose coefficients are staged together
 
-__global__ void __launch_bounds__(256) k_grad(const Problem* __restrict__ probs, WorkMap wm) {
+// Narrow problems are latency bound on the FP64 pipe (17 cycles per warp instruction, whatever the
+// number of active lanes), so a tile's elements and coefficients sit on consecutive threads: 8 x 8
+// blocks fill 2 warps instead of a quarter of 8 (17.4 -> 12 us at num_wann 8 on 64 k).
+__device__ __forceinline__ void grad_body(const Problem* __restrict__ probs, const WorkMap& wm) {
   __shared__ double2 s_alpha[2][kGradBC][kTile];
   __shared__ double2 sP[2][kTile * (kTile + 1)];   // sP[t][j*(33)+i]: P tile t, row i, column j
   __shared__ double red[256];
@@ -444,20 +622,22 @@ __global__ void __launch_bounds__(256) k_grad(const Problem* __restrict__ probs,
     const int R0 = (pass == 0 ? ti : tj) * kTile, C0 = (pass == 0 ? tj : ti) * kTile;
     const int nr = min(kTile, W - R0), nc = min(kTile, W - C0);
     double2 acc[4];
-    int vrow[4];
+    int vrow[4], ei[4], ej[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       acc[q] = cmk(0, 0);
-      const int i = (t + 256 * q) % kTile;
-      vrow[q] = (R0 + i < S) ? 0 : 1;
+      const int e = t + 256 * q;
+      ei[q] = e % nr;
+      ej[q] = e / nr;
+      vrow[q] = (R0 + ei[q] < S) ? 0 : 1;
     }
     for (int b0 = 0; b0 < B; b0 += kGradBC) {
       const int nb = min(kGradBC, B - b0);
       __syncthreads();   // the previous chunk's coefficients are consumed
       // coefficients of the chunk: thread (bl, u) for column n = C0 + u of block b0 + bl
       {
-        const int bl = t / kTile, u = t % kTile;
-        if (bl < nb && u < nc) {
+        const int bl = t / nc, u = t % nc;
+        if (bl < nb) {
           const int b = b0 + bl, n = C0 + u;
           const double w = P.wb[b];
           const double* bv = P.bk + ((size_t)k * B + b) * 3;
@@ -481,17 +661,13 @@ __global__ void __launch_bounds__(256) k_grad(const Problem* __restrict__ probs,
         const double2* Mb = Mk + (size_t)(b0 + bl) * W * W;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int e = t + 256 * q;
-          const int i = e % kTile, j = e / kTile;
-          if (i < nr && j < nc) cfma(acc[q], Mb[(size_t)(C0 + j) * W + R0 + i], s_alpha[vrow[q]][bl][j]);
+          if (ej[q] < nc) cfma(acc[q], Mb[(size_t)(C0 + ej[q]) * W + R0 + ei[q]], s_alpha[vrow[q]][bl][ej[q]]);
         }
       }
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = t + 256 * q;
-      sP[pass][(e / kTile) * (kTile + 1) + e % kTile] = acc[q];
-    }
+    for (int q = 0; q < 4; ++q)
+      if (ej[q] < nc) sP[pass][ej[q] * (kTile + 1) + ei[q]] = acc[q];
   }
   __syncthreads();
   // G = fac (P - P^H) on tile (ti,tj) and, off the diagonal, on tile (tj,ti):
@@ -509,8 +685,8 @@ __global__ void __launch_bounds__(256) k_grad(const Problem* __restrict__ probs,
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int e = t + 256 * q;
-      const int i = e % kTile, j = e / kTile;
-      if (i < nr && j < nc) {
+      const int i = e % nr, j = e / nr;
+      if (j < nc) {
         const double2 a = mine[j * (kTile + 1) + i];
         const double2 c = tr[i * (kTile + 1) + j];   // P_nm: row j, column i of the transposed tile
         const double2 g = cmk(fac * (a.x - c.x), fac * (a.y + c.y));
@@ -529,6 +705,8 @@ __global__ void __launch_bounds__(256) k_grad(const Problem* __restrict__ probs,
     P.gpart[(size_t)local * 2 + 1] = gd;
   }
 }
+
+__global__ void __launch_bounds__(256) k_grad(const Problem* __restrict__ probs, WorkMap wm) { grad_body(probs, wm); }
 
 // ----------------------------------------------------------------------------
 // k_phases: wann_phases (src/wannierise.F90:1756-1976) for guiding centres.
@@ -749,17 +927,14 @@ __global__ void __launch_bounds__(256) k_precond(const Problem* __restrict__ pro
 // handed to k_exp_u, and <G,D> = |G|^2 + gcfac*<G,D_prev> comes from k_grad's partials.
 // One CTA (256 threads) per problem.
 // ----------------------------------------------------------------------------
-__global__ void k_ctrl_search(const Problem* __restrict__ probs) {
-  __shared__ double red[256];
-  const Problem& P = probs[blockIdx.x];
+__device__ __forceinline__ void ctrl_search(const Problem& P, double* red) {
   CtrlState* st = P.st;
-  if (st->done) return;
   const int nt = (P.W + kTile - 1) / kTile;
   const int n = P.K * nt * nt;
   double g2 = 0.0, gd = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    g2 += P.gpart[(size_t)i * 2];
-    gd += P.gpart[(size_t)i * 2 + 1];
+    g2 += __ldcg(P.gpart + (size_t)i * 2);
+    gd += __ldcg(P.gpart + (size_t)i * 2 + 1);
   }
   g2 = block_sum(g2, red);
   gd = block_sum(gd, red);
@@ -836,6 +1011,28 @@ __global__ void k_ctrl_search(const Problem* __restrict__ probs) {
   st->do_second = 0;
 }
 
+__global__ void k_ctrl_search(const Problem* __restrict__ probs) {
+  __shared__ double red[256];
+  const Problem& P = probs[blockIdx.x];
+  if (P.st->done) return;
+  ctrl_search(P, red);
+}
+
+// k_grad and, in the last CTA of each problem, k_ctrl_search: one launch less per iteration where
+// nothing comes between the two (no symmetry, no preconditioner)
+__global__ void __launch_bounds__(256) k_grad_search(const Problem* __restrict__ probs, WorkMap wm) {
+  __shared__ double red[256];
+  int local;
+  const Problem& P = probs[locate(wm, blockIdx.x, local)];
+  CtrlState* st = P.st;
+  if (st->done) return;
+  grad_body(probs, wm);
+  const int nt = (P.W + kTile - 1) / kTile;
+  if (!last_chunk_cta(&st->grad_arrive, P.K * nt * nt)) return;
+  ctrl_search(P, red);
+  if (threadIdx.x == 0) st->grad_arrive = 0u;
+}
+
 // ----------------------------------------------------------------------------
 // C = A * B where the product is known to be Hermitian (sign = +1) or anti-Hermitian
 // (sign = -1): only the upper-triangular 2x2 tiles are computed (whole warps skip the
@@ -843,6 +1040,16 @@ __global__ void k_ctrl_search(const Problem* __restrict__ probs) {
 // ----------------------------------------------------------------------------
 __device__ void cta_gemm_sym(double2* __restrict__ C, const double2* __restrict__ A,
                              const double2* __restrict__ B, int W, double sign) {
+  if (W <= kSmemW) {
+    for (int e = threadIdx.x; e < W * (W + 1) / 2; e += blockDim.x) {
+      int i, j;
+      tri_index(e, i, j);
+      double2 c = cmk(0, 0);
+#pragma unroll 4
+      for (int l = 0; l < W; ++l) cfma(c, A[l * W + i], B[j * W + l]);
+      C[j * W + i] = c;
+    }
+  } else {
   const int nb = (W + 1) >> 1;
   const int ntri = nb * (nb + 1) / 2;
   for (int t = threadIdx.x; t < ntri; t += blockDim.x) {
@@ -873,6 +1080,7 @@ __device__ void cta_gemm_sym(double2* __restrict__ C, const double2* __restrict_
       C[(j0 + 1) * W + i0] = c01;
       if (i1) C[(j0 + 1) * W + i0 + 1] = c11;
     }
+  }
   }
   __syncthreads();
   for (int e = threadIdx.x; e < W * W; e += blockDim.x) {
@@ -906,6 +1114,24 @@ __device__ const double kInvFact[17] = {
     2.0876756987868100e-09, 1.6059043836821613e-10, 1.1470745597729725e-11,
     7.6471637318198164e-13, 4.7794773323873853e-14};
 
+// The number of halvings that bring v >= 0 to theta (a positive normal) or below, at most 60, from
+// the bits with integer operations (halving is exact, and non-negative doubles order like their
+// bit patterns): v 2^-j <= theta first holds at j = e_v - e_theta, or one later where v's mantissa
+// exceeds theta's.  0 for nan, 60 for inf.
+__device__ __forceinline__ int halvings(double v, double theta) {
+  constexpr long long kMant = 0x000FFFFFFFFFFFFFLL;
+  union {
+    double d;
+    long long b;
+  } a, t;
+  a.d = v;
+  t.d = theta;
+  if (a.b <= t.b) return 0;
+  if ((a.b >> 52) == 0x7FF && (a.b & kMant) != 0) return 0;
+  const int j = (int)(a.b >> 52) - (int)(t.b >> 52) + ((a.b & kMant) > (t.b & kMant) ? 1 : 0);
+  return j > 60 ? 60 : j;
+}
+
 __device__ double2* cta_expm(double2* X, double2* Y2, double2* Y3, double2* Y4, double2* R,
                              double2* T, int W, double* red, double* cost_out) {
   const int WW = W * W;
@@ -916,30 +1142,35 @@ __device__ double2* cta_expm(double2* X, double2* Y2, double2* Y3, double2* Y4, 
     colmax = fmax(colmax, s);
   }
   const double nrm = block_max(colmax, red);
-  // candidate degrees (theta_m with a 5% margin for the tail of the series)
-  const int cand_m[5] = {4, 6, 8, 12, 16};
-  const int cand_p[5] = {4, 3, 4, 4, 4};
-  const double cand_theta[5] = {1.6e-3, 1.68e-2, 6.6e-2, 0.32, 0.78};
-  const double cand_cost[5] = {1.5, 2.0, 2.5, 3.5, 4.5};
-  int m = 16, p = 4, js = 0;
-  double best = 1e300;
-  for (int c = 0; c < 5; ++c) {
-    int j = 0;
-    double v = nrm;
-    while (v > cand_theta[c] && j < 60) {
-      v *= 0.5;
-      ++j;
+  // candidate degrees (theta_m with a 5% margin for the tail of the series).  One thread plans: by
+  // all 256 the halvings' FP64 instructions took 7 of the 37 us of a num_wann 8 exp.
+  __shared__ double s_plan[5];
+  if (threadIdx.x == 0) {
+    const int cand_m[5] = {4, 6, 8, 12, 16};
+    const int cand_p[5] = {4, 3, 4, 4, 4};
+    const double cand_theta[5] = {1.6e-3, 1.68e-2, 6.6e-2, 0.32, 0.78};
+    const int cand_cost[5] = {3, 4, 5, 7, 9};   // half products
+    int m = 16, p = 4, js = 0, best = 1 << 30;
+    for (int c = 0; c < 5; ++c) {
+      const int j = halvings(nrm, cand_theta[c]);
+      const int cost = cand_cost[c] + 2 * j;
+      if (cost < best) {
+        best = cost;
+        m = cand_m[c];
+        p = cand_p[c];
+        js = j;
+      }
     }
-    const double cost = cand_cost[c] + j;
-    if (cost < best) {
-      best = cost;
-      m = cand_m[c];
-      p = cand_p[c];
-      js = j;
-    }
+    s_plan[0] = m;
+    s_plan[1] = p;
+    s_plan[2] = js;
+    s_plan[3] = 0.5 * best;
+    s_plan[4] = ldexp(1.0, -js);
   }
-  *cost_out = best;
-  const double sc = ldexp(1.0, -js);
+  __syncthreads();
+  const int m = (int)s_plan[0], p = (int)s_plan[1], js = (int)s_plan[2];
+  *cost_out = s_plan[3];
+  const double sc = s_plan[4];
   for (int e = threadIdx.x; e < WW; e += blockDim.x) X[e] = cscale(X[e], sc);
   __syncthreads();
   // powers: Y2 Hermitian, Y3 = Y2 X anti-Hermitian, Y4 = Y2 Y2 Hermitian
@@ -1097,118 +1328,6 @@ __global__ void __launch_bounds__(256) k_m_update(const Problem* __restrict__ pr
     __syncthreads();
     block_stats(Mout, W, W, P.diag_ln + (size_t)kb * W, P.diag_abs2 + (size_t)kb * W, P.offd + kb, red, &P,
                 (size_t)kb);
-  }
-}
-
-// ----------------------------------------------------------------------------
-// k_ctrl_step: internal_optimal_step (src/wannierise.F90:1528-1596).  One thread per problem.
-// ----------------------------------------------------------------------------
-__global__ void k_ctrl_step(const Problem* __restrict__ probs, int nprob) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nprob) return;
-  const Problem& P = probs[p];
-  CtrlState* st = P.st;
-  if (st->done) return;
-  const Control& c = P.ctl;
-  if (c.lfixstep) {
-    st->lquad = 0;
-    st->do_second = 0;
-    return;
-  }
-  const double trial = st->slot[0].om_tot, cur = st->wann.om_tot;
-  double fac = trial - cur, shift;
-  if (fabs(fac) > 2.2250738585072014e-308) {   // tiny(1.0_dp)
-    fac = 1.0 / fac;
-    shift = 1.0;
-  } else {
-    fac = 1.0e6;
-    shift = fac * trial - fac * cur;
-  }
-  const double eqb = fac * st->doda0;
-  const double eqa = shift - eqb * c.trial_step;
-  int lquad;
-  double alphamin, falphamin;
-  if (fabs(eqa / (fac * cur)) > 2.220446049250313e-16) {
-    lquad = 1;
-    alphamin = -0.5 * eqb / eqa * (c.trial_step * c.trial_step);
-    falphamin = cur - 0.25 * eqb * eqb / (fac * eqa) * (c.trial_step * c.trial_step);
-  } else {
-    lquad = 0;
-    alphamin = c.trial_step;
-    falphamin = trial;
-  }
-  if (st->doda0 * alphamin > 0.0) {
-    lquad = 0;
-    alphamin = c.trial_step;
-    falphamin = trial;
-  }
-  st->lquad = lquad;
-  st->alphamin = alphamin;
-  st->falphamin = falphamin;
-  st->do_second = lquad;
-  st->s_second = alphamin / (4.0 * P.wbtot);
-}
-
-// ----------------------------------------------------------------------------
-// k_ctrl_end: spread bookkeeping, log line, convergence (internal_test_convergence,
-// src/wannierise.F90:1076-1164), buffer flip.  One CTA (128 threads) per problem.
-// ----------------------------------------------------------------------------
-__global__ void k_ctrl_end(const Problem* __restrict__ probs) {
-  const Problem& P = probs[blockIdx.x];
-  CtrlState* st = P.st;
-  if (st->done) return;
-  const int W = P.W;
-  const int acc = st->do_second ? 1 : 0;
-  // accepted centres -> slot 2
-  const double* src = P.centres + (size_t)acc * 4 * W;
-  double* dst = P.centres + (size_t)2 * 4 * W;
-  double* lgc = P.log_centres + (size_t)(st->iter + 1) * 4 * W;
-  for (int i = threadIdx.x; i < 4 * W; i += blockDim.x) {
-    dst[i] = src[i];
-    lgc[i] = src[i];
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  const Control& c = P.ctl;
-  st->old = st->wann;
-  st->wann = st->slot[acc];
-  st->cur ^= 1;
-  const int iter = st->iter + 1;
-  st->iter = iter;
-  double* lg = P.log + (size_t)iter * kLogStride;
-  lg[0] = iter;
-  lg[1] = st->wann.om_tot - st->old.om_tot;
-  lg[2] = sqrt(fabs(st->gcnorm1));
-  lg[3] = st->wann.om_tot;
-  lg[4] = st->wann.om_d;
-  lg[5] = st->wann.om_od;
-  lg[6] = st->lquad;
-  lg[7] = st->alphamin;
-  unsigned long long tns;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(tns));
-  lg[8] = (double)tns;
-  lg[9] = st->wann.om_nu;
-  if (c.conv_window > 1) {
-    const double delta = st->wann.om_tot - st->old.om_tot;
-    const int cw = c.conv_window;
-    if (iter <= cw) {
-      st->history[iter - 1] = delta;
-    } else {
-      for (int j = 0; j < cw - 1; ++j) st->history[j] = st->history[j + 1];
-      st->history[cw - 1] = delta;
-    }
-    st->conv_count += 1;
-    if (st->conv_count >= cw) {
-      bool ok = true;
-      for (int j = 0; j < cw; ++j)
-        if (fabs(st->history[j]) > c.conv_tol) ok = false;
-      if (ok) st->lconverged = 1;   // conv_noise_amp > 0 is rejected on the host
-    }
-  }
-  if (st->lconverged || iter >= c.num_iter) st->done = 1;
-  if (!isfinite(st->wann.om_tot)) {
-    st->error = 1;
-    st->done = 1;
   }
 }
 

@@ -98,6 +98,7 @@ struct CtrlState {
   // last one reduces the chunk partials and sets the count back to 0), and the Omega_OD,
   // Omega_I chunk totals that pass 1's last CTA hands to pass 2's
   unsigned omega_arrive[2];
+  unsigned grad_arrive, pad_arrive;
   double omega_tot[2];
 };
 
