@@ -93,8 +93,54 @@ __device__ __forceinline__ void tri_index(int e, int& i, int& j) {
   i = e - j * (j + 1) / 2;
 }
 
-// One sweep of rotations over all pairs of H, applied to V; pairs with |H_pq| <= tiny or
-// |H_pq|^2 <= thr are skipped.  Returns how many pairs this thread rotated.
+// 1 / sqrt(x) to FP64 for x in FP32's normal range, from FP32 and two Newton steps: 8 FP64
+// operations, where the FP64 square root and divide take about 40 each
+__device__ __forceinline__ double jac_rsqrt(double x) {
+  double y = (double)(1.0f / sqrtf((float)x));
+  y = y * (1.5 - 0.5 * x * y * y);
+  return y * (1.5 - 0.5 * x * y * y);
+}
+
+// Rotation of the pair block [[a, b], [conj(b), d]], b2 = |b|^2 > 0: c, s e^{i phi} and the rotated
+// block (pp, off, qq).  The angle needs no more than FP32 -- it leaves 1e-7 of b for the next sweep,
+// which the sweeps' quadratic convergence hides -- but c and the phase are unitary to FP64, and the
+// block is formed for the angle taken.  (Angle, c and phase in FP64 were 38 % of an m = 26 sweep.)
+__device__ __forceinline__ void jac_rotation(double a, double d, double2 b, double b2, double& c, double2& se,
+                                             double& pp, double& qq, double2& off) {
+  double rinv;
+  if (b2 > 1.0e-30 && b2 < 1.0e30) rinv = jac_rsqrt(b2);
+  else rinv = 1.0 / sqrt(b2);
+  const double ab = b2 * rinv, g = d - a;
+  const float th = (float)(0.5 * g * rinv);
+  const float ath = fabsf(th);
+  // (beyond 1e15 the angle is 1 / (2 th); th^2 would overflow)
+  const float tf = ath < 1.0e15f ? 1.0f / (ath + sqrtf(1.0f + th * th)) : 0.5f / ath;
+  const double t = th >= 0.0f ? (double)tf : -(double)tf;
+  c = jac_rsqrt(1.0 + t * t);
+  const double s = t * c, cs = c * s, ss = s * s;
+  const double2 ph = cmk(b.x * rinv, b.y * rinv);
+  se = cmk(s * ph.x, s * ph.y);
+  const double x = 2.0 * cs * ab - ss * g;     // a - x, d + x
+  pp = a - x;
+  qq = d + x;
+  const double o = (1.0 - 2.0 * ss) * ab - cs * g;
+  off = cmk(o * ph.x, o * ph.y);
+}
+__device__ __forceinline__ void jac_rotation(float a, float d, JacF2 b, float b2, float& c, JacF2& se, float& pp,
+                                             float& qq, JacF2& off) {
+  const float ab = sqrtf(b2), th = (d - a) / (2.0f * ab);
+  const float tt = (th >= 0.0f ? 1.0f : -1.0f) / (fabsf(th) + sqrtf(1.0f + th * th));
+  c = 1.0f / sqrtf(1.0f + tt * tt);
+  const float s = tt * c / ab;
+  se.x = s * b.x;
+  se.y = s * b.y;
+  pp = a - tt * ab;
+  qq = d + tt * ab;
+  off.x = off.y = 0.0f;
+}
+
+// One sweep of rotations over all pairs of H, applied to V; pairs with |H_pq|^2 <= tiny
+// or <= thr are skipped.  Returns how many pairs this thread rotated.
 template <class R, class R2>
 __device__ __forceinline__ int jac_sweep(R2* H, R2* V, int W, R thr, R tiny, R* rc, R2* rse, int* rp, int* rq) {
   const int n = (W + 1) & ~1;     // even number of players (one dummy when W is odd)
@@ -124,20 +170,16 @@ __device__ __forceinline__ int jac_sweep(R2* H, R2* V, int W, R thr, R tiny, R* 
       if (q < W) {
         const R2 b = H[q * W + p];
         const R b2 = b.x * b.x + b.y * b.y;
-        const R ab = sqrt(b2);
-        if (ab > tiny && b2 > thr) {
+        if (b2 > tiny && b2 > thr) {
           live = 1;
           ++rotated;
-          const R a = H[p * W + p].x, d = H[q * W + q].x;
-          const R th = (d - a) / (R(2) * ab);
-          const R tt = (th >= R(0) ? R(1) : R(-1)) / (fabs(th) + sqrt(R(1) + th * th));
-          c = R(1) / sqrt(R(1) + tt * tt);
-          const R s = tt * c / ab;
-          se = jac_mk<R, R2>(s * b.x, s * b.y);
-          // the pair's own block: diag(a - t |b|, d + t |b|)
-          H[p * W + p] = jac_mk<R, R2>(a - tt * ab, R(0));
-          H[q * W + q] = jac_mk<R, R2>(d + tt * ab, R(0));
-          H[q * W + p] = H[p * W + q] = jac_mk<R, R2>(R(0), R(0));
+          R pp, qq;
+          R2 off;
+          jac_rotation(H[p * W + p].x, H[q * W + q].x, b, b2, c, se, pp, qq, off);
+          H[p * W + p] = jac_mk<R, R2>(pp, R(0));
+          H[q * W + q] = jac_mk<R, R2>(qq, R(0));
+          H[q * W + p] = off;
+          H[p * W + q] = jac_conj(off);
         }
       }
       rp[t] = p;
@@ -305,7 +347,7 @@ __device__ __noinline__ static int cta_jacobi(double2* H, double2* V, int W, int
     }
     if (off <= conv * fro || off == 0.0) return sweep;
     if (sweep == max_sweeps) break;
-    const int rotated = jac_sweep<double, double2>(H, V, W, skip * fro, 1.0e-300, rc, rse, rp, rq);
+    const int rotated = jac_sweep<double, double2>(H, V, W, skip * fro, 1.0e-290, rc, rse, rp, rq);
     if (skip > 0.0 && block_sum((double)rotated, red) == 0.0) return sweep + 1;
   }
   return -1;

@@ -77,6 +77,8 @@ struct DisDev {
   const double2* sym_db;
   double2* sym_ws;
   int* sym_status;
+  double2* zfroz;        // [k] nb x nb: the frozen states' part of Zf (it never changes); null: not split off
+  double2* V;            // [k] nb x W (leading dimension nb): U_opt U0 for the final rotation; null: not formed
   const int* pstat;      // [k] kPolarDone where k_oz_polar has formed this kernel's polar factor; null: never
 };
 
@@ -327,6 +329,40 @@ __global__ void __launch_bounds__(256) k_dis_froz(DisDev D) {
 // overlaps:  sum_b w_b |U(k)^H M_w U(k+b)|_F^2 = tr(U^H Zf U), and for a frozen column
 // e_f of U the row sum is Zf_ff.  Upper triangle summed, lower mirrored.  With
 // want_omega, also wk[k] = W wbtot - Re tr(U^H Zf U) (Omega_I(i) part, :2480-2500).
+//
+// Bound by the FP64 pipe, so frozen states are used twice: a frozen column of U is a unit vector,
+// its column of C_b a column of M_w, and their part of Zf the same in every iteration
+// (k_dis_zfroz, once); the other columns are zero on the frozen states, which leaves
+// n' - nf' terms per element of C_b and W - nf' columns.  Where 12 to 16 of 38 to 42 states are
+// frozen (48 bands to 32, 512 k) that is 43 % of the FMAs.
+
+// upper triangle of Z += w C C^H, C n x w columns (ldc), Z n x n (ldz)
+__device__ void cta_zherk(double2* Z, int ldz, const double2* C, int ldc, int n, int wc, double w) {
+  for (int e = threadIdx.x; e < n * (n + 1) / 2; e += blockDim.x) {
+    int p, q;
+    tri_index(e, p, q);
+    double2 acc = cmk(0, 0);
+#pragma unroll 4
+    for (int l = 0; l < wc; ++l) cfma(acc, C[(size_t)l * ldc + p], cconj(C[(size_t)l * ldc + q]));
+    double2& z = Z[(size_t)q * ldz + p];
+    z = cadd(z, cscale(acc, w));
+  }
+}
+
+__global__ void __launch_bounds__(256) k_dis_zfroz(DisDev D) {
+  const int k = blockIdx.x;
+  const int nb = D.nb, n = D.ndim[k], B = D.B;
+  const size_t NN = (size_t)nb * nb;
+  double2* Z = D.zfroz + (size_t)k * NN;
+  for (int e = threadIdx.x; e < (int)NN; e += blockDim.x) Z[e] = cmk(0, 0);
+  __syncthreads();
+  for (int b = 0; b < B; ++b) {
+    const int k2 = D.nnlist[k * B + b];
+    // (each element belongs to one thread: no barrier between the b)
+    cta_zherk(Z, nb, D.Mw + ((size_t)k * B + b) * NN + (size_t)D.ffirst[k2] * nb, nb, n, min(D.nfroz[k2], D.W), D.wb[b]);
+  }
+}
+
 __global__ void __launch_bounds__(256) k_dis_z(DisDev D, int cur, int to_in, int want_omega) {
   __shared__ double red[256];
   const int k = blockIdx.x;
@@ -335,23 +371,29 @@ __global__ void __launch_bounds__(256) k_dis_z(DisDev D, int cur, int to_in, int
   double2* ws = D.ws + (size_t)k * kWs * NN;
   double2* Zacc = ws + NN;
   double2* Z = (to_in ? D.Zin : D.Zout) + (size_t)k * NN;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) Zacc[e] = cmk(0, 0);
+  const double2* Zf = D.zfroz ? D.zfroz + (size_t)k * NN : nullptr;
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x)
+    Zacc[e] = Zf ? Zf[(size_t)(e / n) * nb + e % n] : cmk(0, 0);
   for (int b = 0; b < B; ++b) {
     const int k2 = D.nnlist[k * B + b];
     const int n2 = D.ndim[k2];
+    // split: columns nf2.. of U, which are zero on rows [f2, f2 + nf2)
+    const int nf2 = Zf ? min(D.nfroz[k2], W) : 0, f2 = Zf ? D.ffirst[k2] : 0, wc = W - nf2;
     const double2* Mw = D.Mw + ((size_t)k * B + b) * NN;
-    const double2* U2 = D.U[cur] + (size_t)k2 * nb * W;
+    const double2* U2 = D.U[cur] + (size_t)k2 * nb * W + (size_t)nf2 * nb;
     __syncthreads();
-    cta_zgemm(ws, nb, Mw, nb, false, U2, nb, false, n, W, n2);   // C_b (n x W)
-    __syncthreads();
-    const double w = D.wb[b];
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      const int p = e % n, q = e / n;
-      if (p > q) continue;
+    for (int e = threadIdx.x; e < n * wc; e += blockDim.x) {   // C_b
+      const int i = e % n, j = e / n;
       double2 acc = cmk(0, 0);
-      for (int l = 0; l < W; ++l) cfma(acc, ws[(size_t)l * nb + p], cconj(ws[(size_t)l * nb + q]));
-      Zacc[e] = cadd(Zacc[e], cscale(acc, w));
+      const int cut = nf2 > 0 ? f2 : n2;
+#pragma unroll 4
+      for (int l = 0; l < cut; ++l) cfma(acc, Mw[(size_t)l * nb + i], U2[(size_t)j * nb + l]);
+#pragma unroll 4
+      for (int l = cut + nf2; l < n2; ++l) cfma(acc, Mw[(size_t)l * nb + i], U2[(size_t)j * nb + l]);
+      ws[(size_t)j * nb + i] = acc;
     }
+    __syncthreads();
+    cta_zherk(Zacc, n, ws, nb, n, wc, D.wb[b]);
   }
   __syncthreads();
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
@@ -360,14 +402,17 @@ __global__ void __launch_bounds__(256) k_dis_z(DisDev D, int cur, int to_in, int
   }
   if (!want_omega) return;
   __syncthreads();
-  // tr(U^H Zf U) = sum_{j} sum_p conj(U_pj) (Zf U)_pj
+  // tr(U^H Zf U) = sum_{j} sum_p conj(U_pj) (Zf U)_pj; a frozen column gives Zf_ff
   const double2* Uk = D.U[cur] + (size_t)k * nb * W;
+  const int nf = Zf ? min(D.nfroz[k], W) : 0, ff = Zf ? D.ffirst[k] : 0;
   double t = 0.0;
-  for (int e = threadIdx.x; e < n * W; e += blockDim.x) {
-    const int p = e % n, j = e / n;
+  for (int j = threadIdx.x; j < nf; j += blockDim.x) t += Z[(size_t)(ff + j) * nb + ff + j].x;
+  for (int e = threadIdx.x; e < n * (W - nf); e += blockDim.x) {
+    const int p = e % n, j = nf + e / n;
+    const double2 u = Uk[(size_t)j * nb + p];
+    if (nf > 0 && p >= ff && p < ff + nf) continue;   // u is zero there
     double2 acc = cmk(0, 0);
     for (int q = 0; q < n; ++q) cfma(acc, Z[(size_t)q * nb + p], Uk[(size_t)j * nb + q]);
-    const double2 u = Uk[(size_t)j * nb + p];
     t += u.x * acc.x + u.y * acc.y;
   }
   t = block_sum(t, red);
@@ -508,6 +553,15 @@ __global__ void __launch_bounds__(256) k_dis_findu(DisDev D, int cur) {
   if (threadIdx.x == 0 && sh.flag) D.status[k] = 10 + sh.flag;
 }
 
+// ---- V = U_opt U0: with it the two rotations of M below are one (n + n' and not n + n' + 2 W inner
+// terms per element)
+__global__ void __launch_bounds__(256) k_dis_v(DisDev D, int cur) {
+  const int k = blockIdx.x;
+  const int nb = D.nb, W = D.W;
+  cta_zgemm(D.V + (size_t)k * kWs * nb * nb, nb, D.U[cur] + (size_t)k * nb * W, nb, false, D.U0 + (size_t)k * W * W, W,
+            false, D.ndim[k], W, W);
+}
+
 // ---- dis_main's M_opt = U_opt^H M U_opt' (:220-235) and setup_m_loc's U0^H M_opt U0', per (k,b)
 __global__ void __launch_bounds__(256) k_dis_rotate(DisDev D, int cur) {
   const int kb = blockIdx.x;
@@ -519,6 +573,13 @@ __global__ void __launch_bounds__(256) k_dis_rotate(DisDev D, int cur) {
   extern __shared__ double2 sm[];   // W x nb + 2 W x W
   double2 *T1 = sm, *T2 = sm + (size_t)W * nb, *T3 = T2 + (size_t)W * W;
   const double2* Mw = D.Mw + (size_t)kb * NN;
+  if (D.V) {
+    const size_t sv = (size_t)kWs * NN;
+    cta_zgemm(T1, W, D.V + (size_t)k * sv, nb, true, Mw, nb, false, W, n2, n);      // W x n2
+    __syncthreads();
+    cta_zgemm(D.M0 + (size_t)kb * W * W, W, T1, W, false, D.V + (size_t)k2 * sv, nb, false, W, W, n2);
+    return;
+  }
   const double2* Uk = D.U[cur] + (size_t)k * nb * W;
   const double2* U2 = D.U[cur] + (size_t)k2 * nb * W;
   cta_zgemm(T1, W, Uk, nb, true, Mw, nb, false, W, n2, n);      // W x n2
@@ -995,7 +1056,8 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
                o_zin = take((size_t)K * NN * 16), o_zout = take((size_t)K * NN * 16),
                o_uw = take((size_t)K * W * W * 16), o_m0 = take((size_t)K * B * W * W * 16),
                o_ws = take((size_t)K * kWs * NN * 16), o_wk1 = take(K * 8), o_wk = take(K * 8),
-               o_st = take(K * 4), o_ps = take(K * 4), o_vz = take((size_t)K * NN * 16), o_sw = take(4);
+               o_rw = take(W >= 9 ? (size_t)std::min(kRotateCtas, K * B) * 4 * NN * 16 : 0), o_rf = take(4),
+               o_st = take(K * 4), o_ps = take(K * 4), o_zf = take(any_froz && nir == 0 ? (size_t)K * NN * 16 : 0), o_vz = take((size_t)K * NN * 16), o_sw = take(4);
   // symmetry tables: ik, moff, mem, goff, grp, status; slot matrices; workspace
   std::vector<int> sym_ints;
   if (nir > 0) {
@@ -1009,7 +1071,11 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   int mmax = 0;
   for (int k = 0; k < K; ++k) mmax = std::max(mmax, ndim[k] - nfroz[k]);
   const size_t step_smem = 3 * (size_t)mmax * mmax * 16;
-  int cur = 0, it = 0;
+  // threads of k_dis_step: a round of rotations of an m x m matrix has (m/2)(m/2-1)/2 blocks of H
+  // and m m/2 elements of V, 60 at m = 8, and two CTA barriers: two warps up to m = 12
+  const int step_threads = mmax <= 12 ? 64 : 256;
+  int cur = 0, it = 0, rot_failed = 0;
+  char* a0 = nullptr;
   double womegai = 0.0;
   cudaStream_t st = s.stream;
   bool own_stream = false;
@@ -1044,7 +1110,7 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   DIS_CHECK(cudaFuncSetAttribute(k_dis_rotate, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDisMaxSmem));
   DIS_CHECK(cudaMallocAsync(&arena, off, st));
   {
-    char* a = (char*)arena;
+    char* a = a0 = (char*)arena;
     D.nb = nb;
     D.W = W;
     D.K = K;
@@ -1073,6 +1139,8 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
     D.wk = (double*)(a + o_wk);
     D.status = (int*)(a + o_st);
     D.pstat = (const int*)(a + o_ps);
+    D.zfroz = any_froz && nir == 0 ? (double2*)(a + o_zf) : nullptr;
+    D.V = (double2*)(a + o_ws) + 6 * NN;   // a slot of the workspace that nothing else uses then
     D.Vz = (double2*)(a + o_vz);
     D.max_sweeps = (int*)(a + o_sw);
     D.sym_nir = nir;
@@ -1109,6 +1177,7 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   DIS_CHECK(cudaMemcpyAsync(D.U[0], s.A, (size_t)K * nb * W * 16, in_kind, st));
   DIS_CHECK(cudaMemsetAsync(D.status, 0, K * 4, st));
   DIS_CHECK(cudaMemsetAsync(D.max_sweeps, 0, 4, st));
+  DIS_CHECK(cudaMemsetAsync(a0 + o_rf, 0, 4, st));
   // The polar factors on the tensor cores first (k_oz_polar; from 9 bands on, as in the
   // projection of an isolated group); the kernels after it take what it left alone.
   {
@@ -1143,6 +1212,7 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   // symmetry-adapted U_opt (src/disentangle.F90:186-190)
   if (nir > 0) DIS_CHECK(launch(kDisSym, [&] { k_dis_sym_u<<<nir, 256, 0, st>>>(D, cur, 0); }));
   // ---- dis_extract iterations
+  if (D.zfroz) DIS_CHECK(launch(kDisFroz, [&] { k_dis_zfroz<<<K, 256, 0, st>>>(D); }));
   DIS_CHECK(launch(kDisZ, [&] { k_dis_z<<<K, 256, 0, st>>>(D, cur, 1, 0); }));
   if (nir > 0) DIS_CHECK(launch(kDisSym, [&] { k_dis_sym_z<<<nir, 256, 0, st>>>(D, 0); }));
   r.log.clear();
@@ -1152,7 +1222,7 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
       DIS_CHECK(launch(kDisSym, [&] { k_dis_sym_step<<<nir, 256, 0, st>>>(D, cur, it); }));
       DIS_CHECK(launch(kDisSym, [&] { k_dis_sym_u<<<nir, 256, 0, st>>>(D, cur ^ 1, 0); }));
     } else {
-      DIS_CHECK(launch(kDisStep, [&] { k_dis_step<<<K, 256, step_smem, st>>>(D, cur, it); }));
+      DIS_CHECK(launch(kDisStep, [&] { k_dis_step<<<K, step_threads, step_smem, st>>>(D, cur, it); }));
     }
     DIS_CHECK(launch(kDisZ, [&] { k_dis_z<<<K, 256, 0, st>>>(D, cur ^ 1, 0, 1); }));
     if (nir > 0) DIS_CHECK(launch(kDisSym, [&] { k_dis_sym_z<<<nir, 256, 0, st>>>(D, 1); }));
@@ -1207,10 +1277,35 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   DIS_CHECK(launch(kDisFindU, [&] { k_dis_findu<<<K, 256, 0, st>>>(D, cur); }));
   // symmetric initial U with d = D (sitesym_replace_d_matrix_band, :237, :688-692)
   if (nir > 0) DIS_CHECK(launch(kDisSym, [&] { k_dis_sym_u<<<nir, 256, 0, st>>>(D, cur, 1); }));
-  DIS_CHECK(launch(kDisRotate, [&] { k_dis_rotate<<<K * B, 256, rot_smem, st>>>(D, cur); }));
+  DIS_CHECK(launch(kDisFindU, [&] { k_dis_v<<<K, 256, 0, st>>>(D, cur); }));
+  if (W >= 9) {
+    RotateArgs r{};
+    r.m = D.Mw;
+    r.ldm = r.ldv = nb;
+    r.strideM = NN;
+    r.v = D.V;
+    r.strideV = kWs * NN;
+    r.rows = D.ndim;
+    r.w = W;
+    r.n = *std::max_element(ndim.begin(), ndim.end());
+    r.B = B;
+    r.nnlist = D.nnlist;
+    r.out = D.M0;
+    r.work = (double2*)(a0 + o_rw);
+    r.failed = (int*)(a0 + o_rf);
+    DIS_CHECK(launch(kDisRotate, [&] { oz_rotate_launch(r, K * B, st); }));
+    DIS_CHECK(cudaMemcpyAsync(&rot_failed, r.failed, 4, cudaMemcpyDeviceToHost, st));
+  } else {
+    DIS_CHECK(launch(kDisRotate, [&] { k_dis_rotate<<<K * B, 256, rot_smem, st>>>(D, cur); }));
+  }
   DIS_CHECK(cudaMemcpyAsync(status.data(), D.status, K * 4, cudaMemcpyDeviceToHost, st));
   DIS_CHECK(cudaMemcpyAsync(&r.max_sweeps, D.max_sweeps, 4, cudaMemcpyDeviceToHost, st));
   DIS_CHECK(cudaStreamSynchronize(st));
+  if (rot_failed) {
+    err = "disentangle: a bounded wait of the tensor-core rotation ran out";
+    rc = 1;
+    goto done;
+  }
   for (int k = 0; k < K; ++k) {
     if (status[k]) {
       err = "disentangle: eigensolver failure or rank-deficient U_opt^H A at k-point " + std::to_string(k + 1);

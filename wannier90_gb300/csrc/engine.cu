@@ -35,7 +35,6 @@ __global__ void k_lowdin(const Problem* probs, WorkMap wm, int* status);
 __global__ void k_unitarity(const Problem* probs, WorkMap wm, double* out);
 __global__ void k_all_done(const Problem* probs, int nprob, int* out);
 __global__ void k_fp64_peak(double* out, int iters, double seed);
-__global__ void k_u_final(const Problem* probs, WorkMap wm);
 __global__ void k_u_identity(const Problem* probs, WorkMap wm);
 __global__ void k_precond(const Problem* probs, int dir);
 __global__ void k_phases(const Problem* probs, int mode);
@@ -43,6 +42,7 @@ __global__ void k_phases(const Problem* probs, int mode);
 __global__ void k_sym_grad(const Problem* probs, WorkMap wm);
 __global__ void k_sym_dir(const Problem* probs, WorkMap wm);
 __global__ void k_sym_u(const Problem* probs, WorkMap wm);
+cudaError_t oz_ufinal_launch(int wp, const Problem* probs, WorkMap wm, int grid, cudaStream_t s);
 cudaError_t oz3_launch(int wp, const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, cudaStream_t s);
 cudaError_t oz3_preslice_launch(int wp, const Problem* probs, WorkMap wm, int ngroups, int tmax, cudaStream_t s);
 cudaError_t oz3_set_attributes(int wp);
@@ -490,7 +490,6 @@ int Engine::alloc(std::string& err) {
   // of different widths may run concurrently in the batched form)
   constexpr int wmax = 32;
   W90G_CHECK(cudaFuncSetAttribute(k_exp_u, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * wmax * wmax * 16));
-  W90G_CHECK(cudaFuncSetAttribute(k_u_final, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * wmax * wmax * 16));
   W90G_CHECK(cudaFuncSetAttribute(k_m_update, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * wmax * wmax * 16));
   W90G_CHECK(cudaFuncSetAttribute(k_lowdin, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * wmax * wmax * 16));
   tensor_exp_ = tensor_wp_ != 0;
@@ -677,8 +676,35 @@ int Engine::project(std::string& err) {
       }
     }
   }
-  k_m_update<<<n_kb_, 256, 4 * ws * ws * 16, st>>>(dprobs_, wmkb, 1, 0);
-  W90G_CHECK(cudaGetLastError());
+  // M <- U^H M U': tensor cores under the same rule as the polar factors, work in what the
+  // projection does not use (G, D, dU and the second M buffer follow one another only by chance, so
+  // the largest of them, the M buffer)
+  const ProblemSpec& s0 = specs_[0];
+  const size_t mat = (size_t)s0.W * s0.W;
+  if (nprob() == 1 && s0.W >= kPolarMinW && s0.W <= kPolarMaxN &&
+      (size_t)s0.K * s0.B * mat >= (size_t)std::min(kRotateCtas, s0.K * s0.B) * 4 * mat) {
+    RotateArgs r{};
+    r.m = r.out = hprobs_[0].M[0];
+    r.ldm = r.ldv = r.w = r.n = s0.W;
+    r.strideM = r.strideV = mat;
+    r.v = hprobs_[0].U[0];
+    r.B = s0.B;
+    r.nnlist = hprobs_[0].nnlist;
+    r.work = hprobs_[0].M[1];
+    r.failed = d_status_;
+    W90G_CHECK(cudaMemsetAsync(d_status_, 0, sizeof(int), st));
+    W90G_CHECK(oz_rotate_launch(r, s0.K * s0.B, st));
+    int failed = 0;
+    W90G_CHECK(cudaMemcpyAsync(&failed, d_status_, sizeof(int), cudaMemcpyDeviceToHost, st));
+    W90G_CHECK(cudaStreamSynchronize(st));
+    if (failed) {
+      err = "overlap_project: a bounded wait of the tensor-core rotation ran out";
+      return 1;
+    }
+  } else {
+    k_m_update<<<n_kb_, 256, 4 * ws * ws * 16, st>>>(dprobs_, wmkb, 1, 0);
+    W90G_CHECK(cudaGetLastError());
+  }
   launches_ += 1;
   return 0;
 }
@@ -848,8 +874,7 @@ int Engine::finish(std::string& err) {
   const int np = nprob();
   const WorkMap wmk{d_offs_k_, np};
   if (tensor_wp_) {
-    const int ws = std::max(maxW_small_, 1);
-    k_u_final<<<n_k_, 256, (size_t)3 * ws * ws * 16, st>>>(dprobs_, wmk);
+    W90G_CHECK(oz_ufinal_launch(tensor_wp_, dprobs_, wmk, n_k_, st));
     launches_ += 1;
   }
   // final unitarity check (src/wannierise.F90:890-892)

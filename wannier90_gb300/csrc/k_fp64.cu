@@ -1587,8 +1587,8 @@ __global__ void k_fp64_peak(double* __restrict__ out, int iters, double seed) {
 
 // ----------------------------------------------------------------------------
 // Tensor-path bookkeeping: during the loop U[] holds R = U0^H U (identity at entry),
-// M is always recomputed from the entry overlaps M0; at the end U = U0 R.
-// k_u_identity: U[0](k) = I.   k_u_final: U[cur](k) <- U0(k) U[cur](k).
+// M is always recomputed from the entry overlaps M0; at the end U = U0 R (k_oz_ufinal).
+// k_u_identity: U[0](k) = I.
 // One CTA (256 threads) per (problem, k).
 // ----------------------------------------------------------------------------
 __global__ void k_u_identity(const Problem* __restrict__ probs, WorkMap wm) {
@@ -1598,26 +1598,6 @@ __global__ void k_u_identity(const Problem* __restrict__ probs, WorkMap wm) {
   const int W = P.W;
   double2* U = P.U[0] + (size_t)k * W * W;
   for (int e = threadIdx.x; e < W * W; e += blockDim.x) U[e] = cmk((e % W) == (e / W) ? 1.0 : 0.0, 0.0);
-}
-
-__global__ void __launch_bounds__(256) k_u_final(const Problem* __restrict__ probs, WorkMap wm) {
-  extern __shared__ double2 smem[];
-  int k;
-  const int p = locate(wm, blockIdx.x, k);
-  const Problem& P = probs[p];
-  const int W = P.W, WW = W * W;
-  double2* R = P.U[P.st->cur] + (size_t)k * WW;
-  const double2* U0 = P.U0 + (size_t)k * WW;
-  double2* buf = (W <= kSmemW) ? smem : (P.work + (size_t)k * 6 * WW);
-  double2 *sA = buf, *sR = buf + WW, *sC = buf + 2 * WW;
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) {
-    sA[e] = U0[e];
-    sR[e] = R[e];
-  }
-  __syncthreads();
-  cta_gemm<false>(sC, W, sA, W, sR, W, W);
-  __syncthreads();
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) R[e] = sC[e];
 }
 
 }  // namespace w90g

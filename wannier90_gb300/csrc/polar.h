@@ -1,5 +1,5 @@
-// Unitary polar factors on the tensor cores (k_oz_polar.cu): Q = X (X^H X)^{-1/2} of one
-// rows x cols matrix per CTA.
+// Matrix steps outside the iteration on the tensor cores: unitary polar factors Q = X (X^H X)^{-1/2}
+// of one rows x cols matrix per CTA (k_oz_polar.cu), rotations V(k)^H M(k,b) V(k+b) (k_oz_rotate.cu).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -27,6 +27,26 @@ struct PolarArgs {
 
 constexpr int kPolarMats = 4;
 constexpr int kPolarMaxN = 128;
+
+struct RotateArgs {
+  const double2* m;      // [item] n x n blocks, item = k B + b
+  int ldm;
+  size_t strideM;
+  const double2* v;      // [k] rows(k) x w
+  int ldv;
+  size_t strideV;
+  const int* rows;       // [k] rows of V(k), order of M's blocks; null: w
+  int w, n, B;           // n >= rows(k) and w: order of the work matrices
+  const int* nnlist;     // [item] k + b
+  double2* out;          // [item] w x w (may be m)
+  double2* work;         // [kRotateCtas] 4 n x n
+  int* failed;           // set to 1 when a bounded wait ran out
+};
+
+constexpr int kRotateCtas = 304;   // two per SM
+
+// n <= kPolarMaxN
+cudaError_t oz_rotate_launch(const RotateArgs& a, int items, cudaStream_t s);
 
 // K CTAs; n <= kPolarMaxN
 cudaError_t oz_polar_launch(const PolarArgs& a, int K, cudaStream_t s);
