@@ -208,14 +208,14 @@ int odn_of(int W) { return W <= 32 ? 4 : 4 * (W / 32 + 2); }
 
 struct Sizes {
   size_t M, U, KWW, work, tbuf, diag, offd, gpart, cen, log, logc, nn, bk, wb, st, op1, op2, m0, u0, inv, fr;
-  size_t m0s, m0e, zexp, ub2, ub2e, einfo, odp;
+  size_t m0s, m0e, zexp, ub2, ub2e, einfo, odp, zs, zse;
   size_t pkr, pr2, pgr, pgp, ppart;
   size_t gbka, gneigh, grg, gsheet, gcsheet;
   size_t slwf;
   size_t symi, symd, symw;
   size_t total() const {
     return 2 * M + 2 * U + 3 * KWW + work + tbuf + 2 * diag + offd + gpart + cen + log + logc + nn + bk + wb + st +
-           op1 + op2 + m0 + u0 + inv + fr + m0s + m0e + zexp + ub2 + ub2e + einfo + odp + pkr + 2 * pr2 + pgr + pgp + ppart + gbka + gneigh + grg + gsheet +
+           op1 + op2 + m0 + u0 + inv + fr + m0s + m0e + zexp + ub2 + ub2e + einfo + odp + zs + zse + pkr + 2 * pr2 + pgr + pgp + ppart + gbka + gneigh + grg + gsheet +
            gcsheet + slwf + symi + 2 * symd + symw;
   }
 };
@@ -238,7 +238,7 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
   z.inv = wp ? align_up(K * B * 4) : 0;
   z.odp = wp ? align_up(K * B * odn_of(s.W) * 8) : 0;
   z.fr = wp ? align_up(K * B * 8) : 0;
-  z.m0s = z.m0e = 0;
+  z.m0s = z.m0e = z.zs = z.zse = 0;
   z.zexp = (wp && wp <= 32) ? align_up(K * B * W * 4) : 0;
   z.ub2 = z.ub2e = 0;
   if (wp && wp <= 32) {
@@ -250,8 +250,8 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
   if (wp > 32) {
     size_t b[4];
     oz3_bytes((int)W, (int)K, (int)B, b);
-    z.m0s = align_up(b[0]);
-    z.m0e = align_up(b[1]);
+    z.m0s = z.zs = align_up(b[0]);
+    z.m0e = z.zse = align_up(b[1]);
     z.ub2 = align_up(b[2]);
     z.ub2e = align_up(b[3]);
   } else if (wp) {
@@ -417,6 +417,8 @@ int Engine::alloc(std::string& err) {
     P.odn = odn_of(s.W);
     P.m0s = z.m0s ? (unsigned char*)take(z.m0s) : nullptr;
     P.m0s_exp = z.m0e ? (int*)take(z.m0e) : nullptr;
+    P.zs = z.zs ? (unsigned char*)take(z.zs) : nullptr;
+    P.zs_exp = z.zse ? (int*)take(z.zse) : nullptr;
     P.zexp = z.zexp ? (int*)take(z.zexp) : nullptr;
     P.ub2 = z.ub2 ? (unsigned char*)take(z.ub2) : nullptr;
     P.ub2_exp = z.ub2e ? (int*)take(z.ub2e) : nullptr;
@@ -834,7 +836,7 @@ int Engine::advance(int n, int* d_flag, std::string& err) {
   for (int i = 0; i < n; ++i) W90G_CHECK(cudaGraphLaunch(graph_exec_, st));
   // grad (with the search), 2 x (exp, M update, 1 or 2 spread passes); precond: 2 and the search;
   // symmetry: 2 and the search
-  launches_ += (1LL + 2 * (1 + (tiles3_ ? 3 : (tensor_wp_ ? 2 : 1)) + (omega_two_ ? 2 : 1)) + (pc_tiles_ ? 2 : 0) +
+  launches_ += (1LL + 2 * (1 + (tiles3_ ? 4 : (tensor_wp_ ? 2 : 1)) + (omega_two_ ? 2 : 1)) + (pc_tiles_ ? 2 : 0) +
                 (n_ir_ ? 2 : 0) + (pc_tiles_ || n_ir_ ? 1 : 0) + (guide_w_ ? 1 : 0)) *
                std::max(n, 0);
   launched_iters_ += std::max(n, 0);

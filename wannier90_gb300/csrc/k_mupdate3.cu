@@ -6,20 +6,21 @@
 // indices, then their imaginary parts) of 128 rows of A and of one chunk of B, all 7 digit
 // planes of both: 28 KB + at most 14 KB, five stages in flight.
 //
-//   A           step 1: one bulk copy per stage from the digit image of conj(M0), sliced once
-//               per solve (k_oz_preslice3; the conjugate, so that both steps multiply by the
-//               same U: conj(Z)^T = conj(M0)^T U); step 2: 8 warps slice the rows of Z;
+//   A           one bulk copy per stage from a digit image (k_oz_preslice3): step 1's of conj(M0),
+//               sliced once per solve (the conjugate, so that both steps multiply by the same U:
+//               conj(Z)^T = conj(M0)^T U), step 2's of Z, sliced between the steps.  (Eight warps of
+//               the kernel slicing Z's rows for every column chunk took 3.1 ms a step at num_wann
+//               128 on 512 k and 182 us at 48 on 216, against 1.5 ms and 95 us of step 1.)
 //   B           one bulk copy per stage from the digit image of U(k), sliced once per update
 //               (k_oz_slice_u) instead of once per 128-row tile, column chunk and K chunk;
 //   MMA         one thread: 7 to 11 MMAs a stage (plane t of A against as many planes of B as
 //               fit N = 256), committed to the stage's empty barrier;
 //   epilogue    16 warps: exact recombination of the 7 diagonals in int64, FP64 stores, and in
-//               step 2 the diagonal statistics of the spread.
+//               step 2 the diagonal statistics and off-diagonal sums of the spread.
 //
-// What bounds it: the 28 digit-pair MMAs of a 128 x 64 x 16 stage take ~1100 cycles of the tensor
-// pipe; slicing a stage is ~500 issue cycles and a tile's epilogue ~3000, and the 448 accumulator
-// columns of a chunk leave no room for a second set, so the epilogue and the next chunk's MMAs
-// alternate.  Shapes follow num_wann itself, not a padded width: rows of consecutive blocks share
+// What bounds it: a 128 x 64 x 16 stage is 28 digit-pair MMAs, ~1000 cycles of the tensor pipe, and
+// 43 KB from L2; at num_wann 128 the copies run at 5.5 TB/s.  The 448 accumulator columns of a chunk
+// leave no room for a second set, so the epilogue and the next chunk's MMAs alternate.  Shapes follow num_wann itself, not a padded width: rows of consecutive blocks share
 // a tile (B W / 128 tiles), K stops at the next multiple of 8 complex indices and the columns are
 // cut into equal chunks of at most 32, so num_wann 48 costs 3/4 x 3/4 of 64 and not the same.
 //
@@ -46,14 +47,8 @@ constexpr int kStages = (kDynBudget - 1024) / kStage;
 static_assert(kStages >= 3, "shared memory for at least three stages");
 constexpr size_t kSmem3 = (size_t)kStages * kStage + 1024;
 
-template <int STEP>
-struct Roles3 {
-  static constexpr int EPI = 16;
-  static constexpr int PA = STEP == 1 ? 1 : 8;
-  static constexpr int MMA = EPI + PA;
-  static constexpr int THREADS = (MMA + 1) * 32;
-  static constexpr int ET = EPI * 32, PAT = PA * 32;
-};
+// warps: 16 of the epilogue, the one whose first thread issues the copies, the one that issues MMAs
+constexpr int kEpi3 = 16, kCopy3 = 16, kMma3 = 17, kThreads3 = 18 * 32, kEpiThreads3 = kEpi3 * 32;
 
 // geometry of one problem
 struct Geo3 {
@@ -119,34 +114,29 @@ __device__ __forceinline__ void arrive_expect(uint64_t* bar, uint32_t bytes) {
 // Work items: (group, tile), group-major, `tmax` tiles per group (the widest problem's); a
 // persistent grid walks them.  EIGHT: every problem of the launch has num_wann <= 64.
 template <int STEP, bool EIGHT>
-__global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
+__global__ void __launch_bounds__(kThreads3, 1)
     k_oz_mupdate3(const Problem* __restrict__ probs, WorkMap wm, int which, int ngroups, int tmax) {
-  using R = Roles3<STEP>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t a_full[kStages], a_empty[kStages];
-  __shared__ __align__(8) uint64_t acc_full, acc_empty, exp_full[2], drain_bar;
+  __shared__ __align__(8) uint64_t acc_full, acc_empty, drain_bar;
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_rowexp[2][kTileRows];   // step 2: row scales of the tile, by tile parity
   __shared__ volatile int s_bad;
-  __shared__ int s_bad_prob, s_aflag, s_eflag;
+  __shared__ int s_bad_prob, s_eflag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp == R::MMA) {
+  if (warp == kMma3) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                  :: "r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
-      // step 1: the issuing thread's arrival with the copies' bytes; step 2: that and the slicers
-      mbar_init(&a_full[s], STEP == 1 ? 1u : 1u + (uint32_t)R::PAT);
+      mbar_init(&a_full[s], 1u);   // the issuing thread's arrival with the copies' bytes
       mbar_init(&a_empty[s], 1u);
     }
     mbar_init(&acc_full, 1u);
-    mbar_init(&acc_empty, (uint32_t)R::ET);
-    mbar_init(&exp_full[0], (uint32_t)R::PAT);
-    mbar_init(&exp_full[1], (uint32_t)R::PAT);
+    mbar_init(&acc_empty, (uint32_t)kEpiThreads3);
     mbar_init(&drain_bar, 1u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_bad = 0;
@@ -165,111 +155,46 @@ __global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
     }
   };
 
-  if (warp >= R::EPI && warp < R::MMA) {
-    // =========================== producer ===========================
-    const int pa = tid - R::ET;
-    int sseq = 0, tseq = 0;
-    uint32_t inflight = 0, par = 0;   // thread 0: slots with a copy issued, and its parity
-    auto await = [&](uint64_t* bar, uint32_t parity, int p) -> bool {
-      if (pa == 0) {
-        const bool ok = mbar_wait_role(smem_u32(bar), parity, &s_bad);
-        if (!ok) fail(p);
-        s_aflag = ok ? 0 : 1;
-      }
-      if (STEP == 1) return s_aflag == 0;
-      bar_named(1, R::PAT);
-      const bool ok = s_aflag == 0;
-      bar_named(1, R::PAT);
-      return ok;
-    };
-    bool ok = STEP == 2 || pa == 0;
-    for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
-      int g;
-      const int p = locate(wm, item / tmax, g), tile = item % tmax;
-      const Problem& P = probs[p];
-      const int W = P.W, WW = W * W;
-      const Geo3 G = geo3(W, P.B);
-      if (tile >= G.ntiles || !group_active(P, which)) continue;
-      const uint32_t bst = (uint32_t)bstage3(G);
-      const unsigned char* bimg = P.ub2 + (size_t)g * bimage3(G);
-      // step 2: this thread slices part (pa / 128) of row pa % 128, 8 complex per K-step
-      const double* zrow = nullptr;
-      int zex = 0;
-      if (STEP == 2) {
-        const int r = pa % kTileRows, part = pa / kTileRows, row = tile * kTileRows + r;
-        if (row < P.B * W) {
-          const size_t kb = (size_t)P.inv_nnlist[(size_t)g * P.B + row / W];
-          zrow = (const double*)(P.tbuf + kb * WW + (size_t)(row % W) * W) + part;
-        }
-        // the row's scale: the two parts' maxima meet in shared memory (the exponent of the
-        // larger modulus; the integer maximum does not depend on the order)
-        unsigned long long mx = 0ull;
-        if (zrow)
-          for (int m0 = 0; m0 < W; m0 += 8) {
-            double v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = m0 + i < W ? zrow[2 * (m0 + i)] : 0.0;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) mx = max(mx, abs_bits(v[i]));
-          }
-        const int tb = tseq & 1, mine = mx ? exp_above_bits(mx) : -100000;
-        if (part == 0) s_rowexp[tb][r] = mine;
-        bar_named(1, R::PAT);
-        if (part == 1) {
-          const int e = max(mine, s_rowexp[tb][r]);
-          s_rowexp[tb][r] = e == -100000 ? 0 : e;
-        }
-        bar_named(1, R::PAT);
-        zex = s_rowexp[tb][r];
-        mbar_arrive(&exp_full[tb]);
-      }
-      for (int nc = 0; nc < G.nch && ok; ++nc)
-        for (int ks = 0; ks < G.ksteps; ++ks) {
-          const int s = sseq % kStages;
-          const uint32_t use = (uint32_t)(sseq / kStages);
-          double av[8];
-          if (STEP == 2) {
-            // the stage's elements, loaded before the slot is free
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int m = ks * 8 + i;
-              av[i] = (zrow && m < W) ? zrow[2 * m] : 0.0;
+  if (warp == kCopy3) {
+    // =========================== copies ===========================
+    if (lane == 0) {
+      int sseq = 0;
+      uint32_t inflight = 0, par = 0;   // slots with a copy issued, and its parity
+      bool ok = true;
+      for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+        int g;
+        const int p = locate(wm, item / tmax, g), tile = item % tmax;
+        const Problem& P = probs[p];
+        const Geo3 G = geo3(P.W, P.B);
+        if (tile >= G.ntiles || !group_active(P, which)) continue;
+        const uint32_t bst = (uint32_t)bstage3(G);
+        const unsigned char* bimg = P.ub2 + (size_t)g * bimage3(G);
+        const unsigned char* aimg =
+            (STEP == 1 ? P.m0s : P.zs) + ((size_t)g * G.ntiles + tile) * G.ksteps * (size_t)kStageA;
+        for (int nc = 0; nc < G.nch && ok; ++nc)
+          for (int ks = 0; ks < G.ksteps; ++ks) {
+            const int s = sseq % kStages;
+            const uint32_t use = (uint32_t)(sseq / kStages);
+            // (the first use of each stage slot needs no wait)
+            if (use > 0 && !mbar_wait_role(smem_u32(&a_empty[s]), (use & 1) ^ 1, &s_bad)) {
+              fail(p);
+              ok = false;
+              break;
             }
-          }
-          // (the first use of each stage slot needs no wait)
-          if (use > 0 && !await(&a_empty[s], (use & 1) ^ 1, p)) {
-            ok = false;
-            break;
-          }
-          unsigned char* dA = base + (size_t)s * kStage;
-          if (pa == 0) {
-            arrive_expect(&a_full[s], bst + (STEP == 1 ? (uint32_t)kStageA : 0u));
+            unsigned char* dA = base + (size_t)s * kStage;
+            arrive_expect(&a_full[s], bst + (uint32_t)kStageA);
             bulk_copy(dA + kStageA, bimg + ((size_t)nc * G.ksteps + ks) * bst, bst, &a_full[s]);
-            if (STEP == 1)
-              bulk_copy(dA, P.m0s + (((size_t)g * G.ntiles + tile) * G.ksteps + ks) * kStageA, kStageA, &a_full[s]);
+            bulk_copy(dA, aimg + (size_t)ks * kStageA, kStageA, &a_full[s]);
             inflight |= 1u << s;
             par = (par & ~(1u << s)) | ((use & 1) << s);
+            ++sseq;
           }
-          if (STEP == 2) {
-            uint32_t w[kS][4];
-            slice3<EIGHT>(w, av, zex);
-            const uint32_t o = stage_off(pa % kTileRows, 8 * (pa / kTileRows));
-#pragma unroll
-            for (int t = 0; t < kS; ++t)
-              *(uint4*)(dA + (size_t)t * kPlaneA + o) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive(&a_full[s]);
-          }
-          ++sseq;
-        }
-      ++tseq;
-    }
-    // drain: the last copy into each slot must land before the CTA frees its shared memory (the
-    // slicers' arrivals of that phase may be missing after a failure: then only the limit ends it)
-    if (pa == 0)
+      }
+      // drain: the last copy into each slot must land before the CTA frees its shared memory
       for (int s = 0; s < kStages; ++s)
         if (inflight & (1u << s)) mbar_drain(smem_u32(&a_full[s]), (par >> s) & 1);
-  } else if (warp == R::MMA) {
+    }
+  } else if (warp == kMma3) {
     // =========================== MMA issue ===========================
     if (lane == 0) {
       int sseq = 0, useq = 0;
@@ -333,7 +258,7 @@ __global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
     const int wq = warp & 3, cg = warp >> 2;            // TMEM lane quarter, column group
     const int r = wq * 32 + lane;                       // tile row = TMEM lane
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-    int useq = 0, tseq = 0;
+    int useq = 0;
     bool ok = true;
     // one thread waits, the others at the epilogue's named barrier
     auto await = [&](uint64_t* bar, uint32_t parity, int p) -> bool {
@@ -342,9 +267,9 @@ __global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
         if (!o) fail(p);
         s_eflag = o ? 0 : 1;
       }
-      bar_named(2, R::ET);
+      bar_named(2, kEpiThreads3);
       const bool o = s_eflag == 0;
-      bar_named(2, R::ET);
+      bar_named(2, kEpiThreads3);
       return o;
     };
     for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
@@ -359,15 +284,12 @@ __global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
       const bool valid = row < P.B * W;
       const int bi = row / W, rr = row % W;
       size_t kb = 0;
-      int erow = 0;
       if (STEP == 1) {
         kb = (size_t)g * P.B + bi;
-        erow = P.m0s_exp[((size_t)g * G.ntiles + tile) * kTileRows + r];
-      } else {
-        if (valid) kb = (size_t)P.inv_nnlist[(size_t)g * P.B + bi];
-        if (!await(&exp_full[tseq & 1], (uint32_t)(tseq >> 1) & 1, p)) break;
-        erow = s_rowexp[tseq & 1][r];
+      } else if (valid) {
+        kb = (size_t)P.inv_nnlist[(size_t)g * P.B + bi];
       }
+      const int erow = (STEP == 1 ? P.m0s_exp : P.zs_exp)[((size_t)g * G.ntiles + tile) * kTileRows + r];
       double2* dst = (STEP == 1 ? P.tbuf : P.M[cur ^ 1]) + kb * WW + rr;
       const int* ecol = P.ub2_exp + (size_t)g * W;
       double od = 0.0;   // step 2: |M_mn|^2 off the diagonal, this row and column group
@@ -440,12 +362,11 @@ __global__ void __launch_bounds__(Roles3<STEP>::THREADS, 1)
           }
         }
       }
-      ++tseq;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == R::MMA) {
+  if (warp == kMma3) {
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
@@ -520,45 +441,54 @@ __global__ void __launch_bounds__(256) k_oz_slice_u(const Problem* __restrict__ 
   }
 }
 
-// Step 1's A operand, once per solve: the digit planes of conj(M0)^T's rows (k, b, n) in the
-// stage layout, with the row exponents.  One CTA (256 threads) per (k, tile).
-template <bool EIGHT>
-__global__ void __launch_bounds__(256) k_oz_preslice3(const Problem* __restrict__ probs, WorkMap wm, int tmax) {
+// The A operands' digit planes in the stage layout, with the row exponents: STEP 1 conj(M0)^T's rows
+// (k, b, n), once per solve; STEP 2 the rows of Z(k,b) of group k' = nnlist(k,b), between the steps.
+// One CTA (256 threads) per (group, tile).
+template <int STEP, bool EIGHT>
+__global__ void __launch_bounds__(256) k_oz_preslice3(const Problem* __restrict__ probs, WorkMap wm, int tmax,
+                                                      int which) {
   __shared__ int s_rowexp[kTileRows];
   int g;
   const int p = locate(wm, blockIdx.x / tmax, g), tile = blockIdx.x % tmax;
   const Problem& P = probs[p];
   const int W = P.W, WW = W * W, tid = threadIdx.x;
   const Geo3 G = geo3(W, P.B);
-  if (tile >= G.ntiles || !P.m0s) return;
-  const int r = tid >> 1, row = tile * kTileRows + r;
-  const double2* src = row < P.B * W ? P.M0 + ((size_t)g * P.B + row / W) * WW + (size_t)(row % W) * W : nullptr;
+  if (tile >= G.ntiles || (STEP == 2 && !group_active(P, which))) return;
+  unsigned char* img = STEP == 1 ? P.m0s : P.zs;
+  int* exps = STEP == 1 ? P.m0s_exp : P.zs_exp;
+  auto row_of = [&](int row) -> const double2* {
+    if (row >= P.B * W) return nullptr;
+    const size_t gb = (size_t)g * P.B + row / W;
+    return (STEP == 1 ? P.M0 + gb * WW : P.tbuf + (size_t)P.inv_nnlist[gb] * WW) + (size_t)(row % W) * W;
+  };
+  const int r = tid >> 1;
+  const double2* src = row_of(tile * kTileRows + r);
   {
     unsigned long long mx = 0ull;
     if (src)
+#pragma unroll 8
       for (int m = tid & 1; m < W; m += 2) mx = max(mx, max(abs_bits(src[m].x), abs_bits(src[m].y)));
     mx = max(mx, (unsigned long long)__shfl_xor_sync(0xffffffffu, (long long)mx, 1));
     if ((tid & 1) == 0) {
       s_rowexp[r] = exp_above_bits(mx);
-      P.m0s_exp[((size_t)g * G.ntiles + tile) * kTileRows + r] = s_rowexp[r];
+      exps[((size_t)g * G.ntiles + tile) * kTileRows + r] = s_rowexp[r];
     }
   }
   __syncthreads();
-  const int rs = tid % kTileRows, part = tid / kTileRows, rows = tile * kTileRows + rs;
-  const double* s2 = rows < P.B * W
-                         ? (const double*)(P.M0 + ((size_t)g * P.B + rows / W) * WW + (size_t)(rows % W) * W) + part
-                         : nullptr;
+  const int rs = tid % kTileRows, part = tid / kTileRows;
+  const double2* srow = row_of(tile * kTileRows + rs);
+  const double* s2 = srow ? (const double*)srow + part : nullptr;
   for (int ks = 0; ks < G.ksteps; ++ks) {
     double v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int m = ks * 8 + i;
       const double x = (s2 && m < W) ? s2[2 * m] : 0.0;
-      v[i] = part ? -x : x;
+      v[i] = STEP == 1 && part ? -x : x;
     }
     uint32_t w[kS][4];
     slice3<EIGHT>(w, v, s_rowexp[rs]);
-    unsigned char* dst = P.m0s + (((size_t)g * G.ntiles + tile) * G.ksteps + ks) * (size_t)kStageA;
+    unsigned char* dst = img + (((size_t)g * G.ntiles + tile) * G.ksteps + ks) * (size_t)kStageA;
     const uint32_t o = stage_off(rs, 8 * part);
 #pragma unroll
     for (int t = 0; t < kS; ++t)
@@ -568,7 +498,7 @@ __global__ void __launch_bounds__(256) k_oz_preslice3(const Problem* __restrict_
 
 // ---- host side ----------------------------------------------------------------------
 
-// bytes of a problem's digit images and exponents: m0s, m0s_exp, ub2, ub2_exp
+// bytes of a problem's digit images and exponents: m0s (and zs), m0s_exp (and zs_exp), ub2, ub2_exp
 void oz3_bytes(int W, int K, int B, size_t out[4]) {
   const Geo3 G = geo3(W, B);
   out[0] = (size_t)K * G.ntiles * G.ksteps * kStageA;
@@ -598,11 +528,12 @@ template <bool EIGHT>
 static void oz3_launch_e(const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, cudaStream_t s) {
   const int grid = std::min(ngroups * tmax, sm_count());
   k_oz_slice_u<EIGHT><<<ngroups, 256, 0, s>>>(probs, wm, which);
-  k_oz_mupdate3<1, EIGHT><<<grid, Roles3<1>::THREADS, kSmem3, s>>>(probs, wm, which, ngroups, tmax);
-  k_oz_mupdate3<2, EIGHT><<<grid, Roles3<2>::THREADS, kSmem3, s>>>(probs, wm, which, ngroups, tmax);
+  k_oz_mupdate3<1, EIGHT><<<grid, kThreads3, kSmem3, s>>>(probs, wm, which, ngroups, tmax);
+  k_oz_preslice3<2, EIGHT><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, which);
+  k_oz_mupdate3<2, EIGHT><<<grid, kThreads3, kSmem3, s>>>(probs, wm, which, ngroups, tmax);
 }
 
-// the whole update (three launches) of the ngroups work items of wm; wp: the widest problem's
+// the whole update (four launches) of the ngroups work items of wm; wp: the widest problem's
 // padded width, 64 or 128; tmax: the largest tile count of a group
 cudaError_t oz3_launch(int wp, const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, cudaStream_t s) {
   if (wp <= 64) oz3_launch_e<true>(probs, wm, which, ngroups, tmax, s);
@@ -611,8 +542,8 @@ cudaError_t oz3_launch(int wp, const Problem* probs, WorkMap wm, int which, int 
 }
 
 cudaError_t oz3_preslice_launch(int wp, const Problem* probs, WorkMap wm, int ngroups, int tmax, cudaStream_t s) {
-  if (wp <= 64) k_oz_preslice3<true><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax);
-  else k_oz_preslice3<false><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax);
+  if (wp <= 64) k_oz_preslice3<1, true><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, 0);
+  else k_oz_preslice3<1, false><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, 0);
   return cudaGetLastError();
 }
 

@@ -1,9 +1,7 @@
 // Exact slicing helpers shared by the tensor-core kernels (M update, exp): power-of-two
-// scales, signed 7- and 8-bit digits as FP16 (BF16 for the exp's 65..128-wide form),
+// scales, signed 7- and 8-bit digits as FP16,
 // tcgen05 descriptors, exact int64 recombination.  See k_tensor.cu for the scheme.
 #pragma once
-#include <cuda_bf16.h>
-
 #include "w90g.cuh"
 
 namespace w90g {
@@ -29,14 +27,7 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return d;
 }
 
-// instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major, N, M = 128
-// (one MMA never mixes BF16 and FP16 operands)
-__host__ __device__ constexpr uint32_t idesc_bf16(int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
-}
-
-// the same with A = B = F16 (the FP16 digit planes of the M update and of the exp's
-// second product form)
+// instruction descriptor, kind::f16: D = F32, A = B = F16, both K-major, N, M = 128
 __host__ __device__ constexpr uint32_t idesc_f16(int N) {
   return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
 }
@@ -44,12 +35,6 @@ __host__ __device__ constexpr uint32_t idesc_f16(int N) {
 // element (row, k) of a K-major tile with K_real columns, in bytes
 __device__ __forceinline__ uint32_t kmaj_off(int row, int k, int kreal) {
   return (uint32_t)((row >> 3) * (kreal >> 3) * 128 + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
-}
-
-// exact BF16 bits of a small integer (|x| < 2^22): 1.5*2^23 magic, top 16 bits
-__device__ __forceinline__ uint16_t int_to_bf16(int x) {
-  const float f = __int_as_float(0x4B400000 + x) - 12582912.0f;
-  return (uint16_t)(__float_as_uint(f) >> 16);
 }
 
 // exact integer value of an integer-valued float with |f| < 2^22
@@ -109,19 +94,6 @@ __device__ __forceinline__ long long scaled_int56(double v, int e) {
   return (bits < 0) ? -n : n;
 }
 
-// 8 signed 7-bit digits of N (|N| <= 2^56): x_8..x_2 in [-64, 63], |x_1| <= 128,
-// N = sum_t x_t 2^(7(8-t))
-__device__ __forceinline__ void digits8(long long n, int x[8]) {
-#pragma unroll
-  for (int t = 7; t > 0; --t) {
-    const int lo = (int)n & 127;
-    const int d = lo - ((lo & 64) << 1);
-    x[t] = d;
-    n = (n - d) >> 7;
-  }
-  x[0] = (int)n;
-}
-
 // 8-bit-digit form (56 bits in 7 digits): N = round(v * 2^(55 - e)), |N| <= 2^55
 __device__ __forceinline__ long long scaled_int55(double v, int e) {
   const long long bits = __double_as_longlong(v);
@@ -138,7 +110,7 @@ __device__ __forceinline__ long long scaled_int55(double v, int e) {
 }
 
 // 7 signed 8-bit digits of N (|N| <= 2^55): x_7..x_2 in [-128, 127], |x_1| <= 128,
-// N = sum_t x_t 2^(8(7-t)); every digit is an exact BF16 value
+// N = sum_t x_t 2^(8(7-t)); every digit is an exact FP16 value
 __device__ __forceinline__ void digits7x8(long long n, int x[7]) {
 #pragma unroll
   for (int t = 6; t > 0; --t) {
@@ -194,6 +166,30 @@ __device__ __forceinline__ void pack_digits7(uint32_t (&w)[kS][4], const double 
   }
 }
 
+// The eight 7-bit digit planes of 8 values scaled by 2^(56 - ex), packed as above (the centred
+// recoding of N, |N| <= 2^56, into x_8..x_2 in [-64, 63] and |x_1| <= 128).  C = 64 (1 + 2^7 + ... + 2^42); three 14-bit windows, the seventh field on its own, and
+// the top digit (N + C) >> 49 in [-128, 128].
+__device__ __forceinline__ void pack_digits8(uint32_t (&w)[8][4], const double (&v)[8], int ex) {
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    const long long ma = scaled_int56(v[i], ex) + 0x1020408102040LL;
+    const long long mb = scaled_int56(v[i + 1], ex) + 0x1020408102040LL;
+    const uint32_t la = (uint32_t)ma, lb = (uint32_t)mb;
+    const uint32_t ha = (uint32_t)((unsigned long long)ma >> 32), hb = (uint32_t)((unsigned long long)mb >> 32);
+    const uint32_t q[3] = {__byte_perm(la, lb, 0x5410), __byte_perm(la >> 14, lb >> 14, 0x5410),
+                           __byte_perm(__funnelshift_r(la, ha, 28), __funnelshift_r(lb, hb, 28), 0x5410)};
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      w[7 - 2 * j][i >> 1] = f16x2_sub((q[j] & 0x007F007Fu) | 0x64006400u, 0x64406440u);
+      w[6 - 2 * j][i >> 1] = f16x2_sub(((q[j] >> 7) & 0x007F007Fu) | 0x64006400u, 0x64406440u);
+    }
+    const uint32_t s6 = __byte_perm(ha >> 10, hb >> 10, 0x5410);   // bits 42-48
+    w[1][i >> 1] = f16x2_sub((s6 & 0x007F007Fu) | 0x64006400u, 0x64406440u);
+    const uint32_t ta = (uint32_t)((int)(ma >> 49) + 128), tb = (uint32_t)((int)(mb >> 49) + 128);
+    w[0][i >> 1] = f16x2_sub(ta | (tb << 16) | 0x64006400u, 0x64806480u);
+  }
+}
+
 // The seven 8-bit digit planes of the 8 values scaled by 2^(55 - ex), as packed FP16
 // pairs: w[t][i / 2] holds digit t of values i (low half) and i + 1 -- the digits of
 // digits7x8, without its serial recoding.  With C = 128 (1 + 2^8 + ... + 2^40), byte t' of
@@ -231,28 +227,6 @@ __device__ __forceinline__ int float_to_int_exact24(float f) {
   return (fabsf(f) < 4194304.0f) ? float_to_int_exact(f) : __float2int_rn(f);
 }
 
-// double of S * 2^sc for a 128-bit S, rounded to nearest even, integer ops only
-__device__ __forceinline__ double int128_scaled_to_double(__int128 S, int sc) {
-  if (S == 0) return 0.0;
-  const unsigned long long sign = (S < 0) ? 0x8000000000000000ull : 0ull;
-  unsigned __int128 a = (S < 0) ? (unsigned __int128)(-S) : (unsigned __int128)S;
-  const unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
-  const int lz = hi ? __clzll(hi) : 64 + __clzll(lo);
-  a <<= lz;                                          // leading 1 at bit 127
-  const unsigned long long top = (unsigned long long)(a >> 64);
-  const bool sticky = (unsigned long long)a != 0ull;
-  unsigned long long m = top >> 11;                  // 53 bits
-  const unsigned long long rem = top & 0x7FFull;
-  if (rem > 0x400ull || (rem == 0x400ull && (sticky || (m & 1ull)))) m += 1ull;
-  int ex = 127 - lz + sc;
-  if (m >> 53) {
-    m >>= 1;
-    ex += 1;
-  }
-  const unsigned long long bits = sign | ((unsigned long long)(ex + 1023) << 52) | (m & 0x000FFFFFFFFFFFFFull);
-  return __longlong_as_double((long long)bits);
-}
-
 // exact double of S * 2^sc (|S| < 2^63) with integer ops only (round to nearest even)
 __device__ __forceinline__ double int64_scaled_to_double(long long S, int sc) {
   if (S == 0) return 0.0;
@@ -286,6 +260,18 @@ __device__ __forceinline__ double recombine7x8(const uint32_t* dd, int stride, i
 #pragma unroll
   for (int d = 5; d < 7; ++d) lo = (lo << 8) + float_to_int_exact24(__uint_as_float(dd[d * stride]));
   return int64_scaled_to_double(hi, sc + 24) + int64_scaled_to_double(lo, sc);
+}
+
+// sum_d D_d 2^(7(7-d)) * 2^sc of the 8 diagonal accumulators of that scheme (|D_d| < 2^24): the top
+// and the bottom four exactly in int64, converted exactly, added once in FP64
+__device__ __forceinline__ double recombine8x7(const uint32_t* dd, int stride, int sc) {
+  long long h = float_to_int_exact24(__uint_as_float(dd[0]));
+#pragma unroll
+  for (int d = 1; d < 4; ++d) h = (h << 7) + float_to_int_exact24(__uint_as_float(dd[d * stride]));
+  long long l = float_to_int_exact24(__uint_as_float(dd[4 * stride]));
+#pragma unroll
+  for (int d = 5; d < 8; ++d) l = (l << 7) + float_to_int_exact24(__uint_as_float(dd[d * stride]));
+  return int64_scaled_to_double(h, sc + 28) + int64_scaled_to_double(l, sc);
 }
 
 // S = sum_d D_d 2^(7(6-d)) of the 7 diagonal accumulators dd[0], dd[stride], ... (exact

@@ -198,6 +198,18 @@ __device__ void epi_apply(const double2* C, const Epi& ep, const Add& add, int W
   __syncthreads();
 }
 
+// Part (0 re, 1 im) of 8 values base[(m0 + i) * stride], i < 8 (zero where m0 + i >= W or
+// !valid): the operand run a thread slices.
+__device__ __forceinline__ void load_run8(double (&v)[8], const double2* base, size_t stride, int m0, int W,
+                                          bool valid, int part) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int m = m0 + i;
+    v[i] = 0.0;
+    if (valid && m < W) v[i] = ((const double*)(base + (size_t)m * stride))[part];
+  }
+}
+
 // C = A B for W x W complex column-major matrices (generic pointers; C must not alias
 // A or B), then the Epi applied from C.  All threads call; returns false (uniformly) if
 // an MMA wait timed out.
@@ -213,43 +225,39 @@ __device__ bool oz_cmm(OzCtx& cx, double2* C, const double2* A, const unsigned* 
   bool ok = true;
   for (int nc = 0; nc < NCH && ok; ++nc) {
     for (int kc = 0; kc < NCH && ok; ++kc) {
-      // ---- A chunk: rows r < WP, complex K index l < CW -> real columns l, l + CW
-      for (int e = tid; e < WP * CW; e += blockDim.x) {
-        const int r = e % WP, l = e / WP;
-        const int m = kc * CW + l;
-        double2 a = make_double2(0.0, 0.0);
-        if (r < W && m < W) a = A[(size_t)m * W + r];
-        int xr[kS8], xi[kS8];
-        const int ex = cx.rowexp[r];
-        digits8(scaled_int56(a.x, ex), xr);
-        digits8(scaled_int56(a.y, ex), xi);
-        const uint32_t o_re = kmaj_off(r, l, KC), o_im = kmaj_off(r, l + CW, KC);
+      // ---- A chunk: rows r < WP, complex K index l < CW -> real columns l, l + CW.  A thread
+      // slices one part of 8 consecutive l of a row into a 16-byte core row per digit plane.
+      constexpr int LG = CW / 8;
+      for (int it = tid; it < WP * LG * 2; it += 256) {
+        const int r = it % WP, lg = (it / WP) % LG, part = it / (WP * LG);
+        double v[8];
+        load_run8(v, A + r, (size_t)W, kc * CW + lg * 8, W, r < W, part);
+        uint32_t w[kS8][4];
+        pack_digits8(w, v, cx.rowexp[r]);
+        const uint32_t o = kmaj_off(r, part * CW + lg * 8, KC);
 #pragma unroll
-        for (int t = 0; t < kS8; ++t) {
-          *(uint16_t*)(cx.sA + (size_t)t * E::A_SLICE + o_re) = int_to_bf16(xr[t]);
-          *(uint16_t*)(cx.sA + (size_t)t * E::A_SLICE + o_im) = int_to_bf16(xi[t]);
-        }
+        for (int t = 0; t < kS8; ++t)
+          *(uint4*)(cx.sA + (size_t)t * E::A_SLICE + o) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
       }
-      // ---- B chunk, embedded [[B_r, B_i], [-B_i, B_r]] stored as B^T (K-major):
-      // row = real N index (c | c + CW), column = real K index (l | l + CW)
-      for (int e = tid; e < CW * CW; e += blockDim.x) {
-        const int l = e % CW, c = e / CW;
-        const int mm = kc * CW + l, cc = nc * CW + c;
-        double2 b = make_double2(0.0, 0.0);
-        if (mm < W && cc < W) b = B[(size_t)cc * W + mm];
-        int xr[kS8], xi[kS8];
-        const int ex = cx.colexp[cc < WP ? cc : 0];
-        digits8(scaled_int56(b.x, ex), xr);
-        digits8(scaled_int56(b.y, ex), xi);
-        const uint32_t o00 = kmaj_off(c, l, KC), o01 = kmaj_off(c + CW, l, KC);
-        const uint32_t o10 = kmaj_off(c, l + CW, KC), o11 = kmaj_off(c + CW, l + CW, KC);
+      // ---- B chunk, embedded [[B_r, B_i], [-B_i, B_r]] stored as B^T (K-major): row = real N
+      // index (c | c + CW), column = real K index (l | l + CW); each part goes to two places
+      for (int it = tid; it < CW * LG * 2; it += 256) {
+        const int c = it % CW, lg = (it / CW) % LG, part = it / (CW * LG);
+        const int cc = nc * CW + c;
+        double v[8];
+        load_run8(v, B + (size_t)cc * W, (size_t)1, kc * CW + lg * 8, W, cc < W, part);
+        uint32_t w[kS8][4];
+        pack_digits8(w, v, cx.colexp[cc < WP ? cc : 0]);
+        // B_r: (K re, N re), (K im, N im);  B_i: (K re, N im), negated (K im, N re)
+        const uint32_t o1 = kmaj_off(part == 0 ? c : c + CW, lg * 8, KC);
+        const uint32_t o2 = kmaj_off(part == 0 ? c + CW : c, CW + lg * 8, KC);
 #pragma unroll
         for (int t = 0; t < kS8; ++t) {
           unsigned char* sb = cx.sB + (size_t)t * E::B_BYTES;
-          *(uint16_t*)(sb + o00) = int_to_bf16(xr[t]);    // (K re, N re) =  B_r
-          *(uint16_t*)(sb + o01) = int_to_bf16(xi[t]);    // (K re, N im) =  B_i
-          *(uint16_t*)(sb + o10) = int_to_bf16(-xi[t]);   // (K im, N re) = -B_i
-          *(uint16_t*)(sb + o11) = int_to_bf16(xr[t]);    // (K im, N im) =  B_r
+          *(uint4*)(sb + o1) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
+          *(uint4*)(sb + o2) = part == 0 ? make_uint4(w[t][0], w[t][1], w[t][2], w[t][3])
+                                         : make_uint4(f16x2_neg(w[t][0]), f16x2_neg(w[t][1]), f16x2_neg(w[t][2]),
+                                                      f16x2_neg(w[t][3]));
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -279,7 +287,7 @@ __device__ bool oz_cmm(OzCtx& cx, double2* C, const double2* A, const unsigned* 
                   "{\n\t.reg .pred p;\n\t"
                   "setp.ne.b32 p, %4, 0;\n\t"
                   "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                  :: "r"(dtm), "l"(ad), "l"(bd), "r"(idesc_bf16(n * NC)), "r"(acc)
+                  :: "r"(dtm), "l"(ad), "l"(bd), "r"(idesc_f16(n * NC)), "r"(acc)
                   : "memory");
             }
           }
@@ -299,17 +307,10 @@ __device__ bool oz_cmm(OzCtx& cx, double2* C, const double2* A, const unsigned* 
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     if (!ok) break;
-    // C(r, c) = (sum_d D_d 2^(7(7-d))) 2^(rowexp + colexp - 63), exact in 128 bits
+    // C(r, c) = (sum_d D_d 2^(7(7-d))) 2^(rowexp + colexp - 63)
     auto recombine = [&](const uint32_t* dr, const uint32_t* di, int stride, int r, int c) {
-      __int128 sr = float_to_int_exact24(__uint_as_float(dr[0]));
-      __int128 si = float_to_int_exact24(__uint_as_float(di[0]));
-#pragma unroll
-      for (int d = 1; d < kS8; ++d) {
-        sr = (sr << 7) + float_to_int_exact24(__uint_as_float(dr[d * stride]));
-        si = (si << 7) + float_to_int_exact24(__uint_as_float(di[d * stride]));
-      }
       const int sc = cx.rowexp[r] + cx.colexp[c] - 63;
-      C[(size_t)c * W + r] = make_double2(int128_scaled_to_double(sr, sc), int128_scaled_to_double(si, sc));
+      C[(size_t)c * W + r] = make_double2(recombine8x7(dr, stride, sc), recombine8x7(di, stride, sc));
     };
     const int wq = warp & 3, half = warp >> 2;
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
@@ -425,18 +426,6 @@ struct Exp2Smem {
   static constexpr size_t FLOOR = 233472 / (512 / TMEM_COLS + 1) - 1024 + 16;
   static constexpr size_t BYTES = NEED > FLOOR ? NEED : FLOOR;
 };
-
-// Part (0 re, 1 im) of 8 values base[(m0 + i) * stride], i < 8 (zero where m0 + i >= W or
-// !valid): the operand run a thread slices.
-__device__ __forceinline__ void load_run8(double (&v)[8], const double2* base, size_t stride, int m0, int W,
-                                          bool valid, int part) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int m = m0 + i;
-    v[i] = 0.0;
-    if (valid && m < W) v[i] = ((const double*)(base + (size_t)m * stride))[part];
-  }
-}
 
 // C = A B, then the Epi.  num_wann <= 32 (staged accumulators): the epilogue applies the
 // Epi itself and writes ep.out only (C unused; ep.out may alias B, whose digits are in

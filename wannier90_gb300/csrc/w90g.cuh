@@ -136,6 +136,8 @@ struct Problem {
   double2* M0;          // tensor path: M at entry (never modified)
   unsigned char* m0s;   // tensor path: step 1's A operand (M0 rows) in BF16 digit planes,
                         // the shared-memory image of every (k, tile, K chunk)
+  unsigned char* zs;    // tensor path, num_wann > 32: step 2's A operand (the rows of Z) likewise
+  int* zs_exp;
   int* m0s_exp;         // tensor path: the row exponents of those tiles [k][tile][128]
   int* zexp;            // pipelined tensor path: step 2's row exponents [k][b][row of Z(k,b)],
                         // written by step 1's epilogue
