@@ -767,6 +767,11 @@ void Engine::launch_exp(cudaStream_t s, int which) {
   }
 }
 
+// k_ctrl_search in the gradient's last CTA: where nothing comes between the two, and up to 512 CTAs --
+// a launch saved is 5 to 9 us there; on 1000 k of num_wann 32 counting the CTAs in costs as much
+// (6.59 ms against 6.54 for the solve's four iterations)
+bool Engine::fuse_search() const { return !n_ir_ && !pc_tiles_ && n_grad_ <= 512; }
+
 void Engine::launch_iteration(cudaStream_t s) {
   const int np = nprob();
   const int ws = std::max(maxW_small_, 1);
@@ -774,7 +779,7 @@ void Engine::launch_iteration(cudaStream_t s) {
   const WorkMap wmkb{d_offs_kb_, np};
   const WorkMap wmg{d_offs_grad_, np};
   if (guide_w_) k_phases<<<dim3(guide_w_, np), 256, 0, s>>>(dprobs_, 1);
-  if (n_ir_ || pc_tiles_) {
+  if (!fuse_search()) {
     k_grad<<<n_grad_, 256, 0, s>>>(dprobs_, wmg);
     if (n_ir_) k_sym_grad<<<n_ir_, 256, 0, s>>>(dprobs_, WorkMap{d_offs_ir_, np});
     if (pc_tiles_) {
@@ -834,10 +839,10 @@ int Engine::advance(int n, int* d_flag, std::string& err) {
   cudaStream_t st = stream();
   n = std::min(n, max_iter_ - launched_iters_);
   for (int i = 0; i < n; ++i) W90G_CHECK(cudaGraphLaunch(graph_exec_, st));
-  // grad (with the search), 2 x (exp, M update, 1 or 2 spread passes); precond: 2 and the search;
-  // symmetry: 2 and the search
+  // grad, search (or in grad's last CTA), 2 x (exp, M update, 1 or 2 spread passes); precond and
+  // symmetry: 2 each
   launches_ += (1LL + 2 * (1 + (tiles3_ ? 4 : (tensor_wp_ ? 2 : 1)) + (omega_two_ ? 2 : 1)) + (pc_tiles_ ? 2 : 0) +
-                (n_ir_ ? 2 : 0) + (pc_tiles_ || n_ir_ ? 1 : 0) + (guide_w_ ? 1 : 0)) *
+                (n_ir_ ? 2 : 0) + (fuse_search() ? 0 : 1) + (guide_w_ ? 1 : 0)) *
                std::max(n, 0);
   launched_iters_ += std::max(n, 0);
   if (d_flag) {

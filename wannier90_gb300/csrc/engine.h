@@ -112,6 +112,7 @@ class Engine {
   int alloc(std::string& err);
   void release();
   void launch_iteration(cudaStream_t s);
+  bool fuse_search() const;
   void launch_omega(cudaStream_t s, int slot);
   void launch_mupdate(cudaStream_t s, int which);
   void launch_exp(cudaStream_t s, int which);

@@ -591,10 +591,19 @@ constexpr int kGradBC = 8;   // b values whose coefficients are staged together
 // Narrow problems are latency bound on the FP64 pipe (17 cycles per warp instruction, whatever the
 // number of active lanes), so a tile's elements and coefficients sit on consecutive threads: 8 x 8
 // blocks fill 2 warps instead of a quarter of 8 (17.4 -> 12 us at num_wann 8 on 64 k).
-__device__ __forceinline__ void grad_body(const Problem* __restrict__ probs, const WorkMap& wm) {
+__device__ __forceinline__ void grad_body(const Problem* __restrict__ probs, const WorkMap& wm, double* red) {
+  // element e of a tile of nr rows: a shift where the tile is full
+  auto split = [](int e, int nr, int& i, int& j) {
+    if (nr == kTile) {
+      i = e % kTile;
+      j = e / kTile;
+    } else {
+      i = e % nr;
+      j = e / nr;
+    }
+  };
   __shared__ double2 s_alpha[2][kGradBC][kTile];
   __shared__ double2 sP[2][kTile * (kTile + 1)];   // sP[t][j*(33)+i]: P tile t, row i, column j
-  __shared__ double red[256];
   int local;
   const int p = locate(wm, blockIdx.x, local);
   const Problem& P = probs[p];
@@ -627,8 +636,7 @@ __device__ __forceinline__ void grad_body(const Problem* __restrict__ probs, con
     for (int q = 0; q < 4; ++q) {
       acc[q] = cmk(0, 0);
       const int e = t + 256 * q;
-      ei[q] = e % nr;
-      ej[q] = e / nr;
+      split(e, nr, ei[q], ej[q]);
       vrow[q] = (R0 + ei[q] < S) ? 0 : 1;
     }
     for (int b0 = 0; b0 < B; b0 += kGradBC) {
@@ -636,7 +644,8 @@ __device__ __forceinline__ void grad_body(const Problem* __restrict__ probs, con
       __syncthreads();   // the previous chunk's coefficients are consumed
       // coefficients of the chunk: thread (bl, u) for column n = C0 + u of block b0 + bl
       {
-        const int bl = t / nc, u = t % nc;
+        int bl, u;
+        split(t, nc, u, bl);
         if (bl < nb) {
           const int b = b0 + bl, n = C0 + u;
           const double w = P.wb[b];
@@ -684,8 +693,8 @@ __device__ __forceinline__ void grad_body(const Problem* __restrict__ probs, con
     const double2* tr = sP[pass == 0 ? other : 0];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int e = t + 256 * q;
-      const int i = e % nr, j = e / nr;
+      int i, j;
+      split(t + 256 * q, nr, i, j);
       if (j < nc) {
         const double2 a = mine[j * (kTile + 1) + i];
         const double2 c = tr[i * (kTile + 1) + j];   // P_nm: row j, column i of the transposed tile
@@ -706,7 +715,10 @@ __device__ __forceinline__ void grad_body(const Problem* __restrict__ probs, con
   }
 }
 
-__global__ void __launch_bounds__(256) k_grad(const Problem* __restrict__ probs, WorkMap wm) { grad_body(probs, wm); }
+__global__ void __launch_bounds__(256, 3) k_grad(const Problem* __restrict__ probs, WorkMap wm) {
+  __shared__ double red[256];
+  grad_body(probs, wm, red);
+}
 
 // ----------------------------------------------------------------------------
 // k_phases: wann_phases (src/wannierise.F90:1756-1976) for guiding centres.
@@ -1020,15 +1032,23 @@ __global__ void k_ctrl_search(const Problem* __restrict__ probs) {
 
 // k_grad and, in the last CTA of each problem, k_ctrl_search: one launch less per iteration where
 // nothing comes between the two (no symmetry, no preconditioner)
-__global__ void __launch_bounds__(256) k_grad_search(const Problem* __restrict__ probs, WorkMap wm) {
+__global__ void __launch_bounds__(256, 3) k_grad_search(const Problem* __restrict__ probs, WorkMap wm) {
   __shared__ double red[256];
   int local;
   const Problem& P = probs[locate(wm, blockIdx.x, local)];
   CtrlState* st = P.st;
   if (st->done) return;
-  grad_body(probs, wm);
+  grad_body(probs, wm, red);
+  // thread 0 alone wrote this CTA's partials: its fence is enough
+  __shared__ int s_last;
   const int nt = (P.W + kTile - 1) / kTile;
-  if (!last_chunk_cta(&st->grad_arrive, P.K * nt * nt)) return;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&st->grad_arrive, 1u) == (unsigned)(P.K * nt * nt - 1);
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
   ctrl_search(P, red);
   if (threadIdx.x == 0) st->grad_arrive = 0u;
 }
