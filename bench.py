@@ -395,20 +395,23 @@ def run_reference_arm_dis(args, wl):
 
 
 def _dis_flops(p, w):
-    """Algorithmic FP64 FLOPs of one k_dis_z launch: per (k,b) C_b = M_w(k,b) U_opt(k+b)
-    (n x W x n') and the upper triangle of C_b C_b^H over the window (n(n+1)/2 x W), per k
-    tr(U^H Z U) (n x n x W); 8 real FLOPs per complex multiply-add."""
+    """Algorithmic FP64 FLOPs of one k_dis_z launch: per (k,b) the non-frozen part of C_b =
+    M_w(k,b) U_opt(k+b) (n x (W - nf') x (n' - nf')) and the upper triangle of its C_b C_b^H over
+    the window (n(n+1)/2 x (W - nf')), per k tr(U^H Z U) ((n - nf) x n x (W - nf)); 8 real FLOPs
+    per complex multiply-add.  (The frozen columns' part of Z is formed once per call.)"""
     import numpy as np
     eig = np.ascontiguousarray(p.eig.T)                      # ascending per k
     inwin = (eig >= w["win_min"]) & (eig <= w["win_max"])
     n = inwin.sum(axis=1)                                    # window states per k
+    nf = (inwin & (eig <= w["froz_max"])).sum(axis=1)        # frozen states per k
     W = p.num_wann
     z = 0.0
     for k in range(len(n)):
         for b in range(p.nntot):
             k2 = p.nnlist[k, b]
-            z += 8.0 * (n[k] * W * n[k2] + n[k] * (n[k] + 1) / 2 * W)
-        z += 8.0 * n[k] * n[k] * W
+            wc = W - nf[k2]
+            z += 8.0 * (n[k] * wc * (n[k2] - nf[k2]) + n[k] * (n[k] + 1) / 2 * wc)
+        z += 8.0 * (n[k] - nf[k]) * n[k] * (W - nf[k])
     return z
 
 

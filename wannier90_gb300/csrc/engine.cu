@@ -3,8 +3,8 @@
 // Memory: one arena per batch (cudaMalloc, or stream-ordered cudaMallocAsync for the
 // serving loop), sub-allocated at 256-byte alignment; every
 // per-problem array of the iteration stays resident in HBM for the whole solve.
-// Launch: the 14-kernel iteration (16 with the tensor-core M update, +2 with the
-// preconditioner; see k_fp64.cu) is captured once into a CUDA graph
+// Launch: the iteration (7 kernels for small problems, 16 for many k of num_wann > 32 on the
+// tensor cores, +2 with the preconditioner; see k_fp64.cu) is captured once into a CUDA graph
 // and replayed; the device controller makes replays after convergence no-ops, so the
 // host only polls a single "all done" word every few replays.
 #include <cuda_runtime.h>

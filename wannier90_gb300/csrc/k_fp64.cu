@@ -1,11 +1,12 @@
 // FP64 kernels of the GB300 MLWF engine (the plain FP64 path).
 //
 // One iteration of wann_main (src/wannierise.F90:534-816) is the fixed launch sequence
-//   k_grad [-> k_precond(0) -> k_precond(1)] -> k_ctrl_search -> k_exp_u(0) -> k_m_update(0) -> spread(0) -> k_ctrl_step
-//   -> k_exp_u(1) -> k_m_update(1) -> spread(1) -> k_ctrl_end
-// where spread(slot) = k_omega_p1 -> k_omega_p2.
+//   k_grad [-> k_precond(0) -> k_precond(1)] -> search -> k_exp_u(0) -> k_m_update(0) -> spread(0), step
+//   -> k_exp_u(1) -> k_m_update(1) -> spread(1), end
+// where spread(slot) = k_omega_p1 -> k_omega_p2 (one launch for small problems) with the control steps
+// (ctrl_step, ctrl_end) in its last CTA, and search is k_ctrl_search or the last CTA of k_grad_search.
 // All data-dependent decisions of the reference (CG reset, uphill reversal, parabolic
-// line search, convergence) are taken on the device by the k_ctrl_* kernels, so the
+// line search, convergence) are taken on the device by the ctrl_* functions, so the
 // sequence never needs the host and can be replayed (or graph-captured) blindly:
 // kernels whose work is not needed (second update when the parabola was rejected,
 // anything after convergence) return at entry.

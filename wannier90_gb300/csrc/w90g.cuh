@@ -120,7 +120,7 @@ struct Problem {
   double2* G;
   double2* D;
   double2* dU;
-  double2* work;        // exp / eig workspace (W > 32, or the tensor exp): 6*W*W per k
+  double2* work;        // exp workspace (FP64: W > 32; tensor path: any W): 6*W*W per k
   float* expinfo;       // tensor exp: [k][2] norm and state of the trial step's powers, for the optimal step
   double2* tbuf;        // M-update intermediate (W > 32): W*W per (k,b)
   const int* nnlist;    // [k][b] 0-based
@@ -134,7 +134,7 @@ struct Problem {
   double* log;          // [num_iter+1][kLogStride]
   double* log_centres;  // [num_iter+1][4][W]
   double2* M0;          // tensor path: M at entry (never modified)
-  unsigned char* m0s;   // tensor path: step 1's A operand (M0 rows) in BF16 digit planes,
+  unsigned char* m0s;   // tensor path: step 1's A operand (M0 rows) in FP16 digit planes,
                         // the shared-memory image of every (k, tile, K chunk)
   unsigned char* zs;    // tensor path, num_wann > 32: step 2's A operand (the rows of Z) likewise
   int* zs_exp;
@@ -143,15 +143,16 @@ struct Problem {
                         // written by step 1's epilogue
   unsigned char* ub2;   // pipelined tensor path: step 2's B operand -- the digit planes of U(k)
                         // in the shared-memory layout, per k -- written by step 1's B producer
+                        // (num_wann > 32: both steps' B, written by a kernel before them)
   int* ub2_exp;         // ... and the column exponents of U(k) [k][WP]
   double2* U0;          // tensor path: U at entry; U[] then holds R = U0^H U
   const int* inv_nnlist;  // tensor path: [k'][i] = k*B+b with nnlist(k,b) = k'
-  double* frob0;        // tensor path: |M0(k,b)|_F^2
+  double* frob0;        // tensor path: |M0(k,b)|_F^2 (the first trial step's off-diagonal sums)
   double* odpart;       // tensor path: [k][b][odn] partial sums of |M_mn|^2, m != n, of the last M update
   double* opart1;       // [nchunk][4W+2] spread partials (pass 1)
   double* opart2;       // [nchunk]       Omega_D partials (pass 2)
   int nchunk;           // chunks of the spread passes (at most 64 blocks each)
-  int tensor;           // 1: M update on tensor cores (tcgen05, exact BF16 slicing)
+  int tensor;           // 1: M update on tensor cores (tcgen05, exact FP16 slicing)
   CtrlState* st;
   Control ctl;
   int max_exp_squarings;
