@@ -118,3 +118,33 @@ def test_spread_passes_over_their_chunk_rules(W, mp, tensor):
         assert abs(row[3] - it.spread.om_tot) <= 1e-9 * abs(it.spread.om_tot) + 2e-10
         assert int(row[6]) == int(it.lquad)
     np.testing.assert_allclose(out["centres"].T, ref.centres.T, atol=1e-7)
+
+
+# slabs of several groups and of one, a last slab that is shorter; both digit forms
+@pytest.mark.parametrize("kind,W,mp", [("sc", 33, (3, 3, 3)), ("fcc", 48, (2, 2, 2)), ("sc", 64, (1, 1, 3)),
+                                       ("sc", 40, (1, 1, 2)), ("sc", 100, (2, 2, 2)), ("sc", 128, (2, 2, 2))])
+def test_wide_update_in_slabs_equals_the_whole(kind, W, mp):
+    """A served job that fits its budget only with the image of Z in slabs gives the same bits."""
+    torch = pytest.importorskip("torch")
+    p, km, M0, U0 = _projected(kind, mp, W, seed=9)
+    res = []
+    budget = 1e12
+    for _ in range(2):
+        h = w90.setup(kpoints=p.kpoints, unit_cell_cart=p.real_lattice, num_wann=W, num_iter=4, iprint=0, gpu_tensor=1,
+                      conv_window=-1)
+        m = torch.from_numpy(synth.from_math_m(M0).reshape(-1, order="F").view(np.float64).copy()).cuda()
+        u = torch.from_numpy(synth.from_math_u(U0).reshape(-1, order="F").view(np.float64).copy()).cuda()
+        torch.cuda.synchronize()
+        srv = w90.Server(budget, max_active=1, chunk_iters=2)
+        assert srv.submit(h, m.data_ptr(), u.data_ptr(), 0) == 0, h.last_error()
+        srv.drain()
+        done = srv.poll()
+        peak = srv.stats()["peak_bytes"]
+        srv.close()
+        assert len(done) == 1 and done[0][1] == 0, h.last_error()
+        assert peak <= budget
+        res.append((m.cpu().numpy(), u.cpu().numpy(), w90.w90_get_log(h, 5).copy()))
+        budget = peak - 1
+    (m1, u1, l1), (m2, u2, l2) = res
+    assert np.array_equal(m1, m2) and np.array_equal(u1, u2)
+    assert np.array_equal(l1[:, :8], l2[:, :8])

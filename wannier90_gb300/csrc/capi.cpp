@@ -1447,6 +1447,10 @@ int w90g_server_submit(void* server, void* handle, double* d_m, double* d_u, lon
   j->d_u = d_u;
   build_spec(h, j->spec);
   j->bytes = Engine::estimate_bytes({j->spec});
+  if (j->bytes > sv->budget) {
+    j->spec.lean = 1;
+    j->bytes = Engine::estimate_bytes({j->spec});
+  }
   if (j->bytes > sv->budget) return fail(h, 2, "serve: job needs more device memory than the server's budget");
   std::lock_guard<std::mutex> lk(sv->mu);
   j->t_submit = sv->now();

@@ -43,7 +43,8 @@ __global__ void k_sym_grad(const Problem* probs, WorkMap wm);
 __global__ void k_sym_dir(const Problem* probs, WorkMap wm);
 __global__ void k_sym_u(const Problem* probs, WorkMap wm);
 cudaError_t oz_ufinal_launch(int wp, const Problem* probs, WorkMap wm, int grid, cudaStream_t s);
-cudaError_t oz3_launch(int wp, const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, cudaStream_t s);
+cudaError_t oz3_launch(int wp, const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, int slabs,
+                       cudaStream_t s);
 cudaError_t oz3_preslice_launch(int wp, const Problem* probs, WorkMap wm, int ngroups, int tmax, cudaStream_t s);
 cudaError_t oz3_set_attributes(int wp);
 void oz3_bytes(int W, int K, int B, size_t out[4]);
@@ -143,7 +144,7 @@ int Engine::setup(const std::vector<ProblemSpec>& specs, std::string& err) {
   for (const auto& s : specs)
     key << s.W << ',' << s.K << ',' << s.B << ',' << s.ctl.num_iter << ',' << s.tensor << ',' << s.tensor_exp << ','
         << s.precond << ',' << s.nrpts << ',' << s.guiding << ',' << (s.slwf_num > 0) << ',' << s.sym_nir << ','
-        << s.sym_mem.size() << ',' << s.sym_grp.size() << ',' << s.sym_d.size() << ';';
+        << s.sym_mem.size() << ',' << s.sym_grp.size() << ',' << s.sym_d.size() << ',' << s.lean << ';';
   specs_ = specs;
   if (arena_ && key.str() == layout_key_) {
     // refresh the read-only tables (they may differ at equal shapes)
@@ -206,17 +207,28 @@ int omega_chunks(const ProblemSpec& s) {
 // group, and for num_wann > 32 per 32-row piece of the block (k_mupdate3.cu)
 int odn_of(int W) { return W <= 32 ? 4 : 4 * (W / 32 + 2); }
 
+// An array that may lie inside another one that is dead while it is used: host 1 is M0 (tensor path;
+// read once, to slice it, before any of these is written), host 2 is dU (dead between the exp and the
+// next one; on the FP64 path the M update reads it, so only the spread's arrays may lie there).
+struct Part {
+  size_t n = 0, at = 0;
+  int host = 0;
+  size_t own() const { return host ? 0 : n; }
+};
+
 struct Sizes {
-  size_t M, U, KWW, work, tbuf, diag, offd, gpart, cen, log, logc, nn, bk, wb, st, op1, op2, m0, u0, inv, fr;
-  size_t m0s, m0e, zexp, ub2, ub2e, einfo, odp, zs, zse;
+  size_t M, U, KWW, tbuf, diag, offd, gpart, cen, log, logc, nn, bk, wb, st, m0, u0, inv, fr;
+  size_t m0s, m0e, zexp;
+  Part work, ub2, ub2e, einfo, odp, zs, zse, op1, op2;
+  int slabs;
   size_t pkr, pr2, pgr, pgp, ppart;
   size_t gbka, gneigh, grg, gsheet, gcsheet;
   size_t slwf;
   size_t symi, symd, symw;
   size_t total() const {
-    return 2 * M + 2 * U + 3 * KWW + work + tbuf + 2 * diag + offd + gpart + cen + log + logc + nn + bk + wb + st +
-           op1 + op2 + m0 + u0 + inv + fr + m0s + m0e + zexp + ub2 + ub2e + einfo + odp + zs + zse + pkr + 2 * pr2 + pgr + pgp + ppart + gbka + gneigh + grg + gsheet +
-           gcsheet + slwf + symi + 2 * symd + symw;
+    return 2 * M + 2 * U + 3 * KWW + work.own() + tbuf + 2 * diag + offd + gpart + cen + log + logc + nn + bk + wb + st +
+           op1.own() + op2.own() + m0 + u0 + inv + fr + m0s + m0e + zexp + ub2.own() + ub2e.own() + einfo.own() +
+           odp.own() + zs.own() + zse.own() + pkr + 2 * pr2 + pgr + pgp + ppart + gbka + gneigh + grg + gsheet + gcsheet + slwf + symi + 2 * symd + symw;
   }
 };
 
@@ -230,30 +242,37 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
   z.U = align_up(K * WW * 16);
   z.KWW = align_up(K * WW * 16);
   // exp workspace: FP64 kernels for W > 32; the tensor exp keeps X and its powers here
-  z.work = (s.W > 32 || wp) ? align_up(K * 6 * WW * 16) : 0;
-  z.einfo = wp ? align_up(K * 8) : 0;
+  z.work.n = (s.W > 32 || wp) ? align_up(K * 6 * WW * 16) : 0;
+  z.einfo.n = wp ? align_up(K * 8) : 0;
   z.tbuf = (s.W > 32 || wp) ? align_up(K * B * WW * 16) : 0;
   z.m0 = wp ? align_up(K * B * WW * 16) : 0;
   z.u0 = wp ? align_up(K * WW * 16) : 0;
   z.inv = wp ? align_up(K * B * 4) : 0;
-  z.odp = wp ? align_up(K * B * odn_of(s.W) * 8) : 0;
+  z.odp.n = wp ? align_up(K * B * odn_of(s.W) * 8) : 0;
   z.fr = wp ? align_up(K * B * 8) : 0;
-  z.m0s = z.m0e = z.zs = z.zse = 0;
+  z.m0s = z.m0e = 0;
+  z.slabs = 1;
   z.zexp = (wp && wp <= 32) ? align_up(K * B * W * 4) : 0;
-  z.ub2 = z.ub2e = 0;
   if (wp && wp <= 32) {
     size_t d = 0, e = 0;
     oz2_ub2_bytes(wp, (int)K, &d, &e);
-    z.ub2 = align_up(d);
-    z.ub2e = align_up(e);
+    z.ub2.n = align_up(d);
+    z.ub2e.n = align_up(e);
   }
   if (wp > 32) {
     size_t b[4];
     oz3_bytes((int)W, (int)K, (int)B, b);
-    z.m0s = z.zs = align_up(b[0]);
-    z.m0e = z.zse = align_up(b[1]);
-    z.ub2 = align_up(b[2]);
-    z.ub2e = align_up(b[3]);
+    z.m0s = align_up(b[0]);
+    z.m0e = z.zse.n = align_up(b[1]);
+    z.ub2.n = align_up(b[2]);
+    z.ub2e.n = align_up(b[3]);
+    // the digit image of Z (28 B an element against M0's 16): all groups' at once, or in as many slabs
+    // as it takes to fit into M0 with U's image
+    auto image = [&](int slabs) { return align_up(b[0] / K * ((K + slabs - 1) / slabs)); };
+    if (s.lean)
+      while (z.slabs < (int)K && image(z.slabs) + z.ub2.n > z.m0) ++z.slabs;
+    z.zs.n = image(z.slabs);
+    z.m0 = std::max(z.m0, z.zs.n);
   } else if (wp) {
     size_t d = 0, e = 0;
     oz_preslice_bytes(wp, (int)K, (int)B, &d, &e);
@@ -271,8 +290,28 @@ Sizes problem_sizes(const ProblemSpec& s, int wp, int* pc_tiles) {
   z.wb = align_up(B * 8);
   z.st = align_up(sizeof(CtrlState));
   const size_t nch = omega_chunks(s);
-  z.op1 = align_up(nch * (4 * W + 2) * 8);
-  z.op2 = align_up(nch * 8);
+  z.op1.n = align_up(nch * (4 * W + 2) * 8);
+  z.op2.n = align_up(nch * 8);
+  size_t used[3] = {0, 0, 0};
+  auto inside = [&](Part& q, int host) {
+    const size_t room = host == 1 ? z.m0 : z.KWW;
+    if (q.n == 0 || q.host || used[host] + q.n > room) return;
+    q.host = host;
+    q.at = used[host];
+    used[host] += q.n;
+  };
+  inside(z.op1, 2);
+  inside(z.op2, 2);
+  if (wp) {
+    inside(z.zs, 1);
+    if (wp > 32) inside(z.ub2, 1);
+    else inside(z.work, 1);
+    inside(z.odp, 2);
+    inside(z.einfo, 1);
+    for (Part* q : {&z.odp, &z.zse, &z.op1, &z.op2}) inside(*q, 1);
+    if (wp > 32) inside(z.ub2e, 2);
+    inside(z.zse, 2);
+  }
   z.pkr = z.pr2 = z.pgr = z.pgp = z.ppart = 0;
   if (s.precond) {
     const size_t NR = s.nrpts;
@@ -357,8 +396,22 @@ int Engine::alloc(std::string& err) {
   for (const auto& s : specs_) omega_two_ = omega_two_ || s.K * s.B * s.W > kOmegaOneCta;
   n_ir_ = offs_ir[np];
   total += header_bytes(np, n_k_);
-  if (async_alloc_) W90G_CHECK(cudaMallocAsync(&arena_, total, stream()));
-  else W90G_CHECK(cudaMalloc(&arena_, total));
+  // (no room: the M update's wide form again with its image of Z in slabs)
+  auto grab = [&] { return async_alloc_ ? cudaMallocAsync(&arena_, total, stream()) : cudaMalloc(&arena_, total); };
+  cudaError_t ea = grab();
+  if (ea == cudaErrorMemoryAllocation && tensor_wp_ > 32) {
+    cudaGetLastError();
+    arena_ = nullptr;
+    total = header_bytes(np, n_k_);
+    for (int p = 0; p < np; ++p) {
+      specs_[p].lean = 1;
+      sz[p] = problem_sizes(specs_[p], tensor_wp_, nullptr);
+      total += sz[p].total();
+    }
+    ea = grab();
+  }
+  W90G_CHECK(ea);
+  slabs_ = 1;
   arena_bytes_ = total;
   char* cur = (char*)arena_;
   auto take = [&](size_t n) {
@@ -393,8 +446,13 @@ int Engine::alloc(std::string& err) {
     P.G = (double2*)take(z.KWW);
     P.D = (double2*)take(z.KWW);
     P.dU = (double2*)take(z.KWW);
-    P.work = z.work ? (double2*)take(z.work) : nullptr;
-    P.expinfo = z.einfo ? (float*)take(z.einfo) : nullptr;
+    P.M0 = z.m0 ? (double2*)take(z.m0) : nullptr;
+    auto part = [&](const Part& q) -> void* {
+      if (q.n == 0) return nullptr;
+      return q.host == 0 ? (void*)take(q.n) : (char*)(q.host == 1 ? P.M0 : P.dU) + q.at;
+    };
+    P.work = (double2*)part(z.work);
+    P.expinfo = (float*)part(z.einfo);
     P.tbuf = z.tbuf ? (double2*)take(z.tbuf) : nullptr;
     P.diag_ln = (double*)take(z.diag);
     P.diag_abs2 = (double*)take(z.diag);
@@ -407,21 +465,22 @@ int Engine::alloc(std::string& err) {
     double* bk = (double*)take(z.bk);
     double* wb = (double*)take(z.wb);
     P.st = (CtrlState*)take(z.st);
-    P.M0 = z.m0 ? (double2*)take(z.m0) : nullptr;
     P.U0 = z.u0 ? (double2*)take(z.u0) : nullptr;
     int* inv = z.inv ? (int*)take(z.inv) : nullptr;
     P.inv_nnlist = inv;
     P.tensor = tensor_wp_ ? 1 : 0;
     P.frob0 = z.fr ? (double*)take(z.fr) : nullptr;
-    P.odpart = z.odp ? (double*)take(z.odp) : nullptr;
+    P.odpart = (double*)part(z.odp);
     P.odn = odn_of(s.W);
     P.m0s = z.m0s ? (unsigned char*)take(z.m0s) : nullptr;
     P.m0s_exp = z.m0e ? (int*)take(z.m0e) : nullptr;
-    P.zs = z.zs ? (unsigned char*)take(z.zs) : nullptr;
-    P.zs_exp = z.zse ? (int*)take(z.zse) : nullptr;
+    P.zs = (unsigned char*)part(z.zs);
+    P.zs_exp = (int*)part(z.zse);
+    P.zs_slabs = z.slabs;
+    slabs_ = std::max(slabs_, z.slabs);
     P.zexp = z.zexp ? (int*)take(z.zexp) : nullptr;
-    P.ub2 = z.ub2 ? (unsigned char*)take(z.ub2) : nullptr;
-    P.ub2_exp = z.ub2e ? (int*)take(z.ub2e) : nullptr;
+    P.ub2 = (unsigned char*)part(z.ub2);
+    P.ub2_exp = (int*)part(z.ub2e);
     if (inv) {
       std::vector<int> h_inv((size_t)s.K * s.B), fill(s.K, 0);
       for (int kb = 0; kb < s.K * s.B; ++kb) {
@@ -430,8 +489,8 @@ int Engine::alloc(std::string& err) {
       }
       W90G_CHECK(cudaMemcpyAsync(inv, h_inv.data(), h_inv.size() * sizeof(int), cudaMemcpyHostToDevice, stream()));
     }
-    P.opart1 = (double*)take(z.op1);
-    P.opart2 = (double*)take(z.op2);
+    P.opart1 = (double*)part(z.op1);
+    P.opart2 = (double*)part(z.op2);
     P.nchunk = omega_chunks(s);
     P.ctl = s.ctl;
     W90G_CHECK(cudaMemcpyAsync(nn, s.nnlist.data(), s.nnlist.size() * sizeof(int), cudaMemcpyHostToDevice, stream()));
@@ -744,7 +803,7 @@ void Engine::launch_mupdate(cudaStream_t s, int which) {
   const WorkMap wmk{d_offs_k_, np};
   const WorkMap wmkb{d_offs_kb_, np};
   if (tiles3_) {
-    oz3_launch(tensor_wp_, dprobs_, wmk, which, n_k_, tiles3_, s);
+    oz3_launch(tensor_wp_, dprobs_, wmk, which, n_k_, tiles3_, slabs_, s);
   } else if (pipe_) {
     oz2_launch(tensor_wp_, 1, dprobs_, wmk, which, n_k_, s);
     oz2_launch(tensor_wp_, 2, dprobs_, wmk, which, n_k_, s);
@@ -841,7 +900,7 @@ int Engine::advance(int n, int* d_flag, std::string& err) {
   for (int i = 0; i < n; ++i) W90G_CHECK(cudaGraphLaunch(graph_exec_, st));
   // grad, search (or in grad's last CTA), 2 x (exp, M update, 1 or 2 spread passes); precond and
   // symmetry: 2 each
-  launches_ += (1LL + 2 * (1 + (tiles3_ ? 4 : (tensor_wp_ ? 2 : 1)) + (omega_two_ ? 2 : 1)) + (pc_tiles_ ? 2 : 0) +
+  launches_ += (1LL + 2 * (1 + (tiles3_ ? 2 + 2 * slabs_ : (tensor_wp_ ? 2 : 1)) + (omega_two_ ? 2 : 1)) + (pc_tiles_ ? 2 : 0) +
                 (n_ir_ ? 2 : 0) + (fuse_search() ? 0 : 1) + (guide_w_ ? 1 : 0)) *
                std::max(n, 0);
   launched_iters_ += std::max(n, 0);

@@ -20,6 +20,7 @@ struct ProblemSpec {
   int tensor = 0;            // request the tensor-core M update (W <= 128)
   int tensor_exp = 1;        // with tensor: exp(s D) and U dU on the tensor cores too
   int mupdate_pipe = 1;      // with tensor and W <= 32: the pipelined M-update kernel (k_mupdate2.cu)
+  int lean = 0;              // num_wann > 32 on the tensor path: less memory, Z's digit image in slabs
   int exp_smem = 0;          // with tensor exp and 16 < W <= 32: the exp chain's matrices in shared memory
   // preconditioner (precond = T): Wigner-Seitz points R_r of the Born-von Karman
   // supercell, exp(-i 2 pi k.R) table [k][r] (re, im interleaved), |R|^2, degeneracies
@@ -140,6 +141,7 @@ class Engine {
   int guide_w_ = 0;      // > 0: some problem uses guiding centres; CTAs per problem of k_phases
   int maxW_small_ = 0;   // largest W <= 32 in the batch (shared-memory kernels)
   int tiles3_ = 0;           // num_wann > 32 on the tensor path: 128-row tiles of the largest group
+  int slabs_ = 1;            // of the wide M update's image of Z (the largest over the problems)
   bool omega_two_ = false;   // some problem needs the spread's second pass as a launch of its own
   int tensor_wp_ = 0;    // > 0: tensor M update with padded width 8..128 for the whole batch
   bool tensor_exp_ = false;  // exp(s D) on the tensor cores (k_oz_exp)

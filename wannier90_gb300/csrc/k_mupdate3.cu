@@ -69,6 +69,13 @@ __host__ __device__ __forceinline__ Geo3 geo3(int W, int B) {
 __host__ __device__ __forceinline__ size_t bstage3(const Geo3& g) { return (size_t)kS * (2 * g.cw) * 32; }
 __host__ __device__ __forceinline__ size_t bimage3(const Geo3& g) { return bstage3(g) * g.ksteps * g.nch; }
 
+// Step 2's image may hold the groups of one slab at a time: group g's slot there, or -1 if it is not of
+// slab `slab`.  (One slab: g.)
+__device__ __forceinline__ int zslot(const Problem& P, int g, int slab) {
+  const int per = (P.K + P.zs_slabs - 1) / P.zs_slabs;
+  return g / per == slab ? g - slab * per : -1;
+}
+
 // the 7 digit planes of 8 values with scale exponent ex, 8- or 7-bit digits
 template <bool EIGHT>
 __device__ __forceinline__ void slice3(uint32_t (&w)[kS][4], const double (&v)[8], int ex) {
@@ -115,7 +122,7 @@ __device__ __forceinline__ void arrive_expect(uint64_t* bar, uint32_t bytes) {
 // persistent grid walks them.  EIGHT: every problem of the launch has num_wann <= 64.
 template <int STEP, bool EIGHT>
 __global__ void __launch_bounds__(kThreads3, 1)
-    k_oz_mupdate3(const Problem* __restrict__ probs, WorkMap wm, int which, int ngroups, int tmax) {
+    k_oz_mupdate3(const Problem* __restrict__ probs, WorkMap wm, int which, int ngroups, int tmax, int slab) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t a_full[kStages], a_empty[kStages];
@@ -166,11 +173,12 @@ __global__ void __launch_bounds__(kThreads3, 1)
         const int p = locate(wm, item / tmax, g), tile = item % tmax;
         const Problem& P = probs[p];
         const Geo3 G = geo3(P.W, P.B);
-        if (tile >= G.ntiles || !group_active(P, which)) continue;
+        if (tile >= G.ntiles || !group_active(P, which) || (STEP == 2 && zslot(P, g, slab) < 0)) continue;
         const uint32_t bst = (uint32_t)bstage3(G);
         const unsigned char* bimg = P.ub2 + (size_t)g * bimage3(G);
         const unsigned char* aimg =
-            (STEP == 1 ? P.m0s : P.zs) + ((size_t)g * G.ntiles + tile) * G.ksteps * (size_t)kStageA;
+            (STEP == 1 ? P.m0s : P.zs) +
+            ((size_t)(STEP == 1 ? g : zslot(P, g, slab)) * G.ntiles + tile) * G.ksteps * (size_t)kStageA;
         for (int nc = 0; nc < G.nch && ok; ++nc)
           for (int ks = 0; ks < G.ksteps; ++ks) {
             const int s = sseq % kStages;
@@ -204,7 +212,7 @@ __global__ void __launch_bounds__(kThreads3, 1)
         const int p = locate(wm, item / tmax, g), tile = item % tmax;
         const Problem& P = probs[p];
         const Geo3 G = geo3(P.W, P.B);
-        if (tile >= G.ntiles || !group_active(P, which)) continue;
+        if (tile >= G.ntiles || !group_active(P, which) || (STEP == 2 && zslot(P, g, slab) < 0)) continue;
         const int N = 2 * G.cw, ppm = 256 / N;
         for (int nc = 0; nc < G.nch && ok; ++nc) {
           if (useq > 0 && !mbar_wait_role(smem_u32(&acc_empty), (uint32_t)(useq - 1) & 1, &s_bad)) {
@@ -278,7 +286,7 @@ __global__ void __launch_bounds__(kThreads3, 1)
       const Problem& P = probs[p];
       const int W = P.W, WW = W * W;
       const Geo3 G = geo3(W, P.B);
-      if (tile >= G.ntiles || !group_active(P, which)) continue;
+      if (tile >= G.ntiles || !group_active(P, which) || (STEP == 2 && zslot(P, g, slab) < 0)) continue;
       const int cur = P.st->cur, N = 2 * G.cw, cpg = G.cw / 4;
       const int row = tile * kTileRows + r;
       const bool valid = row < P.B * W;
@@ -446,14 +454,15 @@ __global__ void __launch_bounds__(256) k_oz_slice_u(const Problem* __restrict__ 
 // One CTA (256 threads) per (group, tile).
 template <int STEP, bool EIGHT>
 __global__ void __launch_bounds__(256) k_oz_preslice3(const Problem* __restrict__ probs, WorkMap wm, int tmax,
-                                                      int which) {
+                                                      int which, int slab) {
   __shared__ int s_rowexp[kTileRows];
   int g;
   const int p = locate(wm, blockIdx.x / tmax, g), tile = blockIdx.x % tmax;
   const Problem& P = probs[p];
   const int W = P.W, WW = W * W, tid = threadIdx.x;
   const Geo3 G = geo3(W, P.B);
-  if (tile >= G.ntiles || (STEP == 2 && !group_active(P, which))) return;
+  const int slot = STEP == 1 ? g : zslot(P, g, slab);
+  if (tile >= G.ntiles || (STEP == 2 && (slot < 0 || !group_active(P, which)))) return;
   unsigned char* img = STEP == 1 ? P.m0s : P.zs;
   int* exps = STEP == 1 ? P.m0s_exp : P.zs_exp;
   auto row_of = [&](int row) -> const double2* {
@@ -488,7 +497,7 @@ __global__ void __launch_bounds__(256) k_oz_preslice3(const Problem* __restrict_
     }
     uint32_t w[kS][4];
     slice3<EIGHT>(w, v, s_rowexp[rs]);
-    unsigned char* dst = img + (((size_t)g * G.ntiles + tile) * G.ksteps + ks) * (size_t)kStageA;
+    unsigned char* dst = img + (((size_t)slot * G.ntiles + tile) * G.ksteps + ks) * (size_t)kStageA;
     const uint32_t o = stage_off(rs, 8 * part);
 #pragma unroll
     for (int t = 0; t < kS; ++t)
@@ -525,25 +534,29 @@ cudaError_t oz3_set_attributes(int wp) {
 }
 
 template <bool EIGHT>
-static void oz3_launch_e(const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, cudaStream_t s) {
+static void oz3_launch_e(const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, int slabs,
+                         cudaStream_t s) {
   const int grid = std::min(ngroups * tmax, sm_count());
   k_oz_slice_u<EIGHT><<<ngroups, 256, 0, s>>>(probs, wm, which);
-  k_oz_mupdate3<1, EIGHT><<<grid, kThreads3, kSmem3, s>>>(probs, wm, which, ngroups, tmax);
-  k_oz_preslice3<2, EIGHT><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, which);
-  k_oz_mupdate3<2, EIGHT><<<grid, kThreads3, kSmem3, s>>>(probs, wm, which, ngroups, tmax);
+  k_oz_mupdate3<1, EIGHT><<<grid, kThreads3, kSmem3, s>>>(probs, wm, which, ngroups, tmax, 0);
+  for (int i = 0; i < slabs; ++i) {
+    k_oz_preslice3<2, EIGHT><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, which, i);
+    k_oz_mupdate3<2, EIGHT><<<grid, kThreads3, kSmem3, s>>>(probs, wm, which, ngroups, tmax, i);
+  }
 }
 
-// the whole update (four launches) of the ngroups work items of wm; wp: the widest problem's
+// the whole update (four launches, two more for each slab of Z's image after the first) of the ngroups work items of wm; wp: the widest problem's
 // padded width, 64 or 128; tmax: the largest tile count of a group
-cudaError_t oz3_launch(int wp, const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, cudaStream_t s) {
-  if (wp <= 64) oz3_launch_e<true>(probs, wm, which, ngroups, tmax, s);
-  else oz3_launch_e<false>(probs, wm, which, ngroups, tmax, s);
+cudaError_t oz3_launch(int wp, const Problem* probs, WorkMap wm, int which, int ngroups, int tmax, int slabs,
+                       cudaStream_t s) {
+  if (wp <= 64) oz3_launch_e<true>(probs, wm, which, ngroups, tmax, slabs, s);
+  else oz3_launch_e<false>(probs, wm, which, ngroups, tmax, slabs, s);
   return cudaGetLastError();
 }
 
 cudaError_t oz3_preslice_launch(int wp, const Problem* probs, WorkMap wm, int ngroups, int tmax, cudaStream_t s) {
-  if (wp <= 64) k_oz_preslice3<1, true><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, 0);
-  else k_oz_preslice3<1, false><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, 0);
+  if (wp <= 64) k_oz_preslice3<1, true><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, 0, 0);
+  else k_oz_preslice3<1, false><<<ngroups * tmax, 256, 0, s>>>(probs, wm, tmax, 0, 0);
   return cudaGetLastError();
 }
 

@@ -138,6 +138,7 @@ struct Problem {
                         // the shared-memory image of every (k, tile, K chunk)
   unsigned char* zs;    // tensor path, num_wann > 32: step 2's A operand (the rows of Z) likewise
   int* zs_exp;
+  int zs_slabs, pad6;   // zs holds ceil(K / zs_slabs) groups at a time
   int* m0s_exp;         // tensor path: the row exponents of those tiles [k][tile][128]
   int* zexp;            // pipelined tensor path: step 2's row exponents [k][b][row of Z(k,b)],
                         // written by step 1's epilogue
