@@ -247,10 +247,12 @@ __global__ void k_ctrl_end(const Problem* __restrict__ probs) {
 // On the tensor path the off-diagonal sums come from the M update's epilogue (odpart), summed
 // there directly.  |M0|_F^2 minus the diagonal, the invariant form used before, cancels to ~1e-14 of
 // num_wann and near a minimum hid the trial step's change from the parabola (1000 k, num_wann 32,
-// 1e-12 window: refused steps, Omega 5e-8 after 3107 iterations; with the direct sum 8e-11).  Only
-// the first trial step still takes the invariant form: the first step length is the one quantity
-// that its offset against the entry overlaps' direct sum moves by more than rounding, and with it
-// the whole trajectory, which so stays the earlier one.
+// 1e-12 window: refused steps, Omega 5e-8 after 3107 iterations; with the direct sum 8e-11).  For
+// num_wann <= 32 the first trial step still takes the invariant form: the first step length is the
+// one quantity that its offset against the entry overlaps' direct sum moves by more than rounding
+// (1e-9 in M after four iterations of 1000 k of num_wann 32), and with it the whole trajectory, which
+// so stays the earlier one.  Wider problems take the direct sum there too (M of 512 k of num_wann
+// 128 against 64 bits: 2.9e-10 with the invariant form, 5.8e-12 without).
 // Selective localisation (slwf_num = s > 0, :2144-2211): p1's off-diagonal slot holds
 // sum over n < s of wb (1 - |M_nn|^2 + lambda ln_n^2) (Omega_IOD) and its Omega_I slot
 // sum over n < s of 2 wb lambda ln_n (b.c_n) (the k-sum of Omega_nu); p2 sums over n < s
@@ -418,7 +420,7 @@ __global__ void __launch_bounds__(256) k_omega_p1(const Problem* __restrict__ pr
   } else {
     const bool first = (slot == 2) && st->first_pass;
     const bool parts = P.tensor && slot < 2;   // partials of the tensor M update's epilogue
-    const bool inv = parts && slot == 0 && st->iter == 0;
+    const bool inv = parts && slot == 0 && st->iter == 0 && W <= 32;
     double od = 0.0, oi = 0.0;
     if (parts) {
       // tpk threads share one block (k,b); per <= 64 blocks take one round

@@ -148,7 +148,7 @@ struct Problem {
   int* ub2_exp;         // ... and the column exponents of U(k) [k][WP]
   double2* U0;          // tensor path: U at entry; U[] then holds R = U0^H U
   const int* inv_nnlist;  // tensor path: [k'][i] = k*B+b with nnlist(k,b) = k'
-  double* frob0;        // tensor path: |M0(k,b)|_F^2 (the first trial step's off-diagonal sums)
+  double* frob0;        // tensor path: |M0(k,b)|_F^2 (the first trial step's off-diagonal sums, W <= 32)
   double* odpart;       // tensor path: [k][b][odn] partial sums of |M_mn|^2, m != n, of the last M update
   double* opart1;       // [nchunk][4W+2] spread partials (pass 1)
   double* opart2;       // [nchunk]       Omega_D partials (pass 2)
