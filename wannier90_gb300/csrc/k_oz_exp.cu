@@ -1,6 +1,6 @@
 // Tensor-core rotation step: U(k) <- U(k) exp(s D(k)) (internal_new_u_and_m,
 // src/wannierise.F90:1655-1733) with every W x W complex product on the tcgen05 tensor cores
-// through exact slicing into FP16 / BF16 digits at 56-bit precision (oz_mm.cuh); norms and the
+// through exact slicing into FP16 digits at 56-bit precision (oz_mm.cuh); norms and the
 // polynomials' linear combinations are FP64 (the norms' moduli FP32).
 //
 // The matrix function is a Taylor polynomial of degree 4, 8 or 12 of X 2^-js, squared js times.
