@@ -13,7 +13,7 @@
 // smallest one has not reached 1 after kPolarSteps steps -- a condition number above ~1e5, or
 // a rank-deficient X -- is left alone with status 0: the FP64 kernel that runs next takes it,
 // with its own verdict.  That kernel also takes everything else this one cannot finish
-// (a bounded wait that ran out, NaN or infinities, which never converge).
+// (a bounded wait that ran out, NaN, infinities and scales outside what the digits carry).
 #include "oz_mm.cuh"
 #include "polar.h"
 
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(256, 2) k_oz_polar(PolarArgs g) {
   __syncthreads();
   OzCtx cx{base, base + E::SB_OFFSET, tmem_slot, smem_u32(&mbar), 0u, s_rowexp, s_colexp, &s_bad};
   const NoAdd none;
-  bool ok = true, done = false;
+  bool ok = !__syncthreads_or(keys_wild(rX.row, N)), done = false;
   for (int step = 0; step < kPolarSteps && ok && !done; ++step) {
     for (int e = tid; e < NN; e += 256) XH[e] = cconj(X[(size_t)(e % N) * N + e / N]);
     __syncthreads();

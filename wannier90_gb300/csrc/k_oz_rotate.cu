@@ -6,6 +6,8 @@
 // In FP64 these are bound by the FP64 pipe (8000 blocks of num_wann 32: 3.6 ms, 4096 of 42 states to
 // 32: 2.9 ms, U0 R of 512 x 128: 8.3 ms).  The products here are as accurate as FP64 ones; what
 // bounds them is slicing and recombining, two CTAs per SM hiding each other's latency.
+// Operands whose scales the digits do not carry (exp_wild: NaN, infinities, magnitudes beyond 2^+-290)
+// are multiplied in FP64 here, block by block, so that they come out as FP64 gives them.
 #include <algorithm>
 
 #include "oz_mm.cuh"
@@ -46,6 +48,17 @@ __device__ __forceinline__ void rot_end(RotShared& sh) {
   if (threadIdx.x < 32)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
                  :: "r"(sh.tmem), "r"((uint32_t)E::TMEM_COLS) : "memory");
+}
+
+// C (m x n, ldc) = A B in FP64, inner dimension kk
+__device__ __forceinline__ void rot_fp64(double2* C, int ldc, const double2* A, int lda, const double2* B, int ldb,
+                                         int m, int n, int kk) {
+  for (int e = threadIdx.x; e < m * n; e += blockDim.x) {
+    const int i = e % m, j = e / m;
+    double2 acc = cmk(0.0, 0.0);
+    for (int l = 0; l < kk; ++l) cfma(acc, A[(size_t)l * lda + i], B[(size_t)j * ldb + l]);
+    C[(size_t)j * ldc + i] = acc;
+  }
 }
 
 }  // namespace
@@ -91,11 +104,17 @@ __global__ void __launch_bounds__(256, 2) k_oz_rotate(RotateArgs g, int items) {
       rec_add(rR, i, j, r);
     }
     __syncthreads();
-    ok = E::mm(cx, T, LH, rL.row, M, rM.col, N, Epi{T, 0, rT}, none);
-    if (ok) ok = E::mm(cx, M, T, rT.row, R, rR.col, N, Epi{M, 0, Rec{nullptr, nullptr}}, none);
-    if (ok) {
-      double2* O = g.out + (size_t)it * W * W;
-      for (int e = tid; e < W * W; e += 256) O[e] = M[(size_t)(e / W) * N + e % W];
+    double2* O = g.out + (size_t)it * W * W;
+    if (__syncthreads_or(keys_wild(rL.row, N) || keys_wild(rM.col, N) || keys_wild(rR.col, N))) {
+      // (only the matrices' own extents: a zero of the padding times an infinity is not 0)
+      rot_fp64(T, N, LH, N, M, N, W, n2, n1);
+      __syncthreads();
+      rot_fp64(O, W, T, N, R, N, W, W, n2);
+    } else {
+      ok = E::mm(cx, T, LH, rL.row, M, rM.col, N, Epi{T, 0, rT}, none);
+      if (ok) ok = E::mm(cx, M, T, rT.row, R, rR.col, N, Epi{M, 0, Rec{nullptr, nullptr}}, none);
+      if (ok)
+        for (int e = tid; e < W * W; e += 256) O[e] = M[(size_t)(e / W) * N + e % W];
     }
     __syncthreads();
   }
@@ -118,7 +137,15 @@ __global__ void __launch_bounds__(256, 2) k_oz_ufinal(const Problem* __restrict_
   double2* C = P.dU + (size_t)k * WW;
   rot_begin<E>(sh);
   OzCtx cx{base, base + E::SB_OFFSET, sh.tmem, smem_u32(&sh.mbar), 0u, s_rowexp, s_colexp, &sh.bad};
-  const bool ok = E::mm(cx, C, P.U0 + (size_t)k * WW, nullptr, U, nullptr, W, Epi{C, 0, Rec{nullptr, nullptr}}, NoAdd());
+  const double2* U0 = P.U0 + (size_t)k * WW;
+  const bool ok = E::mm(cx, C, U0, nullptr, U, nullptr, W, Epi{C, 0, Rec{nullptr, nullptr}}, NoAdd());
+  // the scales that the product took
+  bool wild = false;
+  for (int i = threadIdx.x; i < W; i += 256) wild = wild || exp_wild(s_rowexp[i]) || exp_wild(s_colexp[i]);
+  if (__syncthreads_or(wild)) {
+    rot_fp64(C, W, U0, W, U, W, W, W, W);
+    __syncthreads();
+  }
   if (ok)
     for (int e = threadIdx.x; e < WW; e += 256) U[e] = C[e];
   else if (threadIdx.x == 0) P.st->error = 2;

@@ -47,9 +47,11 @@ __device__ __forceinline__ unsigned long long abs_bits(double v) {
   return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
 }
 
-// exponent e with |v| < 2^e from the bits of |v| (0 for v == 0); integer ops only
+// exponent e with |v| < 2^e from the bits of |v| (0 for v == 0); integer ops only.  Not below -900:
+// a product's scale, less its digits' 56 to 63 bits, then stays inside FP64's exponents for any
+// partner of a unitary's size (int64_scaled_to_double does not check), and what lies lower rounds to 0.
 __device__ __forceinline__ int exp_above_bits(unsigned long long ab) {
-  return ab ? (int)(ab >> 52) - 1022 : 0;
+  return ab ? max((int)(ab >> 52) - 1022, -900) : 0;
 }
 
 // N = round(v * 2^(49 - e)) as a signed integer (|N| <= 2^49), integer ops only

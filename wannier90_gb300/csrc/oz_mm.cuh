@@ -75,12 +75,26 @@ __device__ __forceinline__ unsigned scale_key(double re, double im) {
   const unsigned long long ab = max(abs_bits(re), abs_bits(im));
   return ab ? (unsigned)(ab >> 52) + 1u : 0u;
 }
-__device__ __forceinline__ int key_exp(unsigned key) { return key ? (int)key - 1023 : 0; }
+// (two of these scales and a product's 63 digit bits stay inside FP64's exponents)
+constexpr int kExpMin = -480;
+__device__ __forceinline__ int key_exp(unsigned key) { return key ? max((int)key - 1023, kExpMin) : 0; }
 
 struct Rec {
   unsigned* row;
   unsigned* col;
 };
+
+// Scales that the digits carry through two products in a row: outside of this range a scale may
+// leave FP64's exponents on the way, and the keys of NaN and infinities (2048) read as 2^1025.
+// k_oz_rotate, k_oz_ufinal and k_oz_polar leave such operands to FP64.
+constexpr int kExpSafe = 290;
+__device__ __forceinline__ bool exp_wild(int e) { return e > kExpSafe || e < -kExpSafe; }
+// this thread's share of n keys
+__device__ __forceinline__ bool keys_wild(const unsigned* keys, int n) {
+  bool w = false;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) w = w || exp_wild(key_exp(keys[i]));
+  return w;
+}
 
 // Power-of-two scales of a product: the exponent above the largest |re| or |im| of every
 // row of A and every column of B, from the operands' records where given (arow / bcol),
@@ -121,7 +135,7 @@ __device__ __forceinline__ void ab_exponents(OzCtx& cx, const double2* A, const 
     for (int o = 1; o < TPI; o <<= 1)
       mx = max(mx, (unsigned long long)__shfl_xor_sync(0xffffffffu, (long long)mx, o));
     if (idx < ITEMS && sub == 0)
-      (row_of_a ? cx.rowexp : cx.colexp)[r] = rec != nullptr ? key_exp(rec[r]) : exp_above_bits(mx);
+      (row_of_a ? cx.rowexp : cx.colexp)[r] = rec != nullptr ? key_exp(rec[r]) : max(exp_above_bits(mx), kExpMin);
   }
 }
 
