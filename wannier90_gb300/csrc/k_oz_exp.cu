@@ -16,7 +16,8 @@
 //   * the scaling follows sqrt(||X^2||_1), which bounds the 2-norm of the anti-Hermitian X and is
 //     half of ||X||_1 or less for a full W = 32 matrix: one squaring less on average;
 //   * the optimal step's X is a multiple of the trial step's, so its powers are the trial's: the
-//     factor f goes into the coefficients and the second exp starts after them.
+//     factor f goes into the coefficients and the second exp starts after them.  (Where the trial's
+//     norm says too little about the optimal step's -- see `reuse` -- the second exp forms its own.)
 // Truncation: theta^(m+1) / (m+1)! <= 2^-53 at the 2-norm theta (||e^X||_2 = 1).
 //
 // One CTA (256 threads) per (problem, k).
@@ -147,16 +148,22 @@ __global__ void __launch_bounds__(256, 2) k_oz_exp(const Problem* __restrict__ p
   OzCtx cx{base, base + E::SB_OFFSET, tmem_slot, smem_u32(&mbar), 0u, s_rowexp, s_colexp, &s_bad};
   bool ok = true;
   float rho;
-  double f = 1.0;
+  double f = which == 0 ? 1.0 : st->s_second / st->s_trial;
   bool have3 = false;
   int nprod = 0;
-  if (which == 0) {
+  // The trial's powers serve the optimal step where its norm's estimate is sure to 2^-10: abs_est
+  // leaves out moduli of X^2 below 2^-60, at most 2^-53 in a column sum, against 2^-40 or more.  Below
+  // that, a step up to 256 times as long still has a norm under T4's bound, whatever was left out;
+  // a longer one, or any after a trial of length 0 (f is NaN or infinite), starts from its own X.
+  const bool reuse = which == 1 && (fabs(f) <= 256.0 || (info[0] >= 0x1p-20f && fabs(f) <= 0x1p100));
+  if (!reuse) {
     // ---- X = s D (first D = coefG G + coefD D_prev; in the symmetry-adapted mode k_sym_dir has
     // formed D already).  Each product and the sum rounded on its own, as the oracle forms D:
     // no contraction into an FMA, whose choice of product would follow the code's shape.
     double2* Dk = P.D + (size_t)k * WW;
-    const double s = st->s_trial;
-    const bool form_d = P.sym_nir == 0;
+    const double s = which == 0 ? st->s_trial : st->s_second;
+    const bool form_d = which == 0 && P.sym_nir == 0;
+    f = 1.0;
     const double cg = st->coefG, cd = st->coefD;
     const double2* Gk = form_d ? (st->use_gp ? P.pc_gp : P.G) + (size_t)k * WW : nullptr;
 #pragma unroll 4
@@ -192,14 +199,13 @@ __global__ void __launch_bounds__(256, 2) k_oz_exp(const Problem* __restrict__ p
     for (int w = 0; w < 8; ++w) cmax = fmaxf(cmax, s_wmax[w]);
     rho = sqrtf(cmax * 1.001f);
   } else {
-    f = st->s_second / st->s_trial;
     rho = info[0] * fabsf((float)f) * 1.0001f;
     have3 = info[1] != 0.0f;
   }
   int m, js;
   exp_plan(rho, m, js);
   f *= ldexp(1.0, -js);
-  if (which == 1) {
+  if (reuse) {
     // the powers kept by the trial step, with the records of those that enter a product
     const bool need = m < 12 || !have3;
     if (E::MATS_IN_SMEM || need)
