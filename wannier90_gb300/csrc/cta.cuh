@@ -54,7 +54,6 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 //     off-diagonal part of ~1e-6, from which the FP64 sweeps -- the same rotations and the
 //     same convergence test -- need two instead of seven to ten.  14 W^3 FMA for that against
 //     12 W^3 per sweep.
-// Measured on a GB300 at the Loewdin step of 1000 matrices of W = 32: see k_lowdin.
 // ----------------------------------------------------------------------------
 struct JacF2 {
   float x, y;
@@ -351,6 +350,67 @@ __device__ __noinline__ static int cta_jacobi(double2* H, double2* V, int W, int
     if (skip > 0.0 && block_sum((double)rotated, red) == 0.0) return sweep + 1;
   }
   return -1;
+}
+
+// Unitary polar factor X (X^H X)^{-1/2} of an m x w matrix by the Newton-Schulz iteration
+// X <- X (3 I - X^H X) / 2 on X itself: unitary to roundoff, its error that of the products times X's
+// condition number.  (The eigenpairs of X^H X carry the square of that number: above ~1e4 what they
+// give is not unitary, and no first-order correction is enough.)  Singular values below 1 grow by 1.5 a
+// step, so this takes 1.7 log10(cond) + 6 steps or so of 6 m w^2 FMA.  X (ldx) and Y (ldy) take turns,
+// G is w x w scratch, red one double per thread.  Returns the one that holds the result, or null where
+// 120 steps were not enough (a singular value of 0).  All threads call.
+__device__ __noinline__ static double2* cta_polar_ns(double2* X, int ldx, double2* Y, int ldy, double2* G, int m, int w,
+                                                     double* red) {
+  __shared__ int s_far;
+  double sq = 0.0;
+  for (int e = threadIdx.x; e < m * w; e += blockDim.x) sq += cabs2(X[(size_t)(e / m) * ldx + e % m]);
+  sq = block_sum(sq, red);
+  if (!(sq > 0.0) || !isfinite(sq)) return nullptr;
+  // |X|_2 <= |X|_F < 2^half
+  int half;
+  frexp(sq, &half);
+  half = (half + 1) >> 1;
+  const double r = ldexp(1.0, -half);
+  for (int e = threadIdx.x; e < m * w; e += blockDim.x) {
+    double2& x = X[(size_t)(e / m) * ldx + e % m];
+    x = cscale(x, r);
+  }
+  __syncthreads();
+  for (int step = 0; step < 120; ++step) {
+    if (threadIdx.x == 0) s_far = 0;
+    __syncthreads();
+    bool far = false;
+    for (int e = threadIdx.x; e < w * (w + 1) / 2; e += blockDim.x) {
+      int i, j;
+      tri_index(e, i, j);
+      double2 g = cmk(0, 0);
+      for (int l = 0; l < m; ++l) cfmac(g, X[(size_t)i * ldx + l], X[(size_t)j * ldx + l]);
+      if (i == j) g.y = 0.0;
+      // |X^H X - I| below 1e-8 / w elementwise: the step leaves less than 1e-16
+      far = far || !(fabs(g.x - (i == j ? 1.0 : 0.0)) + fabs(g.y) < 1.0e-8 / w);
+      g = cmk((i == j ? 1.5 : 0.0) - 0.5 * g.x, -0.5 * g.y);
+      G[(size_t)j * w + i] = g;
+      if (i < j) G[(size_t)i * w + j] = cconj(g);
+    }
+    if (far) s_far = 1;
+    __syncthreads();
+    const bool done = s_far == 0;
+    for (int e = threadIdx.x; e < m * w; e += blockDim.x) {
+      const int i = e % m, j = e / m;
+      double2 y = cmk(0, 0);
+      for (int l = 0; l < w; ++l) cfma(y, X[(size_t)l * ldx + i], G[(size_t)j * w + l]);
+      Y[(size_t)j * ldy + i] = y;
+    }
+    __syncthreads();
+    double2* t = X;
+    X = Y;
+    Y = t;
+    const int ld = ldx;
+    ldx = ldy;
+    ldy = ld;
+    if (done) return X;
+  }
+  return nullptr;
 }
 
 }  // namespace w90g

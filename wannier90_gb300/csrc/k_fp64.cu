@@ -1385,15 +1385,20 @@ __global__ void k_log_init(const Problem* __restrict__ probs) {
 // k_lowdin: overlap_project's U(k) = Z V^dagger from A(k) = Z S V^dagger
 // (src/overlap.F90:842-860), computed as U = A (A^H A)^{-1/2} = A V L^{-1/2} V^H with the
 // Jacobi eigenpairs (V, L) of A^H A: the same unitary polar factor for full-rank A.  The
-// eigenpairs carry the square of A's condition number; the two steps after them take it back
-// to the condition number itself: one Newton-Schulz step (U unitary again), then U <- U (I + X)
+// eigenpairs carry the square of A's condition number; while that is small (condition numbers up to
+// kLowdinCond, square times 2^-53 below 2e-9) the two steps after them take it back to the
+// condition number itself: one Newton-Schulz step (U unitary again), then U <- U (I + X)
 // with X anti-Hermitian from X H + H X = H1 - H1^H, H1 = U^H A (the polar factor is the U
-// that makes H1 Hermitian), solved in the eigenbasis, where H = L^{1/2}.
+// that makes H1 Hermitian), solved in the eigenbasis, where H = L^{1/2}.  Both are of first order:
+// above kLowdinCond the iteration runs from A itself instead (cta_polar_ns), and the
+// eigenvalues only give the verdict on A's rank.
 // Input A(k) in U[cur](k) (the reference reads A into u_matrix, src/wannier_prog.F90:523-529);
 // output U overwrites it.  One CTA (256 threads) per (problem, k).
 // Status per k: 0 ok, 1 rank deficient, 2 Jacobi not converged.  A matrix whose status is
 // kPolarDone on entry has been finished by k_oz_polar.
 // ----------------------------------------------------------------------------
+constexpr double kLowdinCond = 4.0e3;
+
 __global__ void __launch_bounds__(256) k_lowdin(const Problem* __restrict__ probs, WorkMap wm,
                                                 int* __restrict__ status) {
   extern __shared__ double2 smem[];
@@ -1425,6 +1430,18 @@ __global__ void __launch_bounds__(256) k_lowdin(const Problem* __restrict__ prob
     s_h[j] = sqrt(l);
   }
   __syncthreads();
+  double hmin = s_h[0], hmax = s_h[0];
+  for (int j = 1; j < W; ++j) {
+    hmin = fmin(hmin, s_h[j]);
+    hmax = fmax(hmax, s_h[j]);
+  }
+  if (!bad && hmax > kLowdinCond * hmin && isfinite(hmax)) {
+    const double2* Q = cta_polar_ns(A, W, T, W, S, W, W, red);
+    for (int e = threadIdx.x; e < WW; e += blockDim.x)
+      if (Q) Uk[e] = Q[e];
+    if (threadIdx.x == 0) status[blockIdx.x] = Q ? 0 : 1;
+    return;
+  }
   for (int e = threadIdx.x; e < WW; e += blockDim.x) T[e] = cscale(V[e], 1.0 / s_h[e / W]);
   __syncthreads();
   cta_gemm<false>(S, W, A, W, T, W, W);      // S <- A V L^{-1/2}
