@@ -77,7 +77,8 @@ struct DisDev {
   const double2* sym_db;
   double2* sym_ws;
   int* sym_status;
-  double2* zfroz;        // [k] nb x nb: the frozen states' part of Zf (it never changes); null: not split off
+  double2* zfroz;        // [k] nb x nb, kWs nb^2 apart: the frozen states' part of Zf (it never changes); null: not
+                         // split off
   double2* V;            // [k] nb x W (leading dimension nb): U_opt U0 for the final rotation; null: not formed
   const int* pstat;      // [k] kPolarDone where k_oz_polar has formed this kernel's polar factor; null: never
 };
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(256) k_dis_zfroz(DisDev D) {
   const int k = blockIdx.x;
   const int nb = D.nb, n = D.ndim[k], B = D.B;
   const size_t NN = (size_t)nb * nb;
-  double2* Z = D.zfroz + (size_t)k * NN;
+  double2* Z = D.zfroz + (size_t)k * kWs * NN;
   for (int e = threadIdx.x; e < (int)NN; e += blockDim.x) Z[e] = cmk(0, 0);
   __syncthreads();
   for (int b = 0; b < B; ++b) {
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(256) k_dis_z(DisDev D, int cur, int to_in, int
   double2* ws = D.ws + (size_t)k * kWs * NN;
   double2* Zacc = ws + NN;
   double2* Z = (to_in ? D.Zin : D.Zout) + (size_t)k * NN;
-  const double2* Zf = D.zfroz ? D.zfroz + (size_t)k * NN : nullptr;
+  const double2* Zf = D.zfroz ? D.zfroz + (size_t)k * kWs * NN : nullptr;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x)
     Zacc[e] = Zf ? Zf[(size_t)(e / n) * nb + e % n] : cmk(0, 0);
   for (int b = 0; b < B; ++b) {
@@ -1070,14 +1071,15 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   const size_t NN = (size_t)nb * nb;
   const size_t o_nn = take((size_t)K * B * 4), o_wb = take(B * 8), o_ndim = take(K * 4), o_nfirst = take(K * 4),
                o_nfroz = take(K * 4), o_ffirst = take(K * 4), o_nfidx = take((size_t)K * nb * 4),
-               o_eig = take((size_t)K * nb * 8), o_mraw = take((size_t)K * B * NN * 16),
+               o_eig = take((size_t)K * nb * 8),
+               // (these four one after the other: the last rotation's work matrices lie there, see below)
+               o_mraw = take((size_t)K * B * NN * 16), o_zin = take((size_t)K * NN * 16),
+               o_zout = take((size_t)K * NN * 16), o_vz = take((size_t)K * NN * 16),
                o_mw = take((size_t)K * B * NN * 16), o_a = take((size_t)K * nb * W * 16),
                o_u0b = take((size_t)K * nb * W * 16), o_u1b = take((size_t)K * nb * W * 16),
-               o_zin = take((size_t)K * NN * 16), o_zout = take((size_t)K * NN * 16),
                o_uw = take((size_t)K * W * W * 16), o_m0 = take((size_t)K * B * W * W * 16),
                o_ws = take((size_t)K * kWs * NN * 16), o_wk1 = take(K * 8), o_wk = take(K * 8),
-               o_rw = take(W >= 9 ? (size_t)std::min(kRotateCtas, K * B) * 4 * NN * 16 : 0), o_rf = take(4),
-               o_st = take(K * 4), o_ps = take(K * 4), o_zf = take(any_froz && nir == 0 ? (size_t)K * NN * 16 : 0), o_vz = take((size_t)K * NN * 16), o_sw = take(4);
+               o_st = take(K * 4), o_ps = take(K * 4), o_rf = take(4), o_sw = take(4);
   // symmetry tables: ik, moff, mem, goff, grp, status; slot matrices; workspace
   std::vector<int> sym_ints;
   if (nir > 0) {
@@ -1159,8 +1161,9 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
     D.wk = (double*)(a + o_wk);
     D.status = (int*)(a + o_st);
     D.pstat = (const int*)(a + o_ps);
-    D.zfroz = any_froz && nir == 0 ? (double2*)(a + o_zf) : nullptr;
-    D.V = (double2*)(a + o_ws) + 6 * NN;   // a slot of the workspace that nothing else uses then
+    // (slots of the workspace that nothing else uses, and that nothing else uses then)
+    D.zfroz = any_froz && nir == 0 ? (double2*)(a + o_ws) + 7 * NN : nullptr;
+    D.V = (double2*)(a + o_ws) + 6 * NN;
     D.Vz = (double2*)(a + o_vz);
     D.max_sweeps = (int*)(a + o_sw);
     D.sym_nir = nir;
@@ -1311,7 +1314,10 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
     r.B = B;
     r.nnlist = D.nnlist;
     r.out = D.M0;
-    r.work = (double2*)(a0 + o_rw);
+    // Work matrices where Mraw, Zin, Zout and Vz were: K (B + 3) / 4 CTAs' worth, all of them from 136 k
+    // of 6 neighbours on
+    r.work = (double2*)(a0 + o_mraw);
+    r.ctas = (int)std::min<size_t>(kRotateCtas, (o_mw - o_mraw) / (4 * NN * 16));
     r.failed = (int*)(a0 + o_rf);
     DIS_CHECK(launch(kDisRotate, [&] { oz_rotate_launch(r, K * B, st); }));
     DIS_CHECK(cudaMemcpyAsync(&rot_failed, r.failed, 4, cudaMemcpyDeviceToHost, st));

@@ -770,6 +770,7 @@ int Engine::project(std::string& err) {
     r.B = s0.B;
     r.nnlist = hprobs_[0].nnlist;
     r.work = hprobs_[0].M[1];
+    r.ctas = kRotateCtas;
     r.failed = d_status_;
     W90G_CHECK(cudaMemsetAsync(d_status_, 0, sizeof(int), st));
     W90G_CHECK(oz_rotate_launch(r, s0.K * s0.B, st));

@@ -159,7 +159,7 @@ cudaError_t rotate_wp(const RotateArgs& a, int items, cudaStream_t s) {
   constexpr int sm = (int)ExpProd<WP, false>::BYTES;
   cudaError_t e = cudaFuncSetAttribute(k_oz_rotate<WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   if (e != cudaSuccess) return e;
-  k_oz_rotate<WP><<<std::min(items, kRotateCtas), 256, sm, s>>>(a, items);
+  k_oz_rotate<WP><<<std::min(items, a.ctas), 256, sm, s>>>(a, items);
   return cudaGetLastError();
 }
 

@@ -39,11 +39,12 @@ struct RotateArgs {
   int w, n, B;           // n >= rows(k) and w: order of the work matrices
   const int* nnlist;     // [item] k + b
   double2* out;          // [item] w x w (may be m)
-  double2* work;         // [kRotateCtas] 4 n x n
+  double2* work;         // [ctas] 4 n x n
+  int ctas;              // CTAs launched at most (at least 1)
   int* failed;           // set to 1 when a bounded wait ran out
 };
 
-constexpr int kRotateCtas = 304;   // two per SM
+constexpr int kRotateCtas = 304;   // two per SM: more are of no use
 
 // n <= kPolarMaxN
 cudaError_t oz_rotate_launch(const RotateArgs& a, int items, cudaStream_t s);
