@@ -86,3 +86,56 @@ def test_fused_iteration_equals_the_kernels_one_by_one(emu, shapes, num_iter, wi
         assert len(a) == 1 + len(r.iters)
         for row, it in zip(a, [r.initial] + r.iters):
             assert abs(row[3] - it.spread.om_tot) <= 1e-10 * abs(it.spread.om_tot) + 1e-11
+
+
+@pytest.fixture(scope="module")
+def emu_dis(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ not available")
+    tmp = tmp_path_factory.mktemp("emu_dis_split")
+    src = open(os.path.join(CSRC, "dis.cu")).read()
+    src = src[:src.index("int dis_run(")] + "}  // namespace w90g\n"
+    src = re.sub(r"extern __shared__ double2 (\w+)\[\];", r"double2* \1 = emu_dyn_smem<double2>();", src)
+    (tmp / "dis_emu.cu").write_text(src)
+    out = str(tmp / "emu_dis_split.so")
+    subprocess.run([gxx, "-std=c++20", "-O1", "-shared", "-fPIC", "-D__CUDACC__", "-DEMU_FIBERS", "-I" + str(tmp),
+                    "-I" + os.path.join(HERE, "emu"), "-I" + CSRC, os.path.join(HERE, "emu", "emu_dis_split.cpp"),
+                    os.path.join(CSRC, "sym_tables.cpp"), "-o", out], check=True)
+    return C.CDLL(out)
+
+
+# frozen windows of several states per k, of none, and the silicon case's; 16, 64 and 32 threads a step
+@pytest.mark.parametrize("name,step_threads", [("silicon_dis", 64), ("copper_dis", 16), ("basic2_dis", 32)])
+def test_split_disentanglement_against_the_oracle(emu_dis, name, step_threads):
+    """The engine's forms of the disentanglement kernels -- frozen states split off Z, one rotation by
+    U_opt U0 -- on the reference's cases: Omega_I lines 1e-10, U_opt U and M0 1e-9."""
+    from tests import golden_cases as G
+    d = G.load(name)
+    kn = d["knobs"]
+    km = O.kmesh_get(d["real_lattice"], d["kpt_latt"], int(kn["search_shells"]))
+    M = G.assemble_m(d, km["nnlist"], km["nncell"])
+    nb, W, K, B = int(d["num_bands"]), int(kn["num_wann"]), len(d["kpt_latt"]), km["nntot"]
+    dc = G.dis_control(d)
+    dc.num_iter, dc.conv_tol = 4, 0.0
+    f = lambda X: np.ascontiguousarray(np.swapaxes(X, -1, -2)).astype(np.complex128)
+    Mf, Af, eig = f(M), f(d["amn"]), np.ascontiguousarray(d["eig"])
+    nn, wb = np.ascontiguousarray(km["nnlist"], dtype=np.int32), np.ascontiguousarray(km["wb"])
+    log, status = np.zeros((dc.num_iter, 3)), np.zeros(1, dtype=np.int32)
+    U0, M0, Uo = (np.zeros(s, dtype=np.complex128) for s in ((K, W, W), (K, B, W, W), (K, W, nb)))
+    vp = lambda a: C.c_void_p(a.ctypes.data)
+    lib = emu_dis
+    lib.emu_dis_engine.argtypes = ([C.c_int] * 4 + [C.c_void_p, C.c_void_p, C.c_double] + [C.c_void_p] * 3 +
+                                   [C.c_int] + [C.c_double] * 3 + [C.c_int] + [C.c_double] * 2 + [C.c_int] * 2 +
+                                   [C.c_void_p] * 5)
+    rc = lib.emu_dis_engine(nb, W, K, B, vp(nn), vp(wb), km["wbtot"], vp(eig), vp(Mf), vp(Af), dc.num_iter,
+                            dc.mix_ratio, dc.win_min, dc.win_max, int(dc.frozen_states), dc.froz_min, dc.froz_max, 32,
+                            step_threads, vp(log), vp(U0), vp(M0), vp(Uo), vp(status))
+    assert rc == 0 and status[0] == 0
+    U0o, M0o, Uoo, _, recs = O.dis_main(M, d["amn"], d["eig"], km, W, dc)
+    assert len(recs) == dc.num_iter
+    for row, r in zip(log, recs):
+        assert abs(row[1] - r.omega_i_prev) < 1e-10 and abs(row[2] - r.omega_i) < 1e-10
+    g = lambda X: np.swapaxes(X, -1, -2)
+    np.testing.assert_allclose(g(Uo) @ g(U0), Uoo @ U0o, atol=1e-9)
+    np.testing.assert_allclose(g(M0), M0o, atol=1e-9)
