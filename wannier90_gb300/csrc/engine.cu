@@ -70,7 +70,6 @@ namespace {
 constexpr size_t kAlign = 256;
 size_t align_up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 constexpr int kTileW = 32;
-constexpr int kOmegaFused = 16, kOmegaOneCta = 3072;   // as in k_fp64.cu
 constexpr int kPolarMinW = 9;   // projection on the tensor cores from this width on (see project)
 
 #define W90G_CHECK(call)                                                          \

@@ -277,11 +277,8 @@ __device__ __forceinline__ bool last_chunk_cta(unsigned* arrive, int nchunk) {
   return last;
 }
 
-// kOmegaFused in a pass's slot: the last CTA of the trial's and of the optimal step's second pass
-// goes on with k_ctrl_step and k_ctrl_end, and the first pass of a problem of at most kOmegaOneCta
-// statistics (k,b,n) also does the second's work in its last CTA: one SM's FP64 pipe takes ~4 ns
-// for each, a launch of its own 8 to 10 us.
-constexpr int kOmegaFused = 16, kOmegaOneCta = 3072;
+// (kOmegaOneCta: one SM's FP64 pipe takes ~4 ns for each statistic of the second pass, a launch of its
+// own 8 to 10 us)
 __device__ __forceinline__ bool omega_one(const Problem& P, int slot) {
   return (slot & kOmegaFused) != 0 && P.K * P.B * P.W <= kOmegaOneCta;
 }

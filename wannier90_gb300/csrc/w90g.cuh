@@ -204,6 +204,12 @@ struct Problem {
 
 constexpr int kSymWork = 5;
 
+// kOmegaFused in the slot of a spread pass (k_omega_p1, k_omega_p2): the last CTA of the trial's and of
+// the optimal step's second pass goes on with the control step, and the first pass of a problem of at
+// most kOmegaOneCta statistics (k,b,n) also does the second's work in its last CTA.  The engine
+// leaves the second pass out by the same rule.
+constexpr int kOmegaFused = 16, kOmegaOneCta = 3072;
+
 // Work map: blockIdx.x -> (problem, local index) over a prefix sum.
 struct WorkMap {
   const int* offs;  // nprob+1 prefix sums of work items per problem
