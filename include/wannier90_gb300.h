@@ -238,8 +238,10 @@ int w90g_read_mmn_device(const char* path, int nb, int nk, int nntot, const int*
 long long w90g_kernel_launches(void* handle);
 /* Profiling run of wannierise on device buffers: every kernel launched alone and timed
  * with CUDA events on the launching stream (at most max_iters iterations).  ms[i] and
- * counts[i] (w90g_profile_kernel_name(i), i < 8) receive total time and launches that
- * did work.  Returns ierr.  The per-kernel sequence and arithmetic equal cwannierise's. */
+ * counts[i] (w90g_profile_kernel_name(i), i < 9) receive total time and launches that
+ * did work.  Returns ierr.  The per-kernel sequence and arithmetic equal cwannierise's:
+ * k_omega includes the control steps in its last CTA (k_ctrl_step and k_ctrl_end stay 0), and
+ * k_grad the search where the solve has it there (k_ctrl_search then stays 0). */
 int w90g_profile_device(void* handle, double* d_m_matrix, double* d_u_matrix, int max_iters,
                         double* ms, int* counts);
 const char* w90g_profile_kernel_name(int i);

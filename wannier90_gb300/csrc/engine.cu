@@ -28,8 +28,6 @@ __global__ void k_grad_search(const Problem* probs, WorkMap wm);
 __global__ void k_ctrl_search(const Problem* probs);
 __global__ void k_exp_u(const Problem* probs, WorkMap wm, int which);
 __global__ void k_m_update(const Problem* probs, WorkMap wm, int mode, int which);
-__global__ void k_ctrl_step(const Problem* probs, int nprob);
-__global__ void k_ctrl_end(const Problem* probs);
 __global__ void k_log_init(const Problem* probs);
 __global__ void k_lowdin(const Problem* probs, WorkMap wm, int* status);
 __global__ void k_unitarity(const Problem* probs, WorkMap wm, double* out);
@@ -1047,29 +1045,34 @@ int Engine::wannierise_profiled(int max_iters, double* ms, int* cnt, std::string
   const int iters = std::min(max_iters, max_iter_);
   for (int it = 0; it < iters && !rc; ++it) {
     if (guide_w_) rc |= timed(kPInit, [&] { k_phases<<<dim3(guide_w_, np), 256, 0, st>>>(dprobs_, 1); });
-    rc |= timed(kPGrad, [&] {
-      k_grad<<<n_grad_, 256, 0, st>>>(dprobs_, wmg);
-      if (n_ir_) k_sym_grad<<<n_ir_, 256, 0, st>>>(dprobs_, WorkMap{d_offs_ir_, np});
-    });
-    if (pc_tiles_) {
-      rc |= timed(kPPrecond, [&] { k_precond<<<dim3(pc_tiles_, np), 256, 0, st>>>(dprobs_, 0); });
-      rc |= timed(kPPrecond, [&] { k_precond<<<dim3(pc_tiles_, np), 256, 0, st>>>(dprobs_, 1); });
+    // the launches of launch_iteration
+    if (fuse_search()) {
+      rc |= timed(kPGrad, [&] { k_grad_search<<<n_grad_, 256, 0, st>>>(dprobs_, wmg); });
+    } else {
+      rc |= timed(kPGrad, [&] {
+        k_grad<<<n_grad_, 256, 0, st>>>(dprobs_, wmg);
+        if (n_ir_) k_sym_grad<<<n_ir_, 256, 0, st>>>(dprobs_, WorkMap{d_offs_ir_, np});
+      });
+      if (pc_tiles_) {
+        rc |= timed(kPPrecond, [&] { k_precond<<<dim3(pc_tiles_, np), 256, 0, st>>>(dprobs_, 0); });
+        rc |= timed(kPPrecond, [&] { k_precond<<<dim3(pc_tiles_, np), 256, 0, st>>>(dprobs_, 1); });
+      }
+      rc |= timed(kPCtrlSearch, [&] {
+        k_ctrl_search<<<np, 256, 0, st>>>(dprobs_);
+        if (n_ir_) k_sym_dir<<<n_ir_, 256, 0, st>>>(dprobs_, WorkMap{d_offs_ir_, np});
+      });
     }
-    rc |= timed(kPCtrlSearch, [&] {
-      k_ctrl_search<<<np, 256, 0, st>>>(dprobs_);
-      if (n_ir_) k_sym_dir<<<n_ir_, 256, 0, st>>>(dprobs_, WorkMap{d_offs_ir_, np});
-    });
     rc |= timed(kPExpU, [&] { launch_exp(st, 0); });
     rc |= timed(kPMUpdate, [&] { launch_mupdate(st, 0); });
-    rc |= timed(kPOmega, [&] { launch_omega(st, 0); });
-    rc |= timed(kPCtrlStep, [&] { k_ctrl_step<<<(np + 127) / 128, 128, 0, st>>>(dprobs_, np); });
+    rc |= timed(kPOmega, [&] { launch_omega(st, kOmegaFused); });
     W90G_CHECK(cudaMemcpy(&hs, hprobs_[0].st, sizeof(CtrlState), cudaMemcpyDeviceToHost));
     if (hs.do_second) {
       rc |= timed(kPExpU, [&] { launch_exp(st, 1); });
       rc |= timed(kPMUpdate, [&] { launch_mupdate(st, 1); });
-      rc |= timed(kPOmega, [&] { launch_omega(st, 1); });
+      rc |= timed(kPOmega, [&] { launch_omega(st, kOmegaFused + 1); });
+    } else {
+      launch_omega(st, kOmegaFused + 1);   // the iteration's end alone
     }
-    rc |= timed(kPCtrlEnd, [&] { k_ctrl_end<<<np, 128, 0, st>>>(dprobs_); });
     W90G_CHECK(cudaMemcpy(&hs, hprobs_[0].st, sizeof(CtrlState), cudaMemcpyDeviceToHost));
     if (hs.done) break;
   }

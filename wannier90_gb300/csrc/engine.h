@@ -94,7 +94,7 @@ class Engine {
   size_t arena_bytes() const { return arena_bytes_; }
   // device bytes setup() would allocate for these problems (HBM admission)
   static size_t estimate_bytes(const std::vector<ProblemSpec>& specs);
-  // wann_main with each kernel launched individually and timed with CUDA events on the
+  // wann_main with launch_iteration's kernels launched individually and timed with CUDA events on the
   // launching stream; ms[i] / cnt[i] accumulate per kernel kind (kProfNames order);
   // only launches that did work are counted (skipped second passes are excluded).
   int wannierise_profiled(int max_iters, double* ms, int* cnt, std::string& err);

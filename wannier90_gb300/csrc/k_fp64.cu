@@ -117,7 +117,9 @@ __global__ void k_mdiag(const Problem* __restrict__ probs, WorkMap wm) {
 }
 
 // ----------------------------------------------------------------------------
-// k_ctrl_step: internal_optimal_step (src/wannierise.F90:1528-1596).  One thread per problem.
+// k_ctrl_step: internal_optimal_step (src/wannierise.F90:1528-1596).  One thread per problem.  A solve
+// runs ctrl_step and ctrl_end in the spread passes' last CTAs; as kernels of their own they are the
+// reference sequence of the CPU emulation.
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void ctrl_step(const Problem& P) {
   CtrlState* st = P.st;
