@@ -1093,9 +1093,13 @@ int dis_run(const DisSpec& s, DisResult& r, std::string& err) {
   int mmax = 0;
   for (int k = 0; k < K; ++k) mmax = std::max(mmax, ndim[k] - nfroz[k]);
   const size_t step_smem = 3 * (size_t)mmax * mmax * 16;
-  // threads of k_dis_step: a round of rotations of an m x m matrix has (m/2)(m/2-1)/2 blocks of H
-  // and m m/2 elements of V, 60 at m = 8, and two CTA barriers: two warps up to m = 12
-  const int step_threads = mmax <= 12 ? 64 : 256;
+  // Threads of k_dis_step: a round of rotations of an m x m matrix has (m/2)(m/2-1)/2 blocks of H and
+  // m m/2 elements of V (38 at m = 8, 87 at 12, 156 at 16) and two CTA barriers.  us per iteration
+  // with 64 / 128 / 256 threads:
+  //   m         8             10            11            12            14            16            24
+  //   64 k    150 153 162   194 189 199   247 215 225   261 229 230   315 267 270   389 336 310   934 669 633
+  //   512 k   175 185 207   234 240 262   299 289 311   316 309 327   425 415 437   545 529 535  1460 1397 1396
+  const int step_threads = mmax <= 10 ? 64 : mmax <= 14 ? 128 : 256;
   int cur = 0, it = 0, rot_failed = 0;
   char* a0 = nullptr;
   double womegai = 0.0;

@@ -279,8 +279,9 @@ __device__ __forceinline__ bool last_chunk_cta(unsigned* arrive, int nchunk) {
   return last;
 }
 
-// (kOmegaOneCta: one SM's FP64 pipe takes ~4 ns for each statistic of the second pass, a launch of its
-// own 8 to 10 us)
+// kOmegaOneCta: against a launch of its own the second pass in the first's last CTA takes, per spread,
+// 4 to 6 us less at 648 and 1152 statistics, 2 to 4 at 2304, 2 at 3000 and 3072, -1 to +2 at 3600 to
+// 4608, and 2 to 5 us more at 6144.
 __device__ __forceinline__ bool omega_one(const Problem& P, int slot) {
   return (slot & kOmegaFused) != 0 && P.K * P.B * P.W <= kOmegaOneCta;
 }
