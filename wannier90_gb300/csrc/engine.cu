@@ -752,9 +752,9 @@ int Engine::project(std::string& err) {
       }
     }
   }
-  // M <- U^H M U': tensor cores under the same rule as the polar factors, work in what the
-  // projection does not use (G, D, dU and the second M buffer follow one another only by chance, so
-  // the largest of them, the M buffer)
+  // M <- U^H M U': tensor cores from num_wann 9 on where the second M buffer, which the projection does
+  // not use, holds the work matrices of kRotateCtas CTAs (1216 blocks and more); smaller meshes keep
+  // the FP64 kernel
   const ProblemSpec& s0 = specs_[0];
   const size_t mat = (size_t)s0.W * s0.W;
   if (nprob() == 1 && s0.W >= kPolarMinW && s0.W <= kPolarMaxN &&

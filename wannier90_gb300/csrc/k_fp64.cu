@@ -236,7 +236,7 @@ __global__ void k_ctrl_end(const Problem* __restrict__ probs) {
 
 // ----------------------------------------------------------------------------
 // wann_omega (src/wannierise.F90:1979-2284) as a deterministic two-pass reduction over
-// nchunk chunks of consecutive (k,b) blocks (at most kOmegaChunk each; the engine makes as many
+// nchunk chunks of consecutive (k,b) blocks (at most 64 each; the engine makes as many
 // chunks of at least 16 blocks as the chip has SMs):
 //   p1: per chunk  P_n = sum wb b ln_n (3W), q_n = sum wb (1 - |M_nn|^2 + ln_n^2) (W),
 //       sum wb offd, and (first pass only) sum wb (W - sum|M|^2); the last CTA: totals, centres,
@@ -250,10 +250,11 @@ __global__ void k_ctrl_end(const Problem* __restrict__ probs) {
 // there directly.  |M0|_F^2 minus the diagonal, the invariant form used before, cancels to ~1e-14 of
 // num_wann and near a minimum hid the trial step's change from the parabola (1000 k, num_wann 32,
 // 1e-12 window: refused steps, Omega 5e-8 after 3107 iterations; with the direct sum 8e-11).  For
-// num_wann <= 32 the first trial step still takes the invariant form: the first step length is the
-// one quantity that its offset against the entry overlaps' direct sum moves by more than rounding
-// (1e-9 in M after four iterations of 1000 k of num_wann 32), and with it the whole trajectory, which
-// so stays the earlier one.  Wider problems take the direct sum there too (M of 512 k of num_wann
+// num_wann <= 32 the first trial step still takes the invariant form, for the earlier trajectory's sake
+// and not for accuracy: the first step length is the one quantity that its offset against the entry
+// overlaps' direct sum moves by more than rounding, and with it M after four iterations of 1000 k of
+// num_wann 32 by 1.1e-9 (away from the earlier results, and towards those in 64 bits: with the
+// direct sum and 8-bit digits throughout their distance falls from 1.1e-9 to 2.2e-10).  Wider problems take the direct sum there too (M of 512 k of num_wann
 // 128 against 64 bits: 2.9e-10 with the invariant form, 5.8e-12 without).
 // Selective localisation (slwf_num = s > 0, :2144-2211): p1's off-diagonal slot holds
 // sum over n < s of wb (1 - |M_nn|^2 + lambda ln_n^2) (Omega_IOD) and its Omega_I slot
@@ -262,7 +263,6 @@ __global__ void k_ctrl_end(const Problem* __restrict__ probs) {
 // slot: 0 trial, 1 optimal step, 2 initial (accepted).  Fixed thread ownership and
 // fixed-order reductions make the result independent of scheduling.
 // ----------------------------------------------------------------------------
-constexpr int kOmegaChunk = 64;
 
 // Whether this CTA is the last of the problem's nchunk CTAs to finish (all threads get
 // the answer).  Every CTA makes its partials visible device-wide before it counts itself

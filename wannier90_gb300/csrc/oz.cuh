@@ -68,19 +68,6 @@ __device__ __forceinline__ long long scaled_int(double v, int e) {
   return (bits < 0) ? -n : n;
 }
 
-// signed 7-bit digits of N (|N| <= 2^49), extracted from the bottom:
-// x_7..x_2 in [-64, 63], x_1 the remaining top part (|x_1| <= 128); N = sum_t x_t 2^(7(7-t))
-__device__ __forceinline__ void digits7(long long n, int x[kS]) {
-#pragma unroll
-  for (int t = kS - 1; t > 0; --t) {
-    const int lo = (int)n & 127;
-    const int d = lo - ((lo & 64) << 1);     // centred in [-64, 63]
-    x[t] = d;
-    n = (n - d) >> 7;
-  }
-  x[0] = (int)n;
-}
-
 // 8-digit form (56 bits, used by the exp kernel): N = round(v * 2^(56 - e)), |N| <= 2^56
 __device__ __forceinline__ long long scaled_int56(double v, int e) {
   const long long bits = __double_as_longlong(v);
@@ -111,19 +98,6 @@ __device__ __forceinline__ long long scaled_int55(double v, int e) {
   return (bits < 0) ? -n : n;
 }
 
-// 7 signed 8-bit digits of N (|N| <= 2^55): x_7..x_2 in [-128, 127], |x_1| <= 128,
-// N = sum_t x_t 2^(8(7-t)); every digit is an exact FP16 value
-__device__ __forceinline__ void digits7x8(long long n, int x[7]) {
-#pragma unroll
-  for (int t = 6; t > 0; --t) {
-    const int lo = (int)n & 255;
-    const int d = lo - ((lo & 128) << 1);
-    x[t] = d;
-    n = (n - d) >> 8;
-  }
-  x[0] = (int)n;
-}
-
 // x - c for both halves of a packed FP16 pair (c packed likewise)
 __device__ __forceinline__ uint32_t f16x2_sub(uint32_t x, uint32_t c) {
   uint32_t r;
@@ -131,16 +105,10 @@ __device__ __forceinline__ uint32_t f16x2_sub(uint32_t x, uint32_t c) {
   return r;
 }
 
-// FP16 bits of a small integer (|x| <= 2048: exact)
-__device__ __forceinline__ uint16_t int_to_f16(int x) {
-  uint16_t r;
-  asm("cvt.rn.f16.s32 %0, %1;" : "=h"(r) : "r"(x));
-  return r;
-}
-
 // The seven 7-bit digit planes of 8 values scaled by 2^(49 - ex) (negated first when neg),
-// as packed FP16 pairs: w[t][i / 2] holds digit t of values i (low half) and i + 1 -- the
-// digits of digits7, without its serial recoding.  With C = 64 (1 + 2^7 + ... + 2^35), bits
+// as packed FP16 pairs: w[t][i / 2] holds digit t of values i (low half) and i + 1.  The digits are
+// those of the centred recoding from the bottom, N = sum_t x_t 2^(7(7-t)) with x_7..x_2 in [-64, 63]
+// and |x_1| <= 128 for |N| <= 2^49, without its serial steps.  With C = 64 (1 + 2^7 + ... + 2^35), bits
 // 7t'..7t'+6 of N + C are digit 6 - t' plus 64 (adding 64 at every lower digit position
 // turns the centred digits into the plain 7-bit fields of N + C), and the top digit is
 // (N + C) >> 42 (arithmetic), in [-128, 128].  Two values' 14-bit windows side by side in
@@ -169,8 +137,8 @@ __device__ __forceinline__ void pack_digits7(uint32_t (&w)[kS][4], const double 
 }
 
 // The eight 7-bit digit planes of 8 values scaled by 2^(56 - ex), packed as above (the centred
-// recoding of N, |N| <= 2^56, into x_8..x_2 in [-64, 63] and |x_1| <= 128).  C = 64 (1 + 2^7 + ... + 2^42); three 14-bit windows, the seventh field on its own, and
-// the top digit (N + C) >> 49 in [-128, 128].
+// recoding of N, |N| <= 2^56, into x_8..x_2 in [-64, 63] and |x_1| <= 128).  C = 64 (1 + 2^7 + ... +
+// 2^42); three 14-bit windows, the seventh field on its own, and the top digit (N + C) >> 49 in [-128, 128].
 __device__ __forceinline__ void pack_digits8(uint32_t (&w)[8][4], const double (&v)[8], int ex) {
 #pragma unroll
   for (int i = 0; i < 8; i += 2) {
@@ -193,8 +161,9 @@ __device__ __forceinline__ void pack_digits8(uint32_t (&w)[8][4], const double (
 }
 
 // The seven 8-bit digit planes of the 8 values scaled by 2^(55 - ex), as packed FP16
-// pairs: w[t][i / 2] holds digit t of values i (low half) and i + 1 -- the digits of
-// digits7x8, without its serial recoding.  With C = 128 (1 + 2^8 + ... + 2^40), byte t' of
+// pairs: w[t][i / 2] holds digit t of values i (low half) and i + 1.  The digits are those of
+// the centred recoding, N = sum_t x_t 2^(8(7-t)) with x_7..x_2 in [-128, 127] and |x_1| <= 128 for
+// |N| <= 2^55, without its serial steps.  With C = 128 (1 + 2^8 + ... + 2^40), byte t' of
 // N + C is digit 6 - t' plus 128 (adding 128 at every lower byte position turns the
 // centred digits into the plain bytes of N + C: x_6 = sext8(N mod 2^8) = byte0(N + 128) -
 // 128, and (N - x_6) / 2^8 = (N + 128) >> 8, so the next step repeats on N + 128 shifted),

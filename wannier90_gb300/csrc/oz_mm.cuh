@@ -29,30 +29,9 @@ struct ExpSmem {
   static constexpr int A_BYTES = A_ROWS * KC * 2;
   static constexpr int B_BYTES = NC * KC * 2;                     // per slice
   static constexpr int TMEM_COLS = (kS8 * NC <= 128) ? 128 : ((kS8 * NC <= 256) ? 256 : 512);
-  // W <= 32: the accumulators are staged through shared memory (aliasing the digit
-  // slices, free once the MMAs are done) so that all warps recombine, not just the two
-  // warps that can read the TMEM lanes of rows 0..31
-  static constexpr bool STAGED = WP <= 32;
-  static constexpr int STAGE_LD = NC + 1;                         // u32 row stride
-  static constexpr size_t STAGE_BYTES = STAGED ? (size_t)kS8 * WP * STAGE_LD * 4 : 0;
-  static constexpr size_t DIGIT_BYTES = (size_t)A_BYTES + (size_t)kS8 * B_BYTES;
-  static constexpr size_t REGION = DIGIT_BYTES > STAGE_BYTES ? DIGIT_BYTES : STAGE_BYTES;
-  static constexpr bool MATS_IN_SMEM = WP <= 32;
-  static constexpr size_t MAT_BYTES = (size_t)WP * WP * 16;
-  static constexpr size_t BYTES = REGION + (MATS_IN_SMEM ? 6 * MAT_BYTES : 0) + 1024;
+  static constexpr size_t REGION = (size_t)A_BYTES + (size_t)kS8 * B_BYTES;
+  static constexpr size_t BYTES = REGION + 1024;
 };
-
-__device__ __forceinline__ double cta_max(double v, double* red) {
-  red[threadIdx.x] = v;
-  __syncthreads();
-  for (int s = blockDim.x >> 1; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  const double r = red[0];
-  __syncthreads();
-  return r;
-}
 
 // per-CTA state of the tensor product
 struct OzCtx {
@@ -153,15 +132,6 @@ struct Epi {
 struct NoAdd {
   static constexpr bool kActive = false;
   __device__ double2 operator()(int) const { return make_double2(0.0, 0.0); }
-};
-
-// block q of the Paterson-Stockmeyer polynomial, added by a Horner step's epilogue
-template <class F>
-struct HornerAdd {
-  static constexpr bool kActive = true;
-  const F* f;
-  int q;
-  __device__ double2 operator()(int e) const { return (*f)(q, e); }
 };
 
 __device__ __forceinline__ void rec_clear(const Rec& r, int n) {
@@ -329,66 +299,29 @@ __device__ bool oz_cmm(OzCtx& cx, double2* C, const double2* A, const unsigned* 
     const int wq = warp & 3, half = warp >> 2;
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
     const int jbeg = half * (CW / 2), jend = jbeg + CW / 2;
-    if (E::STAGED) {
-      // ---- TMEM -> shared (warps 0 and 4 hold rows 0..31), then all warps recombine
-      uint32_t* stage = (uint32_t*)cx.sA;
-      if (wq == 0) {
+    // ---- direct: TMEM lane r = row r; warps w and w+4 split the chunk's columns
+    const int r = wq * 32 + lane;
+    if (wq * 32 < W) {   // warp-uniform
 #pragma unroll 1
-        for (int j0 = jbeg; j0 < jend; j0 += 4) {
+      for (int j0 = jbeg; j0 < jend; j0 += 4) {
+        uint32_t q[kS8][4], s4[kS8][4];
 #pragma unroll
-          for (int d = 0; d < kS8; ++d) {
-            uint32_t q[4], s4[4];
-            const uint32_t ta = cx.tmem + lane_base + (uint32_t)(d * NC + j0);
-            const uint32_t tb = cx.tmem + lane_base + (uint32_t)(d * NC + CW + j0);
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(ta));
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(s4[0]), "=r"(s4[1]), "=r"(s4[2]), "=r"(s4[3]) : "r"(tb));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (lane < WP) {
-              uint32_t* row = stage + ((size_t)d * WP + lane) * E::STAGE_LD;
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                row[j0 + j] = q[j];
-                row[CW + j0 + j] = s4[j];
-              }
-            }
-          }
+        for (int d = 0; d < kS8; ++d) {
+          const uint32_t ta = cx.tmem + lane_base + (uint32_t)(d * NC + j0);
+          const uint32_t tb = cx.tmem + lane_base + (uint32_t)(d * NC + CW + j0);
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(q[d][0]), "=r"(q[d][1]), "=r"(q[d][2]), "=r"(q[d][3])
+                       : "r"(ta));
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(s4[d][0]), "=r"(s4[d][1]), "=r"(s4[d][2]), "=r"(s4[d][3])
+                       : "r"(tb));
         }
-      }
-      __syncthreads();
-      for (int e = tid; e < W * CW; e += blockDim.x) {
-        const int r = e % W, j = e / W;
-        const int c = nc * CW + j;
-        if (c >= W) continue;
-        const uint32_t* rowp = stage + (size_t)r * E::STAGE_LD;
-        recombine(rowp + j, rowp + CW + j, WP * E::STAGE_LD, r, c);
-      }
-    } else {
-      // ---- direct: TMEM lane r = row r; warps w and w+4 split the chunk's columns
-      const int r = wq * 32 + lane;
-      if (wq * 32 < W) {   // warp-uniform
-#pragma unroll 1
-        for (int j0 = jbeg; j0 < jend; j0 += 4) {
-          uint32_t q[kS8][4], s4[kS8][4];
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (r < W) {
 #pragma unroll
-          for (int d = 0; d < kS8; ++d) {
-            const uint32_t ta = cx.tmem + lane_base + (uint32_t)(d * NC + j0);
-            const uint32_t tb = cx.tmem + lane_base + (uint32_t)(d * NC + CW + j0);
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(q[d][0]), "=r"(q[d][1]), "=r"(q[d][2]), "=r"(q[d][3])
-                         : "r"(ta));
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(s4[d][0]), "=r"(s4[d][1]), "=r"(s4[d][2]), "=r"(s4[d][3])
-                         : "r"(tb));
-          }
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (r < W) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int c = nc * CW + j0 + j;
-              if (c < W) recombine(&q[0][j], &s4[0][j], 4, r, c);
-            }
+          for (int j = 0; j < 4; ++j) {
+            const int c = nc * CW + j0 + j;
+            if (c < W) recombine(&q[0][j], &s4[0][j], 4, r, c);
           }
         }
       }
@@ -649,7 +582,7 @@ template <int WP>
 struct ProdV1 {
   using E = ExpSmem<WP>;
   static constexpr int TMEM_COLS = E::TMEM_COLS;
-  static constexpr bool MATS_IN_SMEM = E::MATS_IN_SMEM;
+  static constexpr bool MATS_IN_SMEM = false;
   static constexpr size_t REGION = E::REGION, BYTES = E::BYTES;
   static constexpr size_t SB_OFFSET = E::A_BYTES;
   template <class Add>

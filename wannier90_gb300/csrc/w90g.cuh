@@ -119,7 +119,8 @@ struct Problem {
   double2* U[2];
   double2* G;
   double2* D;
-  double2* dU;
+  double2* dU;          // (opart1, opart2, and on the tensor path odpart, ub2_exp and zs_exp, may lie in it: the
+                        // FP64 M update reads dU before the spread passes write)
   double2* work;        // exp workspace (FP64: W > 32; tensor path: any W): 6*W*W per k
   float* expinfo;       // tensor exp: [k][2] norm and state of the trial step's powers, for the optimal step
   double2* tbuf;        // M-update intermediate (W > 32): W*W per (k,b)
@@ -133,7 +134,8 @@ struct Problem {
   double* centres;      // [slot][4][W]: rave(3,W) + r2ave-rave2 (W) per spread slot; slot 2 = accepted
   double* log;          // [num_iter+1][kLogStride]
   double* log_centres;  // [num_iter+1][4][W]
-  double2* M0;          // tensor path: M at entry (never modified)
+  double2* M0;          // tensor path: M at entry, until it is sliced into m0s at the start of a solve; after
+                        // that zs, ub2 and zs_exp or work, and expinfo, odpart, opart1, opart2 may lie in its place
   unsigned char* m0s;   // tensor path: step 1's A operand (M0 rows) in FP16 digit planes,
                         // the shared-memory image of every (k, tile, K chunk)
   unsigned char* zs;    // tensor path, num_wann > 32: step 2's A operand (the rows of Z) likewise
