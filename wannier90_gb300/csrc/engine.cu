@@ -99,18 +99,23 @@ void Engine::release() {
 
 namespace {
 
-// tensor-core M update: every problem asks for it, W <= 128, and every k' has exactly
-// B predecessors (k,b) (true on Monkhorst-Pack meshes); returns the padded width or 0
-int choose_tensor_wp(const std::vector<ProblemSpec>& specs) {
+// every k' has exactly B predecessors (k,b) (true on Monkhorst-Pack meshes)
+bool regular_neighbours(const ProblemSpec& s) {
+  std::vector<int> cnt(s.K, 0);
+  for (int v : s.nnlist) cnt[v]++;
+  for (int c : cnt)
+    if (c != s.B) return false;
+  return true;
+}
+
+// tensor-core M update: every problem asks for it, W <= 128, and has regular neighbour lists; returns
+// the padded width or 0
+int choose_tensor_wp(const std::vector<ProblemSpec>& specs, const std::vector<char>& regular) {
   bool ok = !specs.empty();
   int wmax = 0;
-  for (const auto& s : specs) {
-    ok = ok && s.tensor && s.W <= 128;
-    wmax = std::max(wmax, s.W);
-    if (!ok) break;
-    std::vector<int> cnt(s.K, 0);
-    for (int v : s.nnlist) cnt[v]++;
-    for (int c : cnt) ok = ok && (c == s.B);
+  for (size_t p = 0; p < specs.size(); ++p) {
+    ok = ok && specs[p].tensor && specs[p].W <= 128 && regular[p];
+    wmax = std::max(wmax, specs[p].W);
   }
   if (!ok) return 0;
   return wmax <= 8 ? 8 : (wmax <= 16 ? 16 : (wmax <= 32 ? 32 : (wmax <= 64 ? 64 : 128)));
@@ -169,22 +174,33 @@ int Engine::setup(const std::vector<ProblemSpec>& specs, std::string& err) {
   }
   // layout key: reuse the arena when the problem shapes are unchanged, and with them all that alloc()
   // derives from the neighbour lists (choose_tensor_wp) and the options (which kernels run)
+  // (neighbour lists equal to those on the device are neither examined nor uploaded again)
+  std::vector<char> same(specs.size()), regular(specs.size());
+  for (size_t p = 0; p < specs.size(); ++p) {
+    same[p] = arena_ && p < specs_.size() && p < regular_.size() && specs[p].K == specs_[p].K &&
+              specs[p].B == specs_[p].B && specs[p].nnlist == specs_[p].nnlist;
+    regular[p] = same[p] ? regular_[p] : regular_neighbours(specs[p]);
+  }
+  regular_ = regular;
   std::ostringstream key;
-  key << choose_tensor_wp(specs) << ';';
+  key << choose_tensor_wp(specs, regular_) << ';';
   for (const auto& s : specs)
     key << s.W << ',' << s.K << ',' << s.B << ',' << s.ctl.num_iter << ',' << s.tensor << ',' << s.tensor_exp << ','
         << s.mupdate_pipe << ',' << s.exp_smem << ',' << s.precond << ',' << s.nrpts << ',' << s.guiding << ',' << s.nnh << ',' << (s.slwf_num > 0) << ',' << s.sym_nir << ','
         << s.sym_mem.size() << ',' << s.sym_grp.size() << ',' << s.sym_d.size() << ',' << s.lean << ';';
   specs_ = specs;
   if (arena_ && key.str() == layout_key_) {
-    // refresh the read-only tables (they may differ at equal shapes)
+    // refresh the read-only tables (they may differ at equal shapes); the key again when that is done
+    layout_key_.clear();
     for (size_t p = 0; p < specs_.size(); ++p) {
       const auto& s = specs_[p];
       Problem& P = hprobs_[p];
-      W90G_CHECK(cudaMemcpyAsync((void*)P.nnlist, s.nnlist.data(), s.nnlist.size() * sizeof(int), cudaMemcpyHostToDevice, stream()));
-      if (P.inv_nnlist) {
-        const std::vector<int> inv = inverse_neighbours(s);
-        W90G_CHECK(cudaMemcpyAsync((void*)P.inv_nnlist, inv.data(), inv.size() * sizeof(int), cudaMemcpyHostToDevice, stream()));
+      if (!same[p]) {
+        W90G_CHECK(cudaMemcpyAsync((void*)P.nnlist, s.nnlist.data(), s.nnlist.size() * sizeof(int), cudaMemcpyHostToDevice, stream()));
+        if (P.inv_nnlist) {
+          const std::vector<int> inv = inverse_neighbours(s);
+          W90G_CHECK(cudaMemcpyAsync((void*)P.inv_nnlist, inv.data(), inv.size() * sizeof(int), cudaMemcpyHostToDevice, stream()));
+        }
       }
       P.no_guide_iter = s.no_guide_iter;
       P.guide_cycles = s.guide_cycles;
@@ -205,11 +221,14 @@ int Engine::setup(const std::vector<ProblemSpec>& specs, std::string& err) {
       if (int rc = set_sym(p, err)) return rc;
     }
     W90G_CHECK(cudaMemcpyAsync(dprobs_, hprobs_.data(), hprobs_.size() * sizeof(Problem), cudaMemcpyHostToDevice, stream()));
+    layout_key_ = key.str();
     return 0;
   }
   release();
+  layout_key_.clear();
+  if (int rc = alloc(err)) return rc;
   layout_key_ = key.str();
-  return alloc(err);
+  return 0;
 }
 
 namespace {
@@ -370,7 +389,9 @@ size_t header_bytes(int np, int n_k) {
 }  // namespace
 
 size_t Engine::estimate_bytes(const std::vector<ProblemSpec>& specs) {
-  const int wp = choose_tensor_wp(specs);
+  std::vector<char> regular;
+  for (const auto& s : specs) regular.push_back(regular_neighbours(s));
+  const int wp = choose_tensor_wp(specs, regular);
   size_t total = 0;
   int nk = 0;
   for (const auto& s : specs) {
@@ -382,7 +403,7 @@ size_t Engine::estimate_bytes(const std::vector<ProblemSpec>& specs) {
 
 int Engine::alloc(std::string& err) {
   const int np = (int)specs_.size();
-  tensor_wp_ = choose_tensor_wp(specs_);
+  tensor_wp_ = choose_tensor_wp(specs_, regular_);
   if (!own_stream_) W90G_CHECK(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking));
   std::vector<Sizes> sz(np);
   size_t total = 0;

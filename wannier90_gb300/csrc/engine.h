@@ -152,7 +152,8 @@ class Engine {
   cudaStream_t user_stream_ = nullptr;
   cudaGraphExec_t graph_exec_ = nullptr;
   cudaStream_t graph_stream_ = nullptr;
-  std::string layout_key_;
+  std::string layout_key_;       // of the arrays on the device; empty while they are not complete
+  std::vector<char> regular_;    // per problem: its neighbour lists are regular
   long long launches_ = 0;
   int launched_iters_ = 0;
   std::vector<double> guide_init_;   // host staging of csheet = 1

@@ -104,19 +104,22 @@ __global__ void __launch_bounds__(256, 2) k_oz_rotate(RotateArgs g, int items) {
       rec_add(rR, i, j, r);
     }
     __syncthreads();
+    ok = E::mm(cx, T, LH, rL.row, M, rM.col, N, Epi{T, 0, rT}, none);
+    if (ok) ok = E::mm(cx, M, T, rT.row, R, rR.col, N, Epi{M, 0, Rec{nullptr, nullptr}}, none);
     double2* O = g.out + (size_t)it * W * W;
     if (__syncthreads_or(keys_wild(rL.row, N) || keys_wild(rM.col, N) || keys_wild(rR.col, N))) {
-      // (only the matrices' own extents: a zero of the padding times an infinity is not 0)
+      // again from the caller's block (only the matrices' own extents: a zero of the padding times an
+      // infinity is not 0)
+      for (int e = tid; e < n1 * n2; e += 256)
+        M[(size_t)(e / n1) * N + e % n1] = Mk[(size_t)(e / n1) * g.ldm + e % n1];
+      __syncthreads();
       rot_fp64(T, N, LH, N, M, N, W, n2, n1);
       __syncthreads();
       rot_fp64(O, W, T, N, R, N, W, W, n2);
-    } else {
-      ok = E::mm(cx, T, LH, rL.row, M, rM.col, N, Epi{T, 0, rT}, none);
-      if (ok) ok = E::mm(cx, M, T, rT.row, R, rR.col, N, Epi{M, 0, Rec{nullptr, nullptr}}, none);
-      if (ok)
-        for (int e = tid; e < W * W; e += 256) O[e] = M[(size_t)(e / W) * N + e % W];
+    } else if (ok) {
+      for (int e = tid; e < W * W; e += 256) O[e] = M[(size_t)(e / W) * N + e % W];
     }
-    __syncthreads();
+    // (the next block's loads come after the barrier behind its rec_clear)
   }
   if (!ok && tid == 0) *g.failed = 1;
   rot_end<E>(sh);
