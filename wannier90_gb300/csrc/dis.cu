@@ -147,9 +147,9 @@ __device__ void sort_eigs(const double2* H, int n, int* ord, double* ev) {
 // Q (m x w, ldq) = X (X^H X)^{-1/2}; scratch S, V, T (w x w) and Y (m x w).  Sets *flag
 // to 0, or 1 for a rank-deficient X, 2 when the eigensolver did not converge.  The eigenpairs of
 // X^H X decide on the rank; as X V L^{-1/2} V^H they also give Q where the square of X's condition
-// number, which their errors carry, is at most kPolarCond^2.  (Q was 2e-12 away from orthonormal at a
+// number, which their errors carry, is at most kPolarCond^2 = 64.  (Q was 2e-12 away from orthonormal at a
 // condition number of 100, 2e-6 at 1e5.)  Above that the iteration runs from X.
-constexpr double kPolarCond = 4.0;
+constexpr double kPolarCond = 8.0;
 __device__ void cta_polar(double2* Q, int ldq, const double2* X, int ldx, int m, int w, double2* S, double2* V,
                           double2* T, double2* Y, JacobiScratch js, int* flag) {
   cta_zgram(S, w, X, ldx, w, m);
