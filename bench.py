@@ -1272,9 +1272,9 @@ KNOWN_ITERS = {"dis_fcc8_b48w32": (200, 3053)}
 # kernel, from the committed ncu captures under profiles/ (name of the summary beside each)
 NCU_TRAFFIC = {
     # profiles/k_oz_mupdate2_fcc10_w32.md: steps 1 + 2 of one M update
-    ("fcc10_w32", "k_m_update"): 678.3e6,
+    ("fcc10_w32", "k_m_update"): 678.9e6,
     # profiles/k_oz_exp_fcc10_w32.md: one trial-step exp launch
-    ("fcc10_w32", "k_exp_u"): 131.9e6,
+    ("fcc10_w32", "k_exp_u"): 111.1e6,
 }
 
 if __name__ == "__main__":

@@ -18,9 +18,10 @@
 //   epilogue    16 warps: exact recombination of the 7 diagonals in int64, FP64 stores, and in
 //               step 2 the diagonal statistics and off-diagonal sums of the spread.
 //
-// What bounds it: a 128 x 64 x 16 stage is 28 digit-pair MMAs, ~1000 cycles of the tensor pipe, and
-// 43 KB from L2; at num_wann 128 the copies run at 5.5 TB/s.  The 448 accumulator columns of a chunk
-// leave no room for a second set, so the epilogue and the next chunk's MMAs alternate.  Shapes follow num_wann itself, not a padded width: rows of consecutive blocks share
+// What bounds it: the 448 accumulator columns of a chunk leave no room for a second set, so the
+// epilogue and the next chunk's MMAs alternate -- a 128 x 64 x 16 stage is 28 digit-pair MMAs, and at
+// num_wann 128 the tensor pipe is active 40 and 38 % of the two passes (L2 19 %, DRAM 23 %; the
+// copies run at 5.5 TB/s and are not the limit).  Shapes follow num_wann itself, not a padded width: rows of consecutive blocks share
 // a tile (B W / 128 tiles), K stops at the next multiple of 8 complex indices and the columns are
 // cut into equal chunks of at most 32, so num_wann 48 costs 3/4 x 3/4 of 64 and not the same.
 //

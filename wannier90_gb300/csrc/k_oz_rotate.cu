@@ -5,7 +5,8 @@
 //   k_oz_ufinal  U = U0 R at the end of a tensor-path solve.
 // In FP64 these are bound by the FP64 pipe (8000 blocks of num_wann 32: 3.6 ms, 4096 of 42 states to
 // 32: 2.9 ms, U0 R of 512 x 128: 8.3 ms).  The products here are as accurate as FP64 ones; what
-// bounds them is slicing and recombining, two CTAs per SM hiding each other's latency.
+// bounds them is the chain of slicing, MMAs and recombining, two CTAs per SM hiding some of each other's
+// latency (8000 blocks of 32: 0.79 ms, ALU 39 %, issue 40 %, tensor pipe 12 %).
 // Operands whose scales the digits do not carry (exp_wild: NaN, infinities, magnitudes beyond 2^+-290)
 // are multiplied in FP64 here, block by block, so that they come out as FP64 gives them.
 #include <algorithm>
