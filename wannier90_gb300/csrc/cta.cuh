@@ -355,28 +355,18 @@ __device__ __noinline__ static int cta_jacobi(double2* H, double2* V, int W, int
 // Unitary polar factor X (X^H X)^{-1/2} of an m x w matrix by the Newton-Schulz iteration
 // X <- X (3 I - X^H X) / 2 on X itself: unitary to roundoff, its error that of the products times X's
 // condition number.  (The eigenpairs of X^H X carry the square of that number: above ~1e4 what they
-// give is not unitary, and no first-order correction is enough.)  Singular values below 1 grow by 1.5 a
-// step, so this takes 1.7 log10(cond) + 6 steps or so of 6 m w^2 FMA.  X (ldx) and Y (ldy) take turns,
-// G is w x w scratch, red one double per thread.  Returns the one that holds the result, or null where
-// 120 steps were not enough (a singular value of 0).  All threads call.
+// give is not unitary, and no first-order correction is enough.)  The first step's coefficients scale
+// the mean square of the singular values to 1, or the largest below 1 where it would come near sqrt(3);
+// those below 1 grow by 1.5 a step, so this takes 1.7 log10(cond) + 4 steps or so of 6 m w^2 FMA.
+// X (ldx) and Y (ldy) take turns, G is w x w scratch, red one double per thread.  Returns the one that
+// holds the result, or null where `steps` were not enough (120: a singular value of 0) or X is not
+// finite.  All threads call.
 __device__ __noinline__ static double2* cta_polar_ns(double2* X, int ldx, double2* Y, int ldy, double2* G, int m, int w,
-                                                     double* red) {
+                                                     double* red, int steps = 120) {
   __shared__ int s_far;
-  double sq = 0.0;
-  for (int e = threadIdx.x; e < m * w; e += blockDim.x) sq += cabs2(X[(size_t)(e / m) * ldx + e % m]);
-  sq = block_sum(sq, red);
-  if (!(sq > 0.0) || !isfinite(sq)) return nullptr;
-  // |X|_2 <= |X|_F < 2^half
-  int half;
-  frexp(sq, &half);
-  half = (half + 1) >> 1;
-  const double r = ldexp(1.0, -half);
-  for (int e = threadIdx.x; e < m * w; e += blockDim.x) {
-    double2& x = X[(size_t)(e / m) * ldx + e % m];
-    x = cscale(x, r);
-  }
-  __syncthreads();
-  for (int step = 0; step < 120; ++step) {
+  // G = X^H X in the first step, (I - X^H X) / 2 after it (X + X G rounds relative to what changes), and
+  // whether |X^H X - I| is below 1e-8 / w elementwise: a step then leaves less than 1e-16
+  auto gram = [&](bool first) -> bool {
     if (threadIdx.x == 0) s_far = 0;
     __syncthreads();
     bool far = false;
@@ -386,20 +376,60 @@ __device__ __noinline__ static double2* cta_polar_ns(double2* X, int ldx, double
       double2 g = cmk(0, 0);
       for (int l = 0; l < m; ++l) cfmac(g, X[(size_t)i * ldx + l], X[(size_t)j * ldx + l]);
       if (i == j) g.y = 0.0;
-      // |X^H X - I| below 1e-8 / w elementwise: the step leaves less than 1e-16
-      far = far || !(fabs(g.x - (i == j ? 1.0 : 0.0)) + fabs(g.y) < 1.0e-8 / w);
-      g = cmk((i == j ? 1.5 : 0.0) - 0.5 * g.x, -0.5 * g.y);
+      const double d = (i == j ? 1.0 : 0.0) - g.x;
+      far = far || !(fabs(d) + fabs(g.y) < 1.0e-8 / w);
+      if (!first) g = cmk(0.5 * d, -0.5 * g.y);
       G[(size_t)j * w + i] = g;
       if (i < j) G[(size_t)i * w + j] = cconj(g);
     }
     if (far) s_far = 1;
     __syncthreads();
-    const bool done = s_far == 0;
+    return s_far == 0;
+  };
+  auto mean = [&]() {
+    double t = 0.0;
+    for (int j = 0; j < w; ++j) t += G[(size_t)j * w + j].x;
+    return t / w;
+  };
+  for (int step = 0; step < steps; ++step) {
+    bool done = gram(step == 0);
+    double ca = 1.0, cb = 1.0;
+    if (step == 0) {
+      double mu = mean();
+      if (!(mu > 0.0) || !isfinite(mu)) return nullptr;
+      if (!(mu > 1.0e-60 && mu < 1.0e60)) {
+        // far from 1: an exact scaling first
+        int half;
+        frexp(mu, &half);
+        const double r = ldexp(1.0, -(half >> 1));
+        __syncthreads();
+        for (int e = threadIdx.x; e < m * w; e += blockDim.x) {
+          double2& x = X[(size_t)(e / m) * ldx + e % m];
+          x = cscale(x, r);
+        }
+        __syncthreads();
+        gram(true);
+        mu = mean();
+      }
+      // |X|_2^2 <= |X^H X|_1 <= the largest sum of |re| + |im| down a column
+      double b = 0.0;
+      for (int j = threadIdx.x; j < w; j += blockDim.x) {
+        double t = 0.0;
+        for (int i = 0; i < w; ++i) t += fabs(G[(size_t)j * w + i].x) + fabs(G[(size_t)j * w + i].y);
+        b = fmax(b, t);
+      }
+      b = block_max(b, red);
+      const double r = 1.0 / sqrt(b < 2.8 * mu ? mu : b);
+      ca = 1.5 * r;
+      cb = -0.5 * r * r * r;
+      done = false;
+    }
     for (int e = threadIdx.x; e < m * w; e += blockDim.x) {
       const int i = e % m, j = e / m;
       double2 y = cmk(0, 0);
       for (int l = 0; l < w; ++l) cfma(y, X[(size_t)l * ldx + i], G[(size_t)j * w + l]);
-      Y[(size_t)j * ldy + i] = y;
+      const double2 x = X[(size_t)j * ldx + i];
+      Y[(size_t)j * ldy + i] = cmk(fma(cb, y.x, ca * x.x), fma(cb, y.y, ca * x.y));
     }
     __syncthreads();
     double2* t = X;

@@ -144,44 +144,34 @@ __device__ void sort_eigs(const double2* H, int n, int* ord, double* ev) {
   __syncthreads();
 }
 
-// Q (m x w, ldq) = X (X^H X)^{-1/2}; scratch S, V, T (w x w) and Y (m x w).  Sets *flag
-// to 0, or 1 for a rank-deficient X, 2 when the eigensolver did not converge.  The eigenpairs of
-// X^H X decide on the rank; as X V L^{-1/2} V^H they also give Q where the square of X's condition
-// number, which their errors carry, is at most kPolarCond^2 = 64.  (Q was 2e-12 away from orthonormal at a
-// condition number of 100, 2e-6 at 1e5.)  Above that the iteration runs from X.
-constexpr double kPolarCond = 8.0;
+// Q (m x w, ldq; may be X) = X (X^H X)^{-1/2}; scratch S, T (w x w), V and Y (m x w).  Sets *flag
+// to 0, or 1 for a rank-deficient X, 2 when the eigensolver did not converge.  As in k_lowdin: by the
+// Newton-Schulz iteration from X, and where that takes more steps than usual after a look at the
+// eigenvalues of X^H X.  (X V L^{-1/2} V^H from the eigenpairs was 2e-12 away from orthonormal at a
+// condition number of 100, 2e-6 at 1e5.)
+constexpr int kPolarSteps64 = 32;
+
 __device__ void cta_polar(double2* Q, int ldq, const double2* X, int ldx, int m, int w, double2* S, double2* V,
                           double2* T, double2* Y, JacobiScratch js, int* flag) {
+  auto iterate = [&](int steps) -> bool {
+    for (int e = threadIdx.x; e < m * w; e += blockDim.x) Y[e] = X[(size_t)(e / m) * ldx + e % m];
+    __syncthreads();
+    const double2* R = cta_polar_ns(Y, m, V, m, T, m, w, js.red, steps);
+    if (R)
+      for (int e = threadIdx.x; e < m * w; e += blockDim.x) Q[(size_t)(e / m) * ldq + e % m] = R[e];
+    __syncthreads();
+    return R != nullptr;
+  };
+  if (threadIdx.x == 0) *flag = 0;
+  if (iterate(kPolarSteps64)) return;
   cta_zgram(S, w, X, ldx, w, m);
   const int sw = cta_jacobi(S, V, w, 60, js.red, js.rc, js.rse, js.rp, js.rq, 0.0, T, Y);
   if (threadIdx.x == 0) *flag = (sw < 0) ? 2 : 0;
   __syncthreads();
-  for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-    const int j = e / w;
-    const double l = S[(size_t)j * w + j].x;
-    if (!(l > 0.0)) *flag = 1;
-    T[e] = cscale(V[e], 1.0 / sqrt(fmax(l, 1e-300)));
-  }
+  for (int j = threadIdx.x; j < w; j += blockDim.x)
+    if (!(S[(size_t)j * w + j].x > 0.0)) *flag = 1;
   __syncthreads();
-  double lmin = S[0].x, lmax = lmin;
-  for (int j = 1; j < w; ++j) {
-    const double l = S[(size_t)j * w + j].x;
-    lmin = fmin(lmin, l);
-    lmax = fmax(lmax, l);
-  }
-  if (*flag == 0 && lmax > kPolarCond * kPolarCond * lmin && isfinite(lmax)) {
-    for (int e = threadIdx.x; e < m * w; e += blockDim.x) Y[e] = X[(size_t)(e / m) * ldx + e % m];
-    __syncthreads();
-    const double2* R = cta_polar_ns(Y, m, Q, ldq, T, m, w, js.red);
-    if (R == Y)
-      for (int e = threadIdx.x; e < m * w; e += blockDim.x) Q[(size_t)(e / m) * ldq + e % m] = Y[e];
-    if (R == nullptr && threadIdx.x == 0) *flag = 1;
-    __syncthreads();
-    return;
-  }
-  cta_zgemm(Y, m, X, ldx, false, T, w, false, m, w, w);
-  __syncthreads();
-  cta_zgemm(Q, ldq, Y, m, false, V, w, true, m, w, w);
+  if (*flag == 0 && !iterate(120) && threadIdx.x == 0) *flag = 1;
   __syncthreads();
 }
 

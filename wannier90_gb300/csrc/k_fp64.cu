@@ -1383,30 +1383,27 @@ __global__ void k_log_init(const Problem* __restrict__ probs) {
 
 // ----------------------------------------------------------------------------
 // k_lowdin: overlap_project's U(k) = Z V^dagger from A(k) = Z S V^dagger
-// (src/overlap.F90:842-860), computed as U = A (A^H A)^{-1/2} = A V L^{-1/2} V^H with the
-// Jacobi eigenpairs (V, L) of A^H A: the same unitary polar factor for full-rank A.  The
-// eigenpairs carry the square of A's condition number; while that is small (condition numbers up to
-// kLowdinCond, square times 2^-53 below 2e-9) the two steps after them take it back to the
-// condition number itself: one Newton-Schulz step (U unitary again), then U <- U (I + X)
-// with X anti-Hermitian from X H + H X = H1 - H1^H, H1 = U^H A (the polar factor is the U
-// that makes H1 Hermitian), solved in the eigenbasis, where H = L^{1/2}.  Both are of first order:
-// above kLowdinCond the iteration runs from A itself instead (cta_polar_ns), and the
-// eigenvalues only give the verdict on A's rank.
+// (src/overlap.F90:842-860), the unitary polar factor A (A^H A)^{-1/2}, by the Newton-Schulz iteration
+// from A itself (cta_polar_ns).  Where kLowdinSteps steps are not enough -- condition numbers above
+// ~1e4, a rank-deficient A, NaN -- the Jacobi eigenvalues of A^H A give the verdict, and a matrix of
+// full rank takes as many steps as it needs.  (The factor from those eigenpairs, A V L^{-1/2} V^H and
+// two steps of correction, cost 2.4 times as much at num_wann 8 on 1000 k -- projection 696 us, now
+// 285 -- was no closer to the exact one, and 1e-4 away from unitary at a condition number of 1e7.)
 // Input A(k) in U[cur](k) (the reference reads A into u_matrix, src/wannier_prog.F90:523-529);
 // output U overwrites it.  One CTA (256 threads) per (problem, k).
-// Status per k: 0 ok, 1 rank deficient, 2 Jacobi not converged.  A matrix whose status is
-// kPolarDone on entry has been finished by k_oz_polar.
+// Status per k: 0 ok, 1 rank deficient, 2 Jacobi not converged.  A matrix whose status is kPolarDone on
+// entry has been finished by k_oz_polar, one with kPolarLeft needs more steps than kLowdinSteps.
 // ----------------------------------------------------------------------------
-constexpr double kLowdinCond = 4.0e3;
+constexpr int kLowdinSteps = 32;
 
-__global__ void __launch_bounds__(256) k_lowdin(const Problem* __restrict__ probs, WorkMap wm,
-                                                int* __restrict__ status) {
+__global__ void __launch_bounds__(256, 3) k_lowdin(const Problem* __restrict__ probs, WorkMap wm,
+                                                   int* __restrict__ status) {
   extern __shared__ double2 smem[];
   __shared__ double red[256];
   __shared__ double rc[128];
   __shared__ double2 rse[128];
   __shared__ int rp[128], rq[128];
-  __shared__ double s_h[256];
+  __shared__ int bad, infinite;
   if (status[blockIdx.x] == kPolarDone) return;
   int k;
   const int p = locate(wm, blockIdx.x, k);
@@ -1415,75 +1412,51 @@ __global__ void __launch_bounds__(256) k_lowdin(const Problem* __restrict__ prob
   double2* buf = (W <= kSmemW) ? smem : (P.work + (size_t)k * 6 * WW);
   double2 *A = buf, *S = buf + WW, *V = buf + 2 * WW, *T = buf + 3 * WW;
   double2* Uk = P.U[P.st->cur] + (size_t)k * WW;
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) A[e] = Uk[e];
-  __syncthreads();
+  auto load = [&]() {
+    for (int e = threadIdx.x; e < WW; e += blockDim.x) A[e] = Uk[e];
+    __syncthreads();
+  };
+  auto finish = [&](const double2* Q) {
+    for (int e = threadIdx.x; e < WW; e += blockDim.x) Uk[e] = Q[e];
+    if (threadIdx.x == 0) status[blockIdx.x] = 0;
+  };
+  load();
+  if (status[blockIdx.x] != kPolarLeft) {
+    const double2* Q = cta_polar_ns(A, W, T, W, S, W, W, red, kLowdinSteps);
+    if (Q) {
+      finish(Q);
+      return;
+    }
+    load();
+  }
   jac_mm<true, true>(S, A, A, W);
-  // A is scratch of the eigensolver, and read again afterwards
   const int sweeps = cta_jacobi(S, V, W, 60, red, rc, rse, rp, rq, 0.0, A, T);
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) A[e] = Uk[e];
-  __shared__ int bad;
-  if (threadIdx.x == 0) bad = (sweeps < 0) ? 2 : 0;
+  if (threadIdx.x == 0) {
+    bad = (sweeps < 0) ? 2 : 0;
+    infinite = 0;
+  }
   __syncthreads();
   for (int j = threadIdx.x; j < W; j += blockDim.x) {
     const double l = S[j * W + j].x;
     if (!(l > 0.0)) bad = 1;
-    s_h[j] = sqrt(l);
+    if (!isfinite(l)) infinite = 1;
   }
   __syncthreads();
-  double hmin = s_h[0], hmax = s_h[0];
-  for (int j = 1; j < W; ++j) {
-    hmin = fmin(hmin, s_h[j]);
-    hmax = fmax(hmax, s_h[j]);
-  }
-  if (!bad && hmax > kLowdinCond * hmin && isfinite(hmax)) {
-    const double2* Q = cta_polar_ns(A, W, T, W, S, W, W, red);
-    for (int e = threadIdx.x; e < WW; e += blockDim.x)
-      if (Q) Uk[e] = Q[e];
-    if (threadIdx.x == 0) status[blockIdx.x] = Q ? 0 : 1;
+  if (!bad && infinite) {
+    // a lone infinity in its row and column
+    for (int e = threadIdx.x; e < WW; e += blockDim.x) Uk[e] = cmk(nan(""), nan(""));
+    if (threadIdx.x == 0) status[blockIdx.x] = 0;
     return;
   }
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) T[e] = cscale(V[e], 1.0 / s_h[e / W]);
-  __syncthreads();
-  cta_gemm<false>(S, W, A, W, T, W, W);      // S <- A V L^{-1/2}
-  __syncthreads();
-  // C = X V^H
-  auto mul_vh = [&](double2* C, const double2* X) {
-    for (int e = threadIdx.x; e < WW; e += blockDim.x) {
-      const int i = e % W, j = e / W;
-      double2 acc = cmk(0, 0);
-      for (int l = 0; l < W; ++l) acc = cadd(acc, cmulc(X[l * W + i], V[l * W + j]));
-      C[e] = acc;
+  if (!bad) {
+    load();
+    const double2* Q = cta_polar_ns(A, W, T, W, S, W, W, red);
+    if (Q) {
+      finish(Q);
+      return;
     }
-  };
-  mul_vh(T, S);
-  __syncthreads();
-  // Newton-Schulz: U (3 I - U^H U) / 2
-  jac_mm<true, true>(S, T, T, W);
-  __syncthreads();
-  for (int e = threadIdx.x; e < WW; e += blockDim.x)
-    S[e] = cmk(((e % W) == (e / W) ? 1.5 : 0.0) - 0.5 * S[e].x, -0.5 * S[e].y);
-  __syncthreads();
-  cta_gemm<false>(Uk, W, T, W, S, W, W);
-  __syncthreads();
-  // the anti-Hermitian part of H1 = U^H A, twice: K = H1 - H1^H; X = V [(V^H K V)_ij / (h_i + h_j)] V^H
-  cta_gemm<true>(S, W, Uk, W, A, W, W);
-  __syncthreads();
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) T[e] = csub(S[e], cconj(S[(e % W) * W + e / W]));
-  __syncthreads();
-  cta_gemm<false>(S, W, T, W, V, W, W);
-  __syncthreads();
-  cta_gemm<true>(T, W, V, W, S, W, W);
-  __syncthreads();
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) T[e] = cscale(T[e], 1.0 / (s_h[e % W] + s_h[e / W]));
-  __syncthreads();
-  cta_gemm<false>(S, W, V, W, T, W, W);
-  __syncthreads();
-  mul_vh(T, S);
-  __syncthreads();
-  cta_gemm<false>(S, W, Uk, W, T, W, W);
-  __syncthreads();
-  for (int e = threadIdx.x; e < WW; e += blockDim.x) Uk[e] = cadd(Uk[e], S[e]);
-  if (threadIdx.x == 0) status[blockIdx.x] = bad;
+  }
+  if (threadIdx.x == 0) status[blockIdx.x] = bad ? bad : 1;
 }
 
 // ----------------------------------------------------------------------------

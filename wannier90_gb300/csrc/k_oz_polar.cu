@@ -11,7 +11,7 @@
 // Singular values start in (0, 1] (the first step's coefficients carry the scale, an upper
 // bound on ||X|| from the Gram matrix, so no element of X is rounded for it).  A matrix whose
 // smallest one has not reached 1 after kPolarSteps steps -- a condition number above ~1e5, or
-// a rank-deficient X -- is left alone with status 0: the FP64 kernel that runs next takes it,
+// a rank-deficient X -- is left alone with status kPolarLeft: the FP64 kernel that runs next takes it,
 // with its own verdict.  That kernel also takes everything else this one cannot finish
 // (a bounded wait that ran out, NaN, infinities and scales outside what the digits carry).
 #include "oz_mm.cuh"
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256, 2) k_oz_polar(PolarArgs g) {
       Q[(size_t)j * g.ldq + i] = i < rows ? X[(size_t)j * N + i] : cmk(0.0, 0.0);
     }
   }
-  if (tid == 0) g.status[k] = good ? kPolarDone : 0;
+  if (tid == 0) g.status[k] = good ? kPolarDone : kPolarLeft;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {

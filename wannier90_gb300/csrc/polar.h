@@ -7,6 +7,8 @@ namespace w90g {
 
 // d_status value of a matrix k_oz_polar has finished: the FP64 kernels skip it
 constexpr int kPolarDone = 0x600D;
+// ... and of one it has left alone: k_lowdin does not try its own iteration first
+constexpr int kPolarLeft = 0x1EF7;
 
 struct PolarArgs {
   const double2* x;      // [k] rows(k) x cols, column-major
@@ -22,7 +24,7 @@ struct PolarArgs {
   int n;                 // order of the square work matrices, >= rows(k) and cols
   double2* work;         // [k] kPolarMats n x n
   size_t strideW;
-  int* status;           // [k] kPolarDone, or 0 where the iteration left the matrix alone
+  int* status;           // [k] kPolarDone, or kPolarLeft where the iteration left the matrix alone
 };
 
 constexpr int kPolarMats = 4;
