@@ -106,6 +106,9 @@ __global__ void __launch_bounds__(256, 2) k_oz_exp(const Problem* __restrict__ p
   __shared__ unsigned s_key[5][2][WP];
   __shared__ int s_bad;
   __shared__ float s_wmax[8];
+  __shared__ double s_f;
+  __shared__ float s_rho;
+  __shared__ int s_reuse, s_have3;
 
   int k;
   const int p = locate(wm, blockIdx.x, k);
@@ -144,18 +147,28 @@ __global__ void __launch_bounds__(256, 2) k_oz_exp(const Problem* __restrict__ p
   rec_clear(rP2, WP);
   rec_clear(rZ, WP);
   rec_clear(rL, WP);
+  if (which == 1 && tid == 0) {
+    // (one thread: an FP64 divide by all of them takes the FP64 pipe a microsecond)
+    const double q = st->s_second / st->s_trial;
+    const float r = info[0], g = (float)q;
+    // The trial's powers serve the optimal step where its plan is safe: abs_est leaves out moduli of
+    // X^2 below 2^-60, at most 2^-53 in a column sum.  From a norm of 2^-24 on that is 1.5 % of it,
+    // within the plan's own slack of 5 %; below, as long as T4 covers the step whatever was left out
+    // (steps of a thousand times the trial's are ordinary near the minimum).  A longer step, or any
+    // after a trial of length 0 (the ratio is NaN or infinite), starts from its own X.
+    s_reuse = (r >= 0x1p-24f && fabsf(g) <= 0x1p60f) || (r * r + 0x1p-53f) * (g * g) <= 1.6e-3f * 1.6e-3f;
+    s_f = q;
+    s_rho = r * fabsf(g) * 1.0001f;
+    s_have3 = info[1] != 0.0f;
+  }
   __syncthreads();
   OzCtx cx{base, base + E::SB_OFFSET, tmem_slot, smem_u32(&mbar), 0u, s_rowexp, s_colexp, &s_bad};
   bool ok = true;
   float rho;
-  double f = which == 0 ? 1.0 : st->s_second / st->s_trial;
+  double f = 1.0;
   bool have3 = false;
   int nprod = 0;
-  // The trial's powers serve the optimal step where its norm's estimate is sure to 2^-10: abs_est
-  // leaves out moduli of X^2 below 2^-60, at most 2^-53 in a column sum, against 2^-40 or more.  Below
-  // that, a step up to 256 times as long still has a norm under T4's bound, whatever was left out;
-  // a longer one, or any after a trial of length 0 (f is NaN or infinite), starts from its own X.
-  const bool reuse = which == 1 && (fabs(f) <= 256.0 || (info[0] >= 0x1p-20f && fabs(f) <= 0x1p100));
+  const bool reuse = which == 1 && s_reuse;
   if (!reuse) {
     // ---- X = s D (first D = coefG G + coefD D_prev; in the symmetry-adapted mode k_sym_dir has
     // formed D already).  Each product and the sum rounded on its own, as the oracle forms D:
@@ -163,7 +176,6 @@ __global__ void __launch_bounds__(256, 2) k_oz_exp(const Problem* __restrict__ p
     double2* Dk = P.D + (size_t)k * WW;
     const double s = which == 0 ? st->s_trial : st->s_second;
     const bool form_d = which == 0 && P.sym_nir == 0;
-    f = 1.0;
     const double cg = st->coefG, cd = st->coefD;
     const double2* Gk = form_d ? (st->use_gp ? P.pc_gp : P.G) + (size_t)k * WW : nullptr;
 #pragma unroll 4
@@ -199,8 +211,9 @@ __global__ void __launch_bounds__(256, 2) k_oz_exp(const Problem* __restrict__ p
     for (int w = 0; w < 8; ++w) cmax = fmaxf(cmax, s_wmax[w]);
     rho = sqrtf(cmax * 1.001f);
   } else {
-    rho = info[0] * fabsf((float)f) * 1.0001f;
-    have3 = info[1] != 0.0f;
+    f = s_f;
+    rho = s_rho;
+    have3 = s_have3 != 0;
   }
   int m, js;
   exp_plan(rho, m, js);
